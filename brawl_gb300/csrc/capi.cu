@@ -353,7 +353,7 @@ struct brawl_batch {
   int max_z = 0;
   // chains run by the halo kernel, and its shared-memory size / unrolling
   std::vector<int> halo;
-  uint32_t halo_smem = 0;
+  uint32_t halo_smem = 0, spec_smem = 0;  // one trial at a time; speculative rounds
   int halo_min_z = 0, halo_max_z = 0;
   std::vector<ChainJob> staged;          // jobs in launch order
   int n_halo_launch = 0;
@@ -361,7 +361,7 @@ struct brawl_batch {
   // species, shells) share a class; each class is launched on its own
   // stream with its own shared memory, unrolling and trials per round
   std::vector<int> cls;                  // per chain: class, or -1 (not a halo chain)
-  std::vector<uint32_t> class_smem;
+  std::vector<uint32_t> class_smem, class_spec_smem;
   std::vector<int> class_z, class_depth;
   std::vector<int> class_first, class_count;  // in launch order (upload_jobs)
   std::vector<cudaStream_t> side;        // one per class beyond the first
@@ -525,8 +525,8 @@ int launch_classes(brawl_batch* b, cudaStream_t stream, int only) {
     const int k = ks[i];
     cudaStream_t st = i == 0 ? stream : b->side[i - 1];
     if (i > 0) CUDA_TRY(cudaStreamWaitEvent(st, b->ev_fork, 0));
-    launch_halo_chains(b->d_jobs + b->class_first[k], b->class_count[k], b->class_smem[k], b->class_z[k],
-                       b->class_z[k], b->class_depth[k], b->max_optin, st);
+    launch_halo_chains(b->d_jobs + b->class_first[k], b->class_count[k], b->class_smem[k], b->class_spec_smem[k],
+                       b->class_z[k], b->class_z[k], b->class_depth[k], b->max_optin, st);
     CUDA_TRY(cudaGetLastError());
     if (i > 0) CUDA_TRY(cudaEventRecord(b->ev_side[i - 1], st));
   }
@@ -572,8 +572,8 @@ int launch_sweep(brawl_batch* b, cudaStream_t stream) {
   if (nh > 0 && b->per_class)
     TRY(launch_classes(b, stream, -1));
   else if (nh > 0)
-    launch_halo_chains(b->d_jobs, nh, b->halo_smem, b->halo_min_z, b->halo_max_z, b->spec_nc, b->max_optin,
-                       stream);
+    launch_halo_chains(b->d_jobs, nh, b->halo_smem, b->spec_smem, b->halo_min_z, b->halo_max_z, b->spec_nc,
+                       b->max_optin, stream);
   if (n - nh > 0)
     launch_metropolis(b->d_jobs + nh, n - nh, b->smem_lat, b->use_D, b->smem_bytes, b->max_z, stream);
   CUDA_TRY(cudaGetLastError());
@@ -602,8 +602,8 @@ int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accept
     const int nh = b->n_halo_launch;
     for (int k = 0; k < n; ++k) {
       if (k < nh)
-        launch_halo_chains(b->d_jobs + k, 1, b->halo_smem, b->halo_min_z, b->halo_max_z, b->spec_nc, b->max_optin,
-                           stream);
+        launch_halo_chains(b->d_jobs + k, 1, b->halo_smem, b->spec_smem, b->halo_min_z, b->halo_max_z,
+                           b->spec_nc, b->max_optin, stream);
       else
         launch_metropolis(b->d_jobs + k, 1, b->smem_lat, b->use_D, b->smem_bytes, b->max_z,
                           stream);
@@ -659,7 +659,7 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     HaloGeom H;
     bool ok;
     make_halo(b->models[c].g, H, ok);
-    if (ok && halo_layout(b->models[c].g, H).total <= (uint32_t)max_optin) continue;
+    if (ok && window_layout(b->models[c].g, H).total <= (uint32_t)max_optin) continue;
     need_smem = std::max(need_smem, smem_layout(b->models[c].g, true).total);
     need_gmem = std::max(need_gmem, smem_layout(b->models[c].g, false).total);
   }
@@ -670,7 +670,7 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     HaloGeom H;
     bool ok;
     make_halo(m.g, H, ok);
-    if (ok && halo_layout(m.g, H).total <= (uint32_t)max_optin) {
+    if (ok && window_layout(m.g, H).total <= (uint32_t)max_optin) {
       b->halo[c] = 1;
       int k = 0;
       for (; k < c; ++k) {
@@ -684,11 +684,13 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
         b->cls[c] = b->cls[k];
       } else {
         b->cls[c] = (int)b->class_smem.size();
-        b->class_smem.push_back(halo_layout(m.g, H).total);
+        b->class_smem.push_back(window_layout(m.g, H).total);
+        b->class_spec_smem.push_back(halo_layout(m.g, H).total);
         b->class_z.push_back((int)m.g.z);
         b->class_depth.push_back(kDefaultSpeculation);
       }
-      b->halo_smem = std::max(b->halo_smem, halo_layout(m.g, H).total);
+      b->halo_smem = std::max(b->halo_smem, window_layout(m.g, H).total);
+      b->spec_smem = std::max(b->spec_smem, halo_layout(m.g, H).total);
       b->halo_min_z = b->halo_max_z == 0 ? (int)m.g.z : std::min(b->halo_min_z, (int)m.g.z);
       b->halo_max_z = std::max(b->halo_max_z, (int)m.g.z);
       continue;
@@ -2753,7 +2755,7 @@ int api_batch_chain(brawl_batch* b, int c, ChainSlot& out) {
   HaloGeom H;
   bool ok;
   make_halo(m.g, H, ok);
-  out.halo_smem = out.halo ? halo_layout(m.g, H).total : 0;
+  out.halo_smem = out.halo ? window_layout(m.g, H).total : 0;
   out.smem_lat_bytes = smem_layout(m.g, true).total;
   out.smem_glob_bytes = smem_layout(m.g, false).total;
   out.use_D = smem_layout(m.g, false).use_D;

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "chain_engine.cuh"
+#include "trial_window.cuh"
 
 namespace brawl {
 
@@ -118,6 +119,31 @@ __host__ __device__ inline HaloLayout halo_layout(const Geom& g, const HaloGeom&
   return L;
 }
 
+// Shared-memory layout of a chain of the windowed kernel (metropolis_halo.cu):
+// the stream's rolling block and words (trial_window.cuh), the tables, the
+// lanes' entries as displacements and the lattice with its halo.
+struct WindowLayout {
+  uint32_t mt, V, ents, sstart, I, ecan, lat, total;
+  int32_t D_off;
+};
+
+__host__ __device__ inline WindowLayout window_layout(const Geom& g, const HaloGeom& H) {
+  WindowLayout L;
+  const uint32_t nsp = (uint32_t)g.ns + 1;
+  const uint32_t nF = nsp * (uint32_t)g.nsh * nsp;
+  const uint32_t nD = nsp * nsp * (uint32_t)g.nsh * nsp;
+  L.mt = 0;
+  L.V = align_up(kRollWords * 4, 16);
+  L.ents = L.V + (uint32_t)(g.ns * g.ns * g.nsh) * 8;
+  L.sstart = L.ents + (uint32_t)g.z * 4;
+  L.I = align_up(L.sstart + (uint32_t)(g.nsh + 1) * 2, 16);
+  L.D_off = (int32_t)nF;
+  L.ecan = L.I + (nF + nD) * 4;
+  L.lat = align_up(L.ecan + 32u * kMaxLaneEntries * 4, 16);
+  L.total = align_up(L.lat + (uint32_t)H.padded, 16);
+  return L;
+}
+
 int lane_entries_for(int max_z);
 
 // Sampling reductions of the annealing loop on the device (sampling.cu).
@@ -151,8 +177,9 @@ uint32_t spec_static_smem(int nc);
 // The halo chains: speculative rounds of nc trials when nc >= 2 and the
 // slots fit beside the dynamic shared memory, the one-trial kernel otherwise.
 // min_z/max_z: the smallest and largest neighbour count of the chains.
-void launch_halo_chains(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int min_z, int max_z,
-                        int nc, int max_optin, cudaStream_t stream);
+// smem_bytes, spec_bytes: the chains' largest window_layout and halo_layout.
+void launch_halo_chains(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, uint32_t spec_bytes, int min_z,
+                        int max_z, int nc, int max_optin, cudaStream_t stream);
 void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int min_z,
                             int max_z, cudaStream_t stream);
 

@@ -20,35 +20,6 @@ struct HaloLat {
   }
 };
 
-// Fixed-point delta for any pair (neighbouring sites included), from the
-// canonical neighbour indices.  Out of line: only pairs within the
-// interaction range come here.
-__device__ __noinline__ int halo_delta_general(const ChainJob* __restrict__ Jg, int ents_off,
-                                               int I_off, int F_off, HaloLat lat, int ax, int ay,
-                                               int az, int ai, int bx, int by, int bz, int bi,
-                                               int sa, int sb, int lane) {
-  extern __shared__ int32_t s_i32[];
-  extern __shared__ uint32_t s_u32[];
-  const Geom g = Jg->g;
-  const bool h = lane >= 16;
-  const int cx = h ? bx : ax, cy = h ? by : ay, cz = h ? bz : az;
-  const int own = h ? bi : ai, other = h ? ai : bi;
-  const int so = h ? sb : sa, sn = h ? sa : sb;
-  const int nsp = g.ns + 1;
-  const int rowN = I_off + F_off + sn * g.nsh * nsp;
-  const int rowO = I_off + F_off + so * g.nsh * nsp;
-  int acc = 0;
-  for (int k = lane & 15; k < g.z; k += 16) {
-    int dx, dy, dz, sh;
-    unpack_entry(s_u32[ents_off / 4 + k], dx, dy, dz, sh);
-    const int ni = neighbour_index(g, cx, cy, cz, dx, dy, dz);
-    const int s_before = lat(ni);
-    const int s_after = ni == other ? so : (ni == own ? sn : s_before);
-    acc += s_i32[rowN + sh * nsp + s_after] - s_i32[rowO + sh * nsp + s_before];
-  }
-  return __reduce_add_sync(kFull, acc);
-}
-
 // The reference-order FP64 decision (see metropolis.cu); returns bit 0
 // accept, bit 1 uniform drawn, bit 2 FP64 libm tier, bit 3 double-double.
 __device__ __noinline__ int halo_exact_decision(const ChainJob* __restrict__ Jg, HaloLat lat,
@@ -160,10 +131,82 @@ __device__ __forceinline__ AcceptThresholds accept_thresholds(uint32_t w, float 
   return T;
 }
 
+// A position's two sites as its lane holds them, one word a site:
+//   bits 0-17  padded index of the site
+//   bit  18    its parity (bcc z & 1, fcc x & 1)
+//   bits 19-22 its species
+//   bits 23-28 per axis (x, y, z) 1: it has an image one period up, 2: one
+//              period down (the cells an accepted swap writes too)
+//   bit  29    (site 1) the pair may be within interaction range
+constexpr int kSiteIndex = (1 << 18) - 1;
+constexpr int kSiteParity = 18, kSiteSpecies = 19, kSiteImages = 23, kSiteNear = 29;
+static_assert(kMaxSpecies < 16, "a species takes four bits");
+
+__device__ __forceinline__ int site_species(int v) { return (v >> kSiteSpecies) & 15; }
+
+__device__ __forceinline__ int image_code(int c, int h, int N) { return c < h ? 1 : (c >= N - h ? 2 : 0); }
+
+// The trial that starts at a position, as far as the stream alone decides it.
+struct WinTrial {
+  int a, b;          // the two sites (species not filled in)
+  int d;             // site 2 - site 1 modulo the periods W: x + W1 (y + W2 z)
+  AcceptThresholds th;
+};
+
+// The sites' doubled-grid coordinates and compact (Y', X') from the
+// position's words.
+struct PairCoords {
+  int ax, ay, az, Ya, Xa, bx, by, bz, Yb, Xb;
+};
+
+__device__ __forceinline__ PairCoords pair_coords(const Geom& g, bool bcc, bool nbr, const uint32_t* w) {
+  PairCoords c;
+  draw_site_halo(g, bcc, w[0], w[1], w[2], c.ax, c.ay, c.az, c.Ya, c.Xa);
+  if (nbr) {
+    draw_nbr(g, w[3], c.ax, c.ay, c.az, c.bx, c.by, c.bz);
+    c.Yb = c.by >> g.ys;
+    c.Xb = c.bx >> 1;
+  } else {
+    draw_site_halo(g, bcc, w[3], w[4], w[5], c.bx, c.by, c.bz, c.Yb, c.Xb);
+  }
+  return c;
+}
+
+__device__ __forceinline__ int pack_site(const HaloGeom& H, bool bcc, int x, int z, int Yc, int Xc) {
+  const int par = bcc ? (z & 1) : (x & 1);
+  const int img = image_code(Xc, H.hx, H.NX) | image_code(Yc, H.hy, H.NY) << 2 | image_code(z, H.hz, H.NZ) << 4;
+  return halo_index(H, z, Yc, Xc) | par << kSiteParity | img << kSiteImages;
+}
+
+__device__ __forceinline__ WinTrial win_decode(const Geom& g, const HaloGeom& H, bool bcc, bool nbr,
+                                               const uint32_t* w, float inv_k, float band_f) {
+  WinTrial T;
+  const PairCoords c = pair_coords(g, bcc, nbr, w);
+  const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
+  int dx = c.bx - c.ax, dy = c.by - c.ay, dz = c.bz - c.az;
+  dx += dx < 0 ? W1 : 0;
+  dy += dy < 0 ? W2 : 0;
+  dz += dz < 0 ? W3 : 0;
+  const bool near = (dx <= H.dmx || dx >= W1 - H.dmx) & (dy <= H.dmy || dy >= W2 - H.dmy) &
+                    (dz <= H.dmz || dz >= W3 - H.dmz);
+  T.d = dx + W1 * (dy + W2 * dz);
+  T.a = pack_site(H, bcc, c.ax, c.az, c.Ya, c.Xa) | (near ? 1 << kSiteNear : 0);
+  T.b = pack_site(H, bcc, c.bx, c.bz, c.Yb, c.Xb);
+  T.th = accept_thresholds(w[nbr ? 4 : 6], inv_k, band_f);
+  return T;
+}
+
+// One warp per chain.  What bounds it: a chain's trials are one dependent
+// sequence, so a trial's latency -- the shuffles that fetch its sites, two
+// shared loads (neighbour species, difference table), a redux.sync, the
+// decision -- times the longest chain's trials is the launch's time; neither
+// issue slots nor shared-memory bandwidth are near their limits.  So all work
+// that the stream alone decides is taken off that sequence (trial_window.cuh):
+// the sites, their species, the thresholds and the image cells are decoded for
+// 32 positions at once, and a trial of two like species is a bit of a mask.
 template <int NJ, bool FULL>
 __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __restrict__ jobs) {
   extern __shared__ __align__(16) unsigned char smem[];
-  extern __shared__ uint32_t s_u32[];
   extern __shared__ int32_t s_i32[];
   extern __shared__ int8_t s_i8[];
   const ChainJob* Jg = jobs + blockIdx.x;
@@ -173,11 +216,10 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   const int lane = threadIdx.x;
   __shared__ unsigned long long s_t_start;  // kept out of registers
   if (lane == 0) s_t_start = global_ns();
-  const HaloLayout L = halo_layout(g, H);
+  const WindowLayout L = window_layout(g, H);
   uint32_t* mt = reinterpret_cast<uint32_t*>(smem + L.mt);
-  uint32_t* tbuf = reinterpret_cast<uint32_t*>(smem + L.tbuf);
-  int32_t* ptab = reinterpret_cast<int32_t*>(smem + L.ptab);
-  int32_t* ctab = reinterpret_cast<int32_t*>(smem + L.ctab);
+  uint32_t* old = mt + kMTN;
+  uint32_t* tw = old + kOldWords;
   double* V = reinterpret_cast<double*>(smem + L.V);
   uint32_t* ents = reinterpret_cast<uint32_t*>(smem + L.ents);
   int16_t* sstart = reinterpret_cast<int16_t*>(smem + L.sstart);
@@ -195,138 +237,184 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   for (int i = lane; i <= g.nsh; i += 32) sstart[i] = Jg->shell_start[i];
   __syncwarp();
   halo_fill(g, H, Jg->lat, lat, lane);
-  const SiteDraw S = make_site_draw(g, H);
-  Ring R;
-  ring_init_sites(mt, tbuf, ptab, ctab, S, (int)rng[kMTN], lane, R);
   HaloPlan<NJ> P;
   make_halo_plan<NJ>(g, H, ents, lane, P);
-  __syncwarp();
-
   const int lat_off = (int)L.lat;
-  const int tb = (int)(L.tbuf / 4);
-  const int pt = (int)(L.ptab / 4), ct = (int)(L.ctab / 4);
   const int I_off = (int)(L.I / 4);
   const int D_abs = I_off + L.D_off;
-  const HaloLat hl = {g.sz, g.sy, H.origin, H.SZ, H.SY, lat_off};
   const bool bcc = g.lattice == kBcc;
-  const int ys = g.ys;
-  const int nbr_swap = Jg->nbr_swap;
+  const bool nbr_swap = Jg->nbr_swap != 0;
+  const bool on_b = lane >= 16;  // lanes 0-15 sum site 1's neighbours, 16-31 site 2's
+  // this lane's entries modulo the periods, as the displacement site 2 -
+  // site 1 that makes the entry's neighbour the other site
+  int32_t* ecan = s_i32 + L.ecan / 4;
+  {
+    const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int k = (lane & 15) + 16 * j;
+      int e = -1;  // no entry: matches no displacement
+      if (k < g.z) {
+        int dx, dy, dz, sh;
+        unpack_entry(ents[k], dx, dy, dz, sh);
+        dx = on_b ? -dx : dx;
+        dy = on_b ? -dy : dy;
+        dz = on_b ? -dz : dz;
+        e = (dx < 0 ? dx + W1 : dx) + W1 * ((dy < 0 ? dy + W2 : dy) + W2 * (dz < 0 ? dz + W3 : dz));
+      }
+      ecan[32 * j + lane] = e;
+    }
+  }
   const int band = Jg->band;
   const float inv_k = 1.0f / Jg->beta_q_l2, band_f = (float)band;
-  const int64_t n_trials = Jg->n_trials;
-  const int n_peek = nbr_swap ? 5 : 7;
   const int n_base = nbr_swap ? 4 : 6;
-  // lanes 0-7 write site 1's cells of an accepted swap, lanes 8-15 site 2's
-  const bool img_b = lane >= 8;
+  const int nt = (int)Jg->n_trials;
+  // lanes 0-7 write site 1's cells of an accepted swap, lanes 8-15 site 2's:
+  // lane c of eight takes the image axes that its bits name
+  const int img_axes = ((lane & 1) ? 3 : 0) | ((lane & 2) ? 12 : 0) | ((lane & 4) ? 48 : 0);
   // 32-bit tallies (a launch runs fewer than 2^31 trials per chain, see
   // launch_metropolis_halo); the words drawn follow from them: n_base per
   // trial plus the uniforms
   unsigned int b_eval = 0, b_acc = 0, b_exact = 0;
   unsigned int c_fp64 = 0, c_cr = 0;
-  const int nt = (int)n_trials;
-  // the uniforms drawn follow from the words consumed: n_base a trial plus
-  // one per uniform, counted through the ring's generated blocks
-  const int avail0 = R.avail;
-  unsigned int gens = 0;
+
+  // ---- the stream -----------------------------------------------------------
+  const int pos0 = (int)rng[kMTN];
+  MtRoll R = {pos0, 0, false};
+#pragma unroll 1
+  for (int i = 0; i < kLookAhead / kWin; ++i) mt_roll(mt, old, tw, R, lane);
+  WinTrial cur, nxt;
+  unsigned int n_win = 0;  // windows begun
+  int tb = -kWin;          // the window's place in the tempered ring
+  unsigned diff = 0;       // positions whose two species differ
+  auto decode_next = [&](int at) {
+    uint32_t w[7];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) w[i] = tw[at + lane + i];
+    nxt = win_decode(g, H, bcc, nbr_swap, w, inv_k, band_f);
+  };
+  decode_next(0);
+  // the next window becomes the current one: its species are read, the one
+  // after it is decoded and 32 more words are generated
+  auto advance = [&]() {
+    cur = nxt;
+    tb = (tb + kWin) & (kTwRing - 1);
+    const int sa = s_i8[lat_off + (cur.a & kSiteIndex)], sb = s_i8[lat_off + (cur.b & kSiteIndex)];
+    decode_next((tb + kWin) & (kTwRing - 1));
+    mt_roll(mt, old, tw, R, lane);
+    cur.a |= sa << kSiteSpecies;
+    cur.b |= sb << kSiteSpecies;
+    diff = __ballot_sync(kFull, sa != sb);
+    ++n_win;
+  };
+  int o = 0;  // the next trial's position in the window
+  advance();
 
   for (int t = 0; t < nt; ++t) {
-    gens += R.avail < n_peek ? 1u : 0u;
-    ring_ensure_sites(mt, tbuf, ptab, ctab, S, R, n_peek, lane);
-    const int wb = tb + R.idx;
-    SitePair p;
-    int Ya, Xa, Yb, Xb, pa, pb, ea = 0, eb = 0;
-    if (nbr_swap) {
-      draw_site_halo(g, bcc, s_u32[wb], s_u32[wb + 1], s_u32[wb + 2], p.ax, p.ay, p.az, Ya, Xa);
-      draw_nbr(g, s_u32[wb + 3], p.ax, p.ay, p.az, p.bx, p.by, p.bz);
-      Yb = p.by >> ys;
-      Xb = p.bx >> 1;
-      pa = H.origin + p.az * H.SZ + Ya * H.SY + Xa;
-      pb = H.origin + p.bz * H.SZ + Yb * H.SY + Xb;
-    } else {
-      // the two sites from the site table: padded index and parity
-      ea = s_i32[pt + R.idx];
-      eb = s_i32[pt + R.idx + 3];
-      pa = ea & kPadMask;
-      pb = eb & kPadMask;
+    if (o >= kWin) {
+      o -= kWin;
+      advance();
     }
-    p.sa = s_i8[lat_off + pa];
-    p.sb = s_i8[lat_off + pb];
+    if (!((diff >> o) & 1u)) {
+      // same species: accepted without an energy evaluation or a draw
+      ++b_acc;
+      o += n_base;
+      continue;
+    }
+    ++b_eval;
+    const int a = __shfl_sync(kFull, cur.a, o), b = __shfl_sync(kFull, cur.b, o);
+    const int acc_below = __shfl_sync(kFull, cur.th.acc_below, o);
+    const int rej_above = __shfl_sync(kFull, cur.th.rej_above, o);
+    const int mine = on_b ? b : a;
+    const int base = lat_off + (mine & kSiteIndex);
+    const bool par = (mine >> kSiteParity) & 1;
+    const int so = site_species(mine), sn = site_species(on_b ? a : b);
+    const int K = g.nsh * nsp;
+    const int rowD = D_abs + (so * nsp + sn) * K;
+    int acc = 0;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int s = s_i8[base + (par ? P.d1[j] : P.d0[j])];
+      const int v = s_i32[rowD + P.shp[j] + s];
+      acc += (FULL || ((P.valid >> j) & 1u)) ? v : 0;
+    }
+    const bool near = (a >> kSiteNear) & 1;
+    if (near) {
+      // an entry whose neighbour is the other site: that site holds our old
+      // species after the swap, not its own
+      const int d = __shfl_sync(kFull, cur.d, o);
+      const int rowN = I_off + sn * K;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        if (ecan[32 * j + lane] == d) acc += s_i32[rowN + P.shp[j] + so] - s_i32[rowN + P.shp[j] + sn];
+    }
+    const int dE = __reduce_add_sync(kFull, acc);
     int consumed = n_base;
-    int accept = 1;  // same species: accepted without an energy evaluation or a draw
-    if (p.sa != p.sb) {
-      ++b_eval;
-      bool par_a, par_b;
-      if (nbr_swap) {
-        par_a = bcc ? (p.az & 1) : (p.ax & 1);
-        par_b = bcc ? (p.bz & 1) : (p.bx & 1);
-      } else {
-        site_coords(s_i32[ct + R.idx], p.ax, p.ay, p.az);
-        site_coords(s_i32[ct + R.idx + 3], p.bx, p.by, p.bz);
-        Ya = p.ay >> ys;
-        Xa = p.ax >> 1;
-        Yb = p.by >> ys;
-        Xb = p.bx >> 1;
-        par_a = ea >> 30;
-        par_b = eb >> 30;
-      }
-      // the fast-tier sum is issued first and the near test fills its loads'
-      // latency; a neighbouring pair (which the fast sum assumes away) takes
-      // the general sum instead
-      int dE = halo_delta<NJ, FULL>(g, lat_off, D_abs, P, pa, pb, par_a, par_b, p.sa, p.sb, lane);
-      const bool near = pair_near_flat(g, H, p.ax, p.ay, p.az, p.bx, p.by, p.bz);
-      if (near) {
-        dE = halo_delta_general(Jg, (int)L.ents, I_off, L.F_off, hl, p.ax, p.ay, p.az,
-                                p.az * g.sz + Ya * g.sy + Xa, p.bx, p.by, p.bz,
-                                p.bz * g.sz + Yb * g.sy + Xb, p.sa, p.sb, lane);
-      }
-      const uint32_t wu = s_u32[wb + n_base];
-      accept = -1;
-      if (dE < -band) {
-        accept = 1;
-      } else if (dE > band) {
-        consumed = n_base + 1;
-        const AcceptThresholds th = accept_thresholds(wu, inv_k, band_f);
-        accept = dE < th.acc_below ? 1 : (dE > th.rej_above ? 0 : -1);
-      }
-      if (accept < 0) {
-        ++b_exact;
-        const int r = near ? halo_exact_decision(Jg, hl, V, ents, sstart, p.ax, p.ay, p.az,
-                                                 p.az * g.sz + Ya * g.sy + Xa, p.bx, p.by, p.bz,
-                                                 p.bz * g.sz + Yb * g.sy + Xb, p.sa, p.sb, lane, wu)
-                           : halo_exact_far(Jg, V, ents, sstart, lat_off, H.SZ, H.SY, bcc, g.ns, g.nsh, pa,
-                                            pb, par_a, par_b, p.sa, p.sb, wu, lane);
-        accept = r & 1;
-        consumed = (r & 2) ? n_base + 1 : n_base;
-        c_fp64 += (r >> 2) & 1;
-        c_cr += (r >> 3) & 1;
-      }
-      if (accept) {
-        const int img = halo_image_index(H, lane, p.az, Ya, Xa, p.bz, Yb, Xb);
-        if (img >= 0) s_i8[lat_off + img] = (int8_t)(img_b ? p.sa : p.sb);
-        __syncwarp();
-      }
+    int accept = -1;
+    if (dE < -band) {
+      accept = 1;
+    } else if (dE > band) {
+      consumed = n_base + 1;
+      accept = dE < acc_below ? 1 : (dE > rej_above ? 0 : -1);
     }
-    b_acc += accept;
-    ring_consume(R, consumed);
+    if (accept < 0) {
+      ++b_exact;
+      const uint32_t* w = tw + tb + o;
+      const uint32_t wu = w[n_base];
+      const int sa = site_species(a), sb = site_species(b);
+      int r;
+      if (near) {
+        const PairCoords c = pair_coords(g, bcc, nbr_swap, w);
+        const HaloLat hl = {g.sz, g.sy, H.origin, H.SZ, H.SY, lat_off};
+        r = halo_exact_decision(Jg, hl, V, ents, sstart, c.ax, c.ay, c.az, c.az * g.sz + c.Ya * g.sy + c.Xa,
+                                c.bx, c.by, c.bz, c.bz * g.sz + c.Yb * g.sy + c.Xb, sa, sb, lane, wu);
+      } else {
+        r = halo_exact_far(Jg, V, ents, sstart, lat_off, H.SZ, H.SY, bcc, g.ns, g.nsh, a & kSiteIndex,
+                           b & kSiteIndex, (a >> kSiteParity) & 1, (b >> kSiteParity) & 1, sa, sb, wu, lane);
+      }
+      accept = r & 1;
+      consumed = (r & 2) ? n_base + 1 : n_base;
+      c_fp64 += (r >> 2) & 1;
+      c_cr += (r >> 3) & 1;
+    }
+    if (accept) {
+      ++b_acc;
+      const int sa = site_species(a), sb = site_species(b);
+      const int ia = a & kSiteIndex, ib = b & kSiteIndex;
+      // the cells of the swapped sites: lane c of eight shifts along its axes
+      const int v = lane < 8 ? a : b;
+      const int code = (v >> kSiteImages) & img_axes;
+      int cell = v & kSiteIndex;
+      cell += (code & 1) ? H.NX : ((code & 2) ? -H.NX : 0);
+      cell += (code & 4) ? H.NY * H.SY : ((code & 8) ? -H.NY * H.SY : 0);
+      cell += (code & 16) ? H.NZ * H.SZ : ((code & 32) ? -H.NZ * H.SZ : 0);
+      // every axis of this lane has an image
+      const int has = code | (code >> 1);
+      if (lane < 16 && (has & 0x15) == (img_axes & 0x15)) s_i8[lat_off + cell] = (int8_t)(lane < 8 ? sb : sa);
+      // the window's positions that name either site
+      const int xa = cur.a & kSiteIndex, xb = cur.b & kSiteIndex;
+      const int flip = (sa ^ sb) << kSiteSpecies;
+      if (xa == ia || xa == ib) cur.a ^= flip;
+      if (xb == ia || xb == ib) cur.b ^= flip;
+      diff = __ballot_sync(kFull, ((cur.a ^ cur.b) >> kSiteSpecies) & 15);
+      __syncwarp();  // the written cells are read by the next trial's lanes
+    }
+    o += consumed;
   }
-  const unsigned long long words =
-      (unsigned long long)(avail0 - R.avail) + (unsigned long long)kMTN * gens;
-  const unsigned long long c_exp = words - (unsigned long long)n_base * (unsigned long long)nt;
-  const unsigned long long c_eval = b_eval, c_acc = b_acc, c_exact = b_exact;
-  const unsigned long long c_draws = (unsigned long long)n_base * (unsigned long long)n_trials + c_exp;
 
   // ---- write back ---------------------------------------------------------
   __syncwarp();
+  const unsigned long long words = (unsigned long long)kWin * (n_win - 1) + (unsigned long long)o;
   halo_store(g, H, lat, Jg->lat, lane);
-  ring_writeback(mt, tbuf, R, Jg->rng, lane);
+  mt_roll_store(mt, old, tw, R, pos0, words, (unsigned long long)kWin * n_win + kLookAhead, Jg->rng, lane);
   if (lane == 0) {
     unsigned long long* c = Jg->counters;
-    c[kCntTrials] += (unsigned long long)n_trials;
-    c[kCntEvaluated] += c_eval;
-    c[kCntDraws] += c_draws;
-    c[kCntAccepted] += c_acc;
-    c[kCntExpTests] += c_exp;
-    c[kCntExactPath] += c_exact;
+    c[kCntTrials] += (unsigned long long)nt;
+    c[kCntEvaluated] += b_eval;
+    c[kCntDraws] += words;
+    c[kCntAccepted] += b_acc;
+    c[kCntExpTests] += words - (unsigned long long)n_base * (unsigned long long)nt;
+    c[kCntExactPath] += b_exact;
     c[kCntExpFp64] += c_fp64;
     c[kCntExpCr] += c_cr;
     if (Jg->t_ns) *Jg->t_ns = global_ns() - s_t_start;

@@ -687,8 +687,7 @@ int launch_anneal(brawl_server* S, Pipe& P) {
         zmin = zmax == 0 ? z : std::min(zmin, z);
         zmax = std::max(zmax, z);
       }
-      launch_halo_chains(P.d_chain + first, count, sm[first], zmin, zmax, kDefaultSpeculation,
-                         S->max_optin, st);
+      launch_metropolis_halo(P.d_chain + first, count, sm[first], zmin, zmax, st);
     }));
   }
   if (n - nh > 0) {
