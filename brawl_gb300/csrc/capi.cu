@@ -9,12 +9,16 @@
 #include <cstdio>
 #include <cstring>
 #include <ctime>
+#include <deque>
+#include <map>
 #include <string>
 #include <vector>
 
 #include "../../include/brawl_gpu.h"
 #include "api_internal.h"
 #include "asro.cuh"
+#include "field_engine.cuh"
+#include "halo_shear.cuh"
 #include "kernels.cuh"
 
 using namespace brawl;
@@ -155,8 +159,82 @@ void make_halo(const Geom& g, HaloGeom& H, bool& ok) {
   H.dmz = dmz;
   if (padded > (int64_t)1 << 30) return;
   H.padded = (int32_t)padded;
+  // sheared layout: rows and planes start where the ones before them end
+  const int PX = H.NX + 2 * hx, PY = H.NY + 2 * hy;
+  H.kSY = PX;
+  H.kSZ = g.lattice == kBcc ? PY * PX + PX + 1 : PY * PX + PY / 2 + 1;
+  H.kx = H.NX;
+  H.ky = H.NY * H.kSY + (g.lattice == kBcc ? 0 : g.n2);
+  H.kz = H.NZ * H.kSZ + (g.lattice == kBcc ? -g.n3 * (H.kSY + 1) : g.n3);
+  H.korg = 0;
+  H.korg = -shear_cell(g.lattice == kBcc, H, -hz, -hy, -hx);
+  H.kcells = shear_cell(g.lattice == kBcc, H, H.NZ + hz - 1, H.NY + hy - 1, H.NX + hx - 1) + 1;
+  // a coordinate is within 2 of W u (u the word as a fraction), so two sites
+  // within dm of each other (modulo W) have words within (dm + 3)/W of each other
+  const int dm[3] = {dmz, dmx, dmy}, W[3] = {2 * g.n3, 2 * g.n1, 2 * g.n2};
+  for (int a = 0; a < 3; ++a) {
+    const double c = std::ceil(std::ldexp((dm[a] + 3.0) / W[a], 32));
+    const bool always = 2.0 * c >= 4294967295.0;
+    H.near_c[a] = always ? 0u : (uint32_t)c;
+    H.near_2c[a] = always ? 0xffffffffu : (uint32_t)(2.0 * c);
+  }
   ok = 2 * hx <= H.NX && 2 * hy <= H.NY && 2 * hz <= H.NZ && dmx <= g.n1 && dmy <= g.n2 &&
        dmz <= g.n3 && smem_layout(g, false).use_D;
+}
+
+// Displacement classes (FieldGeom) of an fcc/bcc lattice: usable when no entry
+// leads back to its own site and no further than the opposite one (offsets
+// within n per axis), and the packed coordinates and indices fit.
+struct FieldTabs {
+  FieldGeom fg;
+  std::vector<uint8_t> dtab, sig;
+};
+
+bool make_field(const Geom& g, FieldTabs& T) {
+  std::memset(&T.fg, 0, sizeof(T.fg));
+  if (g.lattice != kBcc && g.lattice != kFcc) return false;
+  const int n[3] = {g.n1, g.n2, g.n3};
+  const int8_t(*offs)[3] = shell_offsets(g.lattice);
+  int dm[3] = {0, 0, 0};
+  for (int k = 0; k < g.z; ++k)
+    for (int a = 0; a < 3; ++a) dm[a] = std::max(dm[a], std::abs((int)offs[k][a]));
+  for (int a = 0; a < 3; ++a) {
+    if (dm[a] > n[a] || n[a] > 512) return false;
+    T.fg.dm[a] = dm[a];
+    T.fg.side[a] = std::min(2 * dm[a] + 1, 2 * n[a]);
+  }
+  if (g.n_sites > 65535) return false;
+  const int cells = T.fg.side[0] * T.fg.side[1] * T.fg.side[2];
+  auto cell = [&](int sign, const int8_t* d) {
+    int t[3];
+    for (int a = 0; a < 3; ++a) t[a] = (sign * d[a] + dm[a]) % (2 * n[a]);
+    return (t[2] * T.fg.side[1] + t[1]) * T.fg.side[0] + t[0];
+  };
+  // per displacement that is an entry's, the entries of site 1 and of site 2
+  // that meet the other site, by shell
+  std::map<int, std::vector<uint8_t>> met;
+  const int16_t* st = shell_starts(g.lattice);
+  for (int sh = 0; sh < g.nsh; ++sh)
+    for (int k = st[sh]; k < st[sh + 1]; ++k)
+      for (int side = 0; side < 2; ++side) {
+        std::vector<uint8_t>& v = met[cell(side == 0 ? 1 : -1, offs[k])];
+        v.resize(2 * g.nsh, 0);
+        v[2 * sh + side] += 1;
+      }
+  T.dtab.assign(cells, 0);
+  T.sig.assign(2 * g.nsh, 0);  // class 0
+  std::map<std::vector<uint8_t>, int> ids;
+  for (const auto& e : met) {
+    auto it = ids.find(e.second);
+    if (it == ids.end()) {
+      it = ids.emplace(e.second, (int)ids.size() + 1).first;
+      T.sig.insert(T.sig.end(), e.second.begin(), e.second.end());
+    }
+    if (it->second > 255) return false;
+    T.dtab[e.first] = (uint8_t)it->second;
+  }
+  T.fg.n_class = (int)ids.size() + 1;
+  return true;
 }
 
 struct Model {
@@ -351,27 +429,26 @@ struct brawl_batch {
   bool smem_lat = true;
   bool use_D = true;
   int max_z = 0;
-  // chains run by the halo kernel, and its shared-memory size / unrolling
-  std::vector<int> halo;
-  uint32_t halo_smem = 0, spec_smem = 0;  // one trial at a time; speculative rounds
-  int halo_min_z = 0, halo_max_z = 0;
+  // Chains run in shared memory: per chain the kernel it takes by default
+  // (shared_kernel), whether the gather kernel can take it, and what each needs.
+  std::vector<int> kernel, halo;
+  std::vector<uint32_t> gather_smem, field_smem;
   std::vector<ChainJob> staged;          // jobs in launch order
-  int n_halo_launch = 0;
+  int n_shared = 0;                      // of them in shared memory (first)
+  std::vector<LaunchGroup> groups;       // their launches (upload_jobs)
   // classes of the shared-memory chains: chains of one (lattice, n1, n2, n3,
-  // species, shells) share a class; each class is launched on its own
-  // stream with its own shared memory, unrolling and trials per round
-  std::vector<int> cls;                  // per chain: class, or -1 (not a halo chain)
-  std::vector<uint32_t> class_smem, class_spec_smem;
-  std::vector<int> class_z, class_depth;
-  std::vector<int> class_first, class_count;  // in launch order (upload_jobs)
-  std::vector<cudaStream_t> side;        // one per class beyond the first
+  // species, shells) share a class, with its own trials per round and, once
+  // those are chosen, its own launch
+  std::vector<int> cls;                  // per chain: class, or -1 (not in shared memory)
+  std::vector<int> class_depth;
+  std::vector<cudaStream_t> side;        // one per launch beyond the first
   std::vector<cudaEvent_t> ev_side;
   cudaEvent_t ev_fork = nullptr;
   bool per_class = false;                // class depths chosen (brawl_batch_autotune_classes)
   std::vector<unsigned long long> last_counters;
   int device = 0;
   int max_optin = 0;
-  int spec_nc = kDefaultSpeculation;  // trials per speculative round (1: none)
+  int spec_nc = kDefaultSpeculation;     // trials per round of every chain (launch_shared_chains)
   double* d_alro = nullptr;              // ALRO counts: per chain ns x n_sites
   int64_t* d_alro_off = nullptr;
   std::vector<int64_t> alro_off;
@@ -433,39 +510,89 @@ int ensure_grid(brawl_batch* b, size_t bytes) {
   return BRAWL_OK;
 }
 
-// Jobs go to the device in launch order: halo chains first, then the rest,
-// each group by decreasing trial count so the longest chains start first.
+// The kernel that chain c takes at `depth` trials per round.
+int chain_kernel(const brawl_batch* b, int c, int depth) {
+  return depth >= 2 && b->halo[c] ? kSharedGather : b->kernel[c];
+}
+
+// Jobs go to the device in launch order: the shared-memory chains first, group
+// after group, then the rest; each group by decreasing trial count so the
+// longest chains start first, and the group with the longest chain first.  A
+// group is one launch: chains of one kernel and unrolling whose shared memory
+// is alike (a launch gives every block the largest one's, so a group ends
+// where a chain needs under two thirds of its largest), or, once depths are
+// chosen per class, one class.
 int upload_jobs(brawl_batch* b) {
   const int n = (int)b->jobs.size();
-  const int nk = (int)b->class_smem.size();
-  // classes by their longest chain, longest first; chains by trials
-  std::vector<int64_t> class_most(nk, 0);
-  for (int c = 0; c < n; ++c)
-    if (b->cls[c] >= 0) class_most[b->cls[c]] = std::max(class_most[b->cls[c]], b->jobs[c].n_trials);
-  std::vector<int> corder(nk), crank(nk);
-  for (int k = 0; k < nk; ++k) corder[k] = k;
-  std::stable_sort(corder.begin(), corder.end(), [&](int x, int y) { return class_most[x] > class_most[y]; });
-  for (int r = 0; r < nk; ++r) crank[corder[r]] = r;
+  std::vector<int> gid(n, -1);
+  std::vector<LaunchGroup> gs;
+  auto add = [&](int c, int g) {
+    LaunchGroup& G = gs[g];
+    gid[c] = g;
+    G.smem = std::max(G.smem, G.kernel == kSharedField ? b->field_smem[c] : b->gather_smem[c]);
+    G.max_z = std::max(G.max_z, (int)b->models[c].g.z);
+    G.max_sites = std::max(G.max_sites, (int)b->models[c].g.n_sites);
+    G.most = std::max(G.most, b->jobs[c].n_trials);
+    G.count += 1;
+  };
+  if (b->per_class) {
+    gs.assign(b->class_depth.size(), LaunchGroup());
+    for (int c = 0; c < n; ++c) {
+      const int k = b->cls[c];
+      if (k < 0) continue;
+      gs[k].depth = b->class_depth[k];
+      gs[k].kernel = chain_kernel(b, c, gs[k].depth);
+      add(c, k);
+    }
+  } else {
+    std::vector<int> by;
+    for (int c = 0; c < n; ++c)
+      if (b->kernel[c] != kSharedNone) by.push_back(c);
+    auto need = [&](int c) {
+      return chain_kernel(b, c, b->spec_nc) == kSharedField ? b->field_smem[c] : b->gather_smem[c];
+    };
+    std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
+      const int kx = chain_kernel(b, x, b->spec_nc), ky = chain_kernel(b, y, b->spec_nc);
+      if (kx != ky) return kx > ky;
+      const int zx = lane_entries_for(b->models[x].g.z), zy = lane_entries_for(b->models[y].g.z);
+      if (zx != zy) return zx > zy;
+      return need(x) > need(y);
+    });
+    int nj = 0;
+    for (int c : by) {
+      const int k = chain_kernel(b, c, b->spec_nc), z = lane_entries_for(b->models[c].g.z);
+      if (gs.empty() || gs.back().kernel != k || nj != z || 3ull * need(c) < 2ull * gs.back().smem) {
+        gs.push_back(LaunchGroup());
+        gs.back().kernel = k;
+        gs.back().depth = b->spec_nc;
+        nj = z;
+      }
+      add(c, (int)gs.size() - 1);
+    }
+  }
+  std::vector<int> rank(gs.size()), at(gs.size());
+  for (size_t k = 0; k < gs.size(); ++k) at[k] = (int)k;
+  std::stable_sort(at.begin(), at.end(), [&](int x, int y) { return gs[x].most > gs[y].most; });
+  for (size_t r = 0; r < at.size(); ++r) rank[at[r]] = (int)r;
   std::vector<int> order(n);
   for (int c = 0; c < n; ++c) order[c] = c;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-    if (b->halo[x] != b->halo[y]) return b->halo[x] > b->halo[y];
-    if (b->halo[x] && b->per_class && b->cls[x] != b->cls[y]) return crank[b->cls[x]] < crank[b->cls[y]];
+    if ((gid[x] < 0) != (gid[y] < 0)) return gid[x] >= 0;
+    if (gid[x] >= 0 && gid[x] != gid[y]) return rank[gid[x]] < rank[gid[y]];
     return b->jobs[x].n_trials > b->jobs[y].n_trials;
   });
   b->staged.resize(n);
-  b->n_halo_launch = 0;
-  b->class_first.assign(nk, 0);
-  b->class_count.assign(nk, 0);
+  b->n_shared = 0;
   for (int k = 0; k < n; ++k) {
     b->staged[k] = b->jobs[order[k]];
-    b->n_halo_launch += b->halo[order[k]];
-    const int cl = b->cls[order[k]];
-    if (cl >= 0) {
-      if (b->class_count[cl] == 0) b->class_first[cl] = k;
-      b->class_count[cl] += 1;
-    }
+    const int g = gid[order[k]];
+    if (g < 0) continue;
+    if (gs[g].first < 0) gs[g].first = k;
+    b->n_shared += 1;
   }
+  b->groups.clear();
+  for (int g : at)
+    if (gs[g].count > 0) b->groups.push_back(gs[g]);
   CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->staged.data(), n * sizeof(ChainJob),
                            cudaMemcpyHostToDevice, b->stream));
   return BRAWL_OK;
@@ -494,10 +621,10 @@ int set_chain_config(brawl_batch* b, int c, const int8_t* config) {
 int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accepted, bool serial,
                         cudaStream_t stream, bool wait);
 
-// Side streams for the classes beyond the first (created once).
+// Side streams for the launches beyond the first (created once).
 int ensure_side_streams(brawl_batch* b) {
-  const size_t need = b->class_smem.empty() ? 0 : b->class_smem.size() - 1;
-  if (!b->ev_fork) CUDA_TRY(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
+  const size_t need = b->groups.empty() ? 0 : b->groups.size() - 1;
+  if (need > 0 && !b->ev_fork) CUDA_TRY(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
   while (b->side.size() < need) {
     cudaStream_t st;
     cudaEvent_t ev;
@@ -509,28 +636,21 @@ int ensure_side_streams(brawl_batch* b) {
   return BRAWL_OK;
 }
 
-// The shared-memory chains of every class (only = -1) or of class `only`,
-// each class in its own launch with its own shared memory, unrolling and
-// trials per round: the first on `stream`, the others on side streams
-// forked from it and joined back.
-int launch_classes(brawl_batch* b, cudaStream_t stream, int only) {
+// The shared-memory chains, each group in its own launch with its own shared
+// memory, unrolling and trials per round: the first on `stream`, the others on
+// side streams forked from it and joined back.
+int launch_groups(brawl_batch* b, cudaStream_t stream) {
   TRY(ensure_side_streams(b));
-  const int nk = (int)b->class_smem.size();
-  std::vector<int> ks;
-  for (int k = 0; k < nk; ++k)
-    if (b->class_count[k] > 0 && (only < 0 || k == only)) ks.push_back(k);
-  std::sort(ks.begin(), ks.end(), [&](int x, int y) { return b->class_first[x] < b->class_first[y]; });
-  if (ks.size() > 1) CUDA_TRY(cudaEventRecord(b->ev_fork, stream));
-  for (size_t i = 0; i < ks.size(); ++i) {
-    const int k = ks[i];
+  const std::vector<LaunchGroup>& gs = b->groups;
+  if (gs.size() > 1) CUDA_TRY(cudaEventRecord(b->ev_fork, stream));
+  for (size_t i = 0; i < gs.size(); ++i) {
     cudaStream_t st = i == 0 ? stream : b->side[i - 1];
     if (i > 0) CUDA_TRY(cudaStreamWaitEvent(st, b->ev_fork, 0));
-    launch_halo_chains(b->d_jobs + b->class_first[k], b->class_count[k], b->class_smem[k], b->class_spec_smem[k],
-                       b->class_z[k], b->class_z[k], b->class_depth[k], b->max_optin, st);
+    launch_shared_chains(b->d_jobs + gs[i].first, gs[i].count, gs[i], st);
     CUDA_TRY(cudaGetLastError());
     if (i > 0) CUDA_TRY(cudaEventRecord(b->ev_side[i - 1], st));
   }
-  for (size_t i = 1; i < ks.size(); ++i) CUDA_TRY(cudaStreamWaitEvent(stream, b->ev_side[i - 1], 0));
+  for (size_t i = 1; i < gs.size(); ++i) CUDA_TRY(cudaStreamWaitEvent(stream, b->ev_side[i - 1], 0));
   return BRAWL_OK;
 }
 
@@ -564,20 +684,15 @@ int run_metropolis(brawl_batch* b, const int64_t* n_trials, int64_t* accepted, b
   return BRAWL_OK;
 }
 
-// Every chain's uploaded job (b->d_jobs) once on `stream`: the halo chains
-// per class or in one launch, the others in one launch of the plain kernel.
+// Every chain's uploaded job (b->d_jobs) once on `stream`: the shared-memory
+// chains' launches, the others in one launch of the plain kernel.
 int launch_sweep(brawl_batch* b, cudaStream_t stream) {
   const int n = (int)b->jobs.size();
-  const int nh = b->n_halo_launch;
-  if (nh > 0 && b->per_class)
-    TRY(launch_classes(b, stream, -1));
-  else if (nh > 0)
-    launch_halo_chains(b->d_jobs, nh, b->halo_smem, b->spec_smem, b->halo_min_z, b->halo_max_z, b->spec_nc,
-                       b->max_optin, stream);
-  if (n - nh > 0)
-    launch_metropolis(b->d_jobs + nh, n - nh, b->smem_lat, b->use_D, b->smem_bytes, b->max_z, stream);
+  if (n > b->n_shared)
+    launch_metropolis(b->d_jobs + b->n_shared, n - b->n_shared, b->smem_lat, b->use_D, b->smem_bytes, b->max_z,
+                      stream);
   CUDA_TRY(cudaGetLastError());
-  return BRAWL_OK;
+  return launch_groups(b, stream);
 }
 
 int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accepted, bool serial,
@@ -599,14 +714,14 @@ int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accept
   if (!serial) {
     TRY(launch_sweep(b, stream));
   } else {
-    const int nh = b->n_halo_launch;
-    for (int k = 0; k < n; ++k) {
-      if (k < nh)
-        launch_halo_chains(b->d_jobs + k, 1, b->halo_smem, b->spec_smem, b->halo_min_z, b->halo_max_z,
-                           b->spec_nc, b->max_optin, stream);
-      else
-        launch_metropolis(b->d_jobs + k, 1, b->smem_lat, b->use_D, b->smem_bytes, b->max_z,
-                          stream);
+    for (const LaunchGroup& G : b->groups)
+      for (int k = G.first; k < G.first + G.count; ++k) {
+        launch_shared_chains(b->d_jobs + k, 1, G, stream);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(stream_wait(stream));
+      }
+    for (int k = b->n_shared; k < n; ++k) {
+      launch_metropolis(b->d_jobs + k, 1, b->smem_lat, b->use_D, b->smem_bytes, b->max_z, stream);
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(stream_wait(stream));
     }
@@ -650,51 +765,63 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     if (r != BRAWL_OK) return cleanup(fail(r, "chain " + std::to_string(c) + ": " + g_err));
     b->nbr_swap[c] = chains[c].nbr_swap ? 1 : 0;
   }
-  // shared memory: lattice staged when every chain fits
+  // The kernel each chain takes: with the sites' fields in shared memory where
+  // they fit, with the lattice alone there where that fits, else the plain one
+  // (whose lattices are staged when every one of them fits).
   int max_optin = 0;
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
   b->max_optin = max_optin;
   uint32_t need_smem = 0, need_gmem = 0;
-  for (size_t c = 0; c < b->models.size(); ++c) {
-    HaloGeom H;
-    bool ok;
-    make_halo(b->models[c].g, H, ok);
-    if (ok && window_layout(b->models[c].g, H).total <= (uint32_t)max_optin) continue;
-    need_smem = std::max(need_smem, smem_layout(b->models[c].g, true).total);
-    need_gmem = std::max(need_gmem, smem_layout(b->models[c].g, false).total);
-  }
+  b->kernel.assign(n_chains, kSharedNone);
   b->halo.assign(n_chains, 0);
+  b->gather_smem.assign(n_chains, 0);
+  b->field_smem.assign(n_chains, 0);
   b->cls.assign(n_chains, -1);
+  std::vector<const FieldTabs*> tabs(n_chains, nullptr);
+  std::vector<int> class_chain;  // a chain of each class
+  std::deque<FieldTabs> field_tabs;
   for (int c = 0; c < n_chains; ++c) {
     const Model& m = b->models[c];
-    HaloGeom H;
-    bool ok;
-    make_halo(m.g, H, ok);
-    if (ok && window_layout(m.g, H).total <= (uint32_t)max_optin) {
-      b->halo[c] = 1;
-      int k = 0;
-      for (; k < c; ++k) {
-        if (b->cls[k] < 0) continue;
-        const Geom& o = b->models[k].g;
-        if (o.lattice == m.g.lattice && o.n1 == m.g.n1 && o.n2 == m.g.n2 && o.n3 == m.g.n3 &&
-            o.ns == m.g.ns && o.nsh == m.g.nsh)
-          break;
+    int k = 0;
+    for (; k < (int)class_chain.size(); ++k) {
+      const Geom& o = b->models[class_chain[k]].g;
+      if (o.lattice == m.g.lattice && o.n1 == m.g.n1 && o.n2 == m.g.n2 && o.n3 == m.g.n3 && o.ns == m.g.ns &&
+          o.nsh == m.g.nsh)
+        break;
+    }
+    if (k < (int)class_chain.size()) {
+      const int o = class_chain[k];
+      b->kernel[c] = b->kernel[o];
+      b->halo[c] = b->halo[o];
+      b->gather_smem[c] = b->gather_smem[o];
+      b->field_smem[c] = b->field_smem[o];
+      tabs[c] = tabs[o];
+      b->cls[c] = b->kernel[c] != kSharedNone ? k : -1;
+    } else {
+      HaloGeom H;
+      bool ok;
+      make_halo(m.g, H, ok);
+      if (ok && window_layout(m.g, H).total <= (uint32_t)max_optin) {
+        b->halo[c] = 1;
+        b->gather_smem[c] = window_layout(m.g, H).total;
+        b->kernel[c] = kSharedGather;
       }
-      if (k < c) {
-        b->cls[c] = b->cls[k];
-      } else {
-        b->cls[c] = (int)b->class_smem.size();
-        b->class_smem.push_back(window_layout(m.g, H).total);
-        b->class_spec_smem.push_back(halo_layout(m.g, H).total);
-        b->class_z.push_back((int)m.g.z);
+      field_tabs.emplace_back();
+      if (make_field(m.g, field_tabs.back()) &&
+          field_layout(m.g, field_tabs.back().fg).total <= (uint32_t)max_optin) {
+        tabs[c] = &field_tabs.back();
+        b->field_smem[c] = field_layout(m.g, field_tabs.back().fg).total;
+        b->kernel[c] = kSharedField;
+      }
+      if (b->kernel[c] != kSharedNone) {
+        b->cls[c] = (int)class_chain.size();
+        class_chain.push_back(c);
         b->class_depth.push_back(kDefaultSpeculation);
       }
-      b->halo_smem = std::max(b->halo_smem, window_layout(m.g, H).total);
-      b->spec_smem = std::max(b->spec_smem, halo_layout(m.g, H).total);
-      b->halo_min_z = b->halo_max_z == 0 ? (int)m.g.z : std::min(b->halo_min_z, (int)m.g.z);
-      b->halo_max_z = std::max(b->halo_max_z, (int)m.g.z);
-      continue;
     }
+    if (b->kernel[c] != kSharedNone) continue;
+    need_smem = std::max(need_smem, smem_layout(m.g, true).total);
+    need_gmem = std::max(need_gmem, smem_layout(m.g, false).total);
     b->max_z = std::max(b->max_z, (int)m.g.z);
     if (!smem_layout(m.g, false).use_D) b->use_D = false;
   }
@@ -722,6 +849,11 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     off_s[c] = total;
     total = al(total + m.sstart.size() * 2);
   }
+  std::vector<size_t> off_tabs(field_tabs.size());
+  for (size_t k = 0; k < field_tabs.size(); ++k) {
+    off_tabs[k] = total;
+    total = al(total + field_tabs[k].dtab.size() + field_tabs[k].sig.size());
+  }
   const size_t off_jobs = total;
   total = al(total + n_chains * sizeof(ChainJob));
   const size_t off_ejobs = total;
@@ -744,6 +876,13 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     return cleanup(fail(BRAWL_ENOMEM, std::string("arena: ") + cudaGetErrorString(e)));
   }
   std::vector<unsigned char> h(total, 0);
+  for (size_t k = 0; k < field_tabs.size(); ++k) {
+    FieldTabs& t = field_tabs[k];
+    std::copy(t.dtab.begin(), t.dtab.end(), h.begin() + off_tabs[k]);
+    std::copy(t.sig.begin(), t.sig.end(), h.begin() + off_tabs[k] + t.dtab.size());
+    t.fg.dtab = b->arena + off_tabs[k];
+    t.fg.sig = t.fg.dtab + t.dtab.size();
+  }
   for (int c = 0; c < n_chains; ++c) {
     const Model& m = b->models[c];
     mt_seed_host(chains[c].seed, reinterpret_cast<uint32_t*>(&h[off_rng[c]]));
@@ -758,6 +897,7 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
       bool ok;
       make_halo(m.g, j.hg, ok);
       j.halo = b->halo[c];
+      if (tabs[c]) j.fg = tabs[c]->fg;
     }
     j.nbr_swap = b->nbr_swap[c];
     j.band = m.band;
@@ -878,7 +1018,7 @@ int brawl_batch_autotune_classes(brawl_batch* b, const int64_t* n_trials, int ma
   if (!b || !n_trials || max_depth < 1 || max_depth > 4) return fail(BRAWL_EINVAL, "bad argument");
   for (size_t c = 0; c < b->jobs.size(); ++c)
     if (n_trials[c] < 0) return fail(BRAWL_EINVAL, "n_trials < 0");
-  const int nk = (int)b->class_smem.size();
+  const int nk = (int)b->class_depth.size();
   if (n_classes) *n_classes = nk;
   if (nk == 0) return BRAWL_OK;
   cudaStream_t s = b->stream;
@@ -2751,11 +2891,8 @@ int api_batch_chain(brawl_batch* b, int c, ChainSlot& out) {
   if (!b || c < 0 || c >= (int)b->jobs.size()) return fail(BRAWL_EINVAL, "bad chain");
   const Model& m = b->models[c];
   out.job = b->jobs[c];
-  out.halo = b->halo[c];
-  HaloGeom H;
-  bool ok;
-  make_halo(m.g, H, ok);
-  out.halo_smem = out.halo ? window_layout(m.g, H).total : 0;
+  out.kernel = b->kernel[c];
+  out.shared_smem = out.kernel == kSharedField ? b->field_smem[c] : b->gather_smem[c];
   out.smem_lat_bytes = smem_layout(m.g, true).total;
   out.smem_glob_bytes = smem_layout(m.g, false).total;
   out.use_D = smem_layout(m.g, false).use_D;

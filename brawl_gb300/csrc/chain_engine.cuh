@@ -96,13 +96,30 @@ struct HaloGeom {
   int32_t padded;         // padded byte count
   int32_t origin;         // hz*SZ + hy*SY + hx
   int32_t dmx, dmy, dmz;  // largest |offset| component per axis (doubled grid)
+  // Sheared layout of the windowed kernel (halo_shear.cuh): the same cells,
+  // rows of kSY and planes of kSZ shifted so that an entry's index step is
+  // the same at every site.
+  int32_t kSY, kSZ, korg, kcells;
+  int32_t kx, ky, kz;     // index step of one period along each axis
+  uint32_t near_c[3], near_2c[3];  // near test on the words of z, x, y (pair_near_words)
+};
+
+// Displacement classes of an fcc/bcc lattice (see field_engine.cuh): two
+// sites whose displacement is the same number of entries of each shell of
+// either site share a class; class 0 is no entry at all.
+struct FieldGeom {
+  int32_t dm[3], side[3];   // per axis: offsets run to +-dm, values of (d + dm) mod W looked up
+  int32_t n_class;
   int32_t pad;
+  const uint8_t* dtab;      // class by displacement, side[0] fastest
+  const uint8_t* sig;       // per class and shell: entries of site 1, of site 2, that meet the other site
 };
 
 // One chain's work order for a launch.  Plain data, shared with the host.
 struct ChainJob {
   Geom g;
   HaloGeom hg;
+  FieldGeom fg;
   int32_t nbr_swap;
   int32_t band;               // decision band of the fixed-point tier, quanta
   double beta;

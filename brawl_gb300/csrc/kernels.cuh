@@ -119,28 +119,30 @@ __host__ __device__ inline HaloLayout halo_layout(const Geom& g, const HaloGeom&
   return L;
 }
 
-// Shared-memory layout of a chain of the windowed kernel (metropolis_halo.cu):
-// the stream's rolling block and words (trial_window.cuh), the tables, the
-// lanes' entries as displacements and the lattice with its halo.
+// Shared memory of a chain of the windowed kernel (metropolis_halo.cu): the
+// stream's rings (trial_window.cuh), the positions' records and the lattice
+// with its halo (halo_shear.cuh) at fixed places, then the tables.
 struct WindowLayout {
-  uint32_t mt, V, ents, sstart, I, ecan, lat, total;
-  int32_t D_off;
+  static constexpr uint32_t kRec = kRollWords * 4;           // kRecRing records of 16 bytes
+  static constexpr uint32_t kFlags = kRec + kRecRing * 16;   // and a word of flags each
+  static constexpr uint32_t kLat = kFlags + kRecRing * 4;
+  uint32_t V, I, D, edelta, ecan, dnbr, sstart, total;
+  int32_t Dk;  // bytes of D per species pair: nsh + 1 shells (the last all zero) of ns + 1
 };
+static_assert(WindowLayout::kRec % 16 == 0 && WindowLayout::kLat % 16 == 0, "16-byte records, lattice and tables");
 
 __host__ __device__ inline WindowLayout window_layout(const Geom& g, const HaloGeom& H) {
   WindowLayout L;
   const uint32_t nsp = (uint32_t)g.ns + 1;
-  const uint32_t nF = nsp * (uint32_t)g.nsh * nsp;
-  const uint32_t nD = nsp * nsp * (uint32_t)g.nsh * nsp;
-  L.mt = 0;
-  L.V = align_up(kRollWords * 4, 16);
-  L.ents = L.V + (uint32_t)(g.ns * g.ns * g.nsh) * 8;
-  L.sstart = L.ents + (uint32_t)g.z * 4;
-  L.I = align_up(L.sstart + (uint32_t)(g.nsh + 1) * 2, 16);
-  L.D_off = (int32_t)nF;
-  L.ecan = L.I + (nF + nD) * 4;
-  L.lat = align_up(L.ecan + 32u * kMaxLaneEntries * 4, 16);
-  L.total = align_up(L.lat + (uint32_t)H.padded, 16);
+  L.Dk = (int32_t)(((uint32_t)g.nsh + 1) * nsp * 4);
+  L.V = align_up(WindowLayout::kLat + (uint32_t)H.kcells, 16);
+  L.I = L.V + (uint32_t)(g.ns * g.ns * g.nsh) * 8;
+  L.D = L.I + nsp * (uint32_t)g.nsh * nsp * 4;
+  L.edelta = L.D + nsp * nsp * (uint32_t)L.Dk;
+  L.ecan = L.edelta + (uint32_t)g.z * 4;
+  L.dnbr = L.ecan + 2u * (uint32_t)entry_pad(g.z) * 4;
+  L.sstart = L.dnbr + 12 * 4;
+  L.total = align_up(L.sstart + (uint32_t)(g.nsh + 1) * 2, 16);
   return L;
 }
 
@@ -163,25 +165,38 @@ void launch_asro_stats(int n, int m, const double* d_rho_sum, double n_save, dou
 // kernels already running on the device).
 void preload_metropolis_kernels();
 void preload_halo_kernels();
+void preload_field_kernels();
 void preload_ns_kernels();
 void preload_wl_kernels();
 void preload_lattice_kernels();
 
-// Metropolis swap trials for chains staged with a halo (fcc/bcc that fit).
-// Speculative rounds of nc (2-4) trials per chain, nc(nc+1)/2 warps per CTA
-// (metropolis_spec.cu); spec_static_smem is the static shared memory the
-// kernel adds to smem_bytes.
-void launch_metropolis_spec(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int nc,
+// Kernels of the chains that run in shared memory (fcc/bcc).
+enum shared_kernel : int {
+  kSharedNone = 0,
+  kSharedGather = 1,  // the lattice there, neighbours' sums gathered (metropolis_halo.cu)
+  kSharedField = 2,   // the sites' fields there too (metropolis_field.cu)
+};
+
+// One launch of them: `count` chains from `first` in launch order, the largest
+// shared memory, neighbour count and lattice among them, and the trials per
+// round of the gather kernel (1: kGatherDefault).
+struct LaunchGroup {
+  int kernel = kSharedNone, depth = 1, first = -1, count = 0;
+  uint32_t smem = 0;
+  int max_z = 0, max_sites = 0;
+  int64_t most = 0;  // the most trials of one chain
+};
+constexpr int kGatherDefault = 4;
+void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int depth,
                             cudaStream_t stream);
-uint32_t spec_static_smem(int nc);
-// The halo chains: speculative rounds of nc trials when nc >= 2 and the
-// slots fit beside the dynamic shared memory, the one-trial kernel otherwise.
-// min_z/max_z: the smallest and largest neighbour count of the chains.
-// smem_bytes, spec_bytes: the chains' largest window_layout and halo_layout.
-void launch_halo_chains(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, uint32_t spec_bytes, int min_z,
-                        int max_z, int nc, int max_optin, cudaStream_t stream);
-void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int min_z,
-                            int max_z, cudaStream_t stream);
+void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_sites, int max_z,
+                             cudaStream_t stream);
+inline void launch_shared_chains(const ChainJob* d_jobs, int n_jobs, const LaunchGroup& G, cudaStream_t stream) {
+  if (G.kernel == kSharedField)
+    launch_metropolis_field(d_jobs, n_jobs, G.smem, G.max_sites, G.max_z, stream);
+  else
+    launch_metropolis_halo(d_jobs, n_jobs, G.smem, G.max_z, G.depth, stream);
+}
 
 // Metropolis swap trials, one warp (CTA) per chain; max_z is the largest
 // neighbour count in the batch (it selects the unrolling of the fast tier).

@@ -298,10 +298,13 @@ struct Group {
   int first, count;
 };
 
-std::vector<Group> smem_groups(const std::vector<uint32_t>& smem) {
+std::vector<Group> smem_groups(const std::vector<uint32_t>& smem, const std::vector<int>* kind = nullptr) {
   std::vector<Group> gs;
+  const int most = kind ? kSide - 1 : kSide;  // room for the change of kind
   for (int i = 0; i < (int)smem.size(); ++i) {
-    if (gs.empty() || ((int)gs.size() <= kSide && 3ull * smem[i] < 2ull * smem[gs.back().first]))
+    const bool other = kind && i > 0 && (*kind)[i] != (*kind)[i - 1];
+    if (gs.empty() || other ||
+        ((int)gs.size() <= most && 3ull * smem[i] < 2ull * smem[gs.back().first]))
       gs.push_back({i, 0});
     gs.back().count += 1;
   }
@@ -649,11 +652,12 @@ int launch_anneal(brawl_server* S, Pipe& P) {
   SV_TRY(grow(P.d_tns, P.tns_cap, std::max<size_t>(P.jobs.size(), 1), P.s));
   const double t_round = round_ns(S, P.jobs);
   std::stable_sort(P.jobs.begin(), P.jobs.end(), [](const JobP& a, const JobP& b) {
-    return a->slot.halo_smem > b->slot.halo_smem;
+    if (a->slot.kernel != b->slot.kernel) return a->slot.kernel > b->slot.kernel;
+    return a->slot.shared_smem > b->slot.shared_smem;
   });
   for (int pass = 0; pass < 2; ++pass)
     for (auto& j : P.jobs) {
-      if (j->slot.halo != (pass == 0 ? 1 : 0)) continue;
+      if ((j->slot.kernel != kSharedNone) != (pass == 0)) continue;
       j->quantum = next_quantum(t_round, *j, j->stage_left, kFirstTrials, S->o.max_trials);
       ChainJob c = j->slot.job;
       c.n_trials = j->quantum;
@@ -673,21 +677,26 @@ int launch_anneal(brawl_server* S, Pipe& P) {
       }
     }
   int nh = 0;
-  for (auto& j : P.launched) nh += j->slot.halo;
+  for (auto& j : P.launched) nh += j->slot.kernel != kSharedNone;
   const int n = (int)staged.size();
   SV_TRY(grow(P.d_chain, P.chain_cap, (size_t)n, P.s));
   SV_TRY(stage_copy(P, P.d_chain, staged.data(), n * sizeof(ChainJob)));
   if (nh > 0) {
     std::vector<uint32_t> sm(nh);
-    for (int k = 0; k < nh; ++k) sm[k] = P.launched[k]->slot.halo_smem;
-    SV_TRY(launch_groups(P, smem_groups(sm), [&](int first, int count, cudaStream_t st) {
-      int zmin = 0, zmax = 0;
+    std::vector<int> kind(nh);
+    for (int k = 0; k < nh; ++k) {
+      sm[k] = P.launched[k]->slot.shared_smem;
+      kind[k] = P.launched[k]->slot.kernel;
+    }
+    SV_TRY(launch_groups(P, smem_groups(sm, &kind), [&](int first, int count, cudaStream_t st) {
+      LaunchGroup G;
+      G.kernel = kind[first];
+      G.smem = sm[first];
       for (int k = first; k < first + count; ++k) {
-        const int z = staged[k].g.z;
-        zmin = zmax == 0 ? z : std::min(zmin, z);
-        zmax = std::max(zmax, z);
+        G.max_z = std::max(G.max_z, (int)staged[k].g.z);
+        G.max_sites = std::max(G.max_sites, (int)staged[k].g.n_sites);
       }
-      launch_metropolis_halo(P.d_chain + first, count, sm[first], zmin, zmax, st);
+      launch_shared_chains(P.d_chain + first, count, G, st);
     }));
   }
   if (n - nh > 0) {
@@ -1197,6 +1206,7 @@ int brawl_serve_create(const brawl_server_opts* opts, brawl_server** out) {
   // a variant would otherwise wait for every round in flight
   preload_metropolis_kernels();
   preload_halo_kernels();
+  preload_field_kernels();
   preload_ns_kernels();
   preload_wl_kernels();
   preload_lattice_kernels();
