@@ -25,8 +25,8 @@ int api_make_geom(const brawl_setup& s, Geom& g);
 // job (site_energy / out / site_offset left for the caller).
 struct ChainSlot {
   ChainJob job;
-  int kernel;              // shared_kernel
-  uint32_t shared_smem;    // its shared memory
+  int kernel;              // shared_kernel: with fields where it can
+  uint32_t gather_smem, field_smem;  // shared memory of the two (0: it cannot)
   uint32_t smem_lat_bytes, smem_glob_bytes;
   bool use_D;
   EnergyJob energy;

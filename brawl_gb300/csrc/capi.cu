@@ -121,6 +121,19 @@ int make_geom(const brawl_setup& s, Geom& g) {
   return BRAWL_OK;
 }
 
+// words_near's constants (of the words of z, x, y) for offsets of up to dm:
+// a coordinate is within 2 of W u (u the word as a fraction), so two sites within
+// dm of each other (modulo W) have words within (dm + 3)/W of each other.
+void words_within(const Geom& g, int dmx, int dmy, int dmz, uint32_t c[3], uint32_t c2[3]) {
+  const int dm[3] = {dmz, dmx, dmy}, W[3] = {2 * g.n3, 2 * g.n1, 2 * g.n2};
+  for (int a = 0; a < 3; ++a) {
+    const double w = std::ceil(std::ldexp((dm[a] + 3.0) / W[a], 32));
+    const bool always = 2.0 * w >= 4294967295.0;
+    c[a] = always ? 0u : (uint32_t)w;
+    c2[a] = always ? 0xffffffffu : (uint32_t)(2.0 * w);
+  }
+}
+
 // Halo staging of an fcc/bcc lattice (halo_engine.cuh): halo widths from the
 // largest compact-index step of any entry at either parity; usable when the
 // images of a site are unique (2h <= N per axis), the pair-distance test is
@@ -169,15 +182,7 @@ void make_halo(const Geom& g, HaloGeom& H, bool& ok) {
   H.korg = 0;
   H.korg = -shear_cell(g.lattice == kBcc, H, -hz, -hy, -hx);
   H.kcells = shear_cell(g.lattice == kBcc, H, H.NZ + hz - 1, H.NY + hy - 1, H.NX + hx - 1) + 1;
-  // a coordinate is within 2 of W u (u the word as a fraction), so two sites
-  // within dm of each other (modulo W) have words within (dm + 3)/W of each other
-  const int dm[3] = {dmz, dmx, dmy}, W[3] = {2 * g.n3, 2 * g.n1, 2 * g.n2};
-  for (int a = 0; a < 3; ++a) {
-    const double c = std::ceil(std::ldexp((dm[a] + 3.0) / W[a], 32));
-    const bool always = 2.0 * c >= 4294967295.0;
-    H.near_c[a] = always ? 0u : (uint32_t)c;
-    H.near_2c[a] = always ? 0xffffffffu : (uint32_t)(2.0 * c);
-  }
+  words_within(g, dmx, dmy, dmz, H.near_c, H.near_2c);
   ok = 2 * hx <= H.NX && 2 * hy <= H.NY && 2 * hz <= H.NZ && dmx <= g.n1 && dmy <= g.n2 &&
        dmz <= g.n3 && smem_layout(g, false).use_D;
 }
@@ -204,6 +209,7 @@ bool make_field(const Geom& g, FieldTabs& T) {
     T.fg.side[a] = std::min(2 * dm[a] + 1, 2 * n[a]);
   }
   if (g.n_sites > 65535) return false;
+  words_within(g, 2 * dm[0], 2 * dm[1], 2 * dm[2], T.fg.both_c, T.fg.both_2c);
   const int cells = T.fg.side[0] * T.fg.side[1] * T.fg.side[2];
   auto cell = [&](int sign, const int8_t* d) {
     int t[3];
@@ -221,6 +227,12 @@ bool make_field(const Geom& g, FieldTabs& T) {
         v.resize(2 * g.nsh, 0);
         v[2 * sh + side] += 1;
       }
+  T.fg.distinct = 1;
+  for (const auto& e : met) {
+    int once = 0;
+    for (int sh = 0; sh < g.nsh; ++sh) once += e.second[2 * sh];
+    if (once > 1) T.fg.distinct = 0;
+  }
   T.dtab.assign(cells, 0);
   T.sig.assign(2 * g.nsh, 0);  // class 0
   std::map<std::vector<uint8_t>, int> ids;
@@ -531,7 +543,7 @@ int upload_jobs(brawl_batch* b) {
     gid[c] = g;
     G.smem = std::max(G.smem, G.kernel == kSharedField ? b->field_smem[c] : b->gather_smem[c]);
     G.max_z = std::max(G.max_z, (int)b->models[c].g.z);
-    G.max_sites = std::max(G.max_sites, (int)b->models[c].g.n_sites);
+    G.ns = b->models[c].g.ns;
     G.most = std::max(G.most, b->jobs[c].n_trials);
     G.count += 1;
   };
@@ -551,16 +563,22 @@ int upload_jobs(brawl_batch* b) {
     auto need = [&](int c) {
       return chain_kernel(b, c, b->spec_nc) == kSharedField ? b->field_smem[c] : b->gather_smem[c];
     };
+    // the unrolling, and with fields their number per site
+    auto variant = [&](int c) {
+      const Geom& g = b->models[c].g;
+      return chain_kernel(b, c, b->spec_nc) == kSharedField ? 16 * ((g.z + kFieldHalf - 1) / kFieldHalf) + field_variant(g.ns)
+                                                           : lane_entries_for(g.z);
+    };
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
       const int kx = chain_kernel(b, x, b->spec_nc), ky = chain_kernel(b, y, b->spec_nc);
       if (kx != ky) return kx > ky;
-      const int zx = lane_entries_for(b->models[x].g.z), zy = lane_entries_for(b->models[y].g.z);
-      if (zx != zy) return zx > zy;
+      const int vx = variant(x), vy = variant(y);
+      if (vx != vy) return vx > vy;
       return need(x) > need(y);
     });
     int nj = 0;
     for (int c : by) {
-      const int k = chain_kernel(b, c, b->spec_nc), z = lane_entries_for(b->models[c].g.z);
+      const int k = chain_kernel(b, c, b->spec_nc), z = variant(c);
       if (gs.empty() || gs.back().kernel != k || nj != z || 3ull * need(c) < 2ull * gs.back().smem) {
         gs.push_back(LaunchGroup());
         gs.back().kernel = k;
@@ -778,25 +796,25 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
   b->field_smem.assign(n_chains, 0);
   b->cls.assign(n_chains, -1);
   std::vector<const FieldTabs*> tabs(n_chains, nullptr);
-  std::vector<int> class_chain;  // a chain of each class
+  std::vector<int> kind_chain;  // a chain of each (lattice, n1, n2, n3, species, shells)
+  std::vector<int> kind_class;  // and the class of those in shared memory, or -1
   std::deque<FieldTabs> field_tabs;
   for (int c = 0; c < n_chains; ++c) {
     const Model& m = b->models[c];
-    int k = 0;
-    for (; k < (int)class_chain.size(); ++k) {
-      const Geom& o = b->models[class_chain[k]].g;
+    size_t k = 0;
+    for (; k < kind_chain.size(); ++k) {
+      const Geom& o = b->models[kind_chain[k]].g;
       if (o.lattice == m.g.lattice && o.n1 == m.g.n1 && o.n2 == m.g.n2 && o.n3 == m.g.n3 && o.ns == m.g.ns &&
           o.nsh == m.g.nsh)
         break;
     }
-    if (k < (int)class_chain.size()) {
-      const int o = class_chain[k];
+    if (k < kind_chain.size()) {
+      const int o = kind_chain[k];
       b->kernel[c] = b->kernel[o];
       b->halo[c] = b->halo[o];
       b->gather_smem[c] = b->gather_smem[o];
       b->field_smem[c] = b->field_smem[o];
       tabs[c] = tabs[o];
-      b->cls[c] = b->kernel[c] != kSharedNone ? k : -1;
     } else {
       HaloGeom H;
       bool ok;
@@ -806,24 +824,37 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
         b->gather_smem[c] = window_layout(m.g, H).total;
         b->kernel[c] = kSharedGather;
       }
-      field_tabs.emplace_back();
-      if (make_field(m.g, field_tabs.back()) &&
-          field_layout(m.g, field_tabs.back().fg).total <= (uint32_t)max_optin) {
+      FieldTabs T;
+      if (make_field(m.g, T) && field_layout(m.g, T.fg).total <= (uint32_t)max_optin) {
+        field_tabs.push_back(std::move(T));
         tabs[c] = &field_tabs.back();
-        b->field_smem[c] = field_layout(m.g, field_tabs.back().fg).total;
+        b->field_smem[c] = field_layout(m.g, tabs[c]->fg).total;
         b->kernel[c] = kSharedField;
       }
+      kind_chain.push_back(c);
+      kind_class.push_back(-1);
       if (b->kernel[c] != kSharedNone) {
-        b->cls[c] = (int)class_chain.size();
-        class_chain.push_back(c);
+        kind_class[k] = (int)b->class_depth.size();
         b->class_depth.push_back(kDefaultSpeculation);
       }
     }
+    b->cls[c] = kind_class[k];
     if (b->kernel[c] != kSharedNone) continue;
     need_smem = std::max(need_smem, smem_layout(m.g, true).total);
     need_gmem = std::max(need_gmem, smem_layout(m.g, false).total);
     b->max_z = std::max(b->max_z, (int)m.g.z);
     if (!smem_layout(m.g, false).use_D) b->use_D = false;
+  }
+  {
+    // many chains: the gather kernel keeps more of them on an SM
+    int n_sm = 0;
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, b->device);
+    double load = 0.0;
+    for (int c = 0; c < n_chains; ++c)
+      if (b->kernel[c] == kSharedField) load += field_load(b->field_smem[c]);
+    if (!fields_pay(load, n_sm))
+      for (int c = 0; c < n_chains; ++c)
+        if (b->halo[c]) b->kernel[c] = kSharedGather;
   }
   b->smem_lat = need_smem <= (uint32_t)max_optin;
   b->smem_bytes = b->smem_lat ? need_smem : need_gmem;
@@ -2891,8 +2922,9 @@ int api_batch_chain(brawl_batch* b, int c, ChainSlot& out) {
   if (!b || c < 0 || c >= (int)b->jobs.size()) return fail(BRAWL_EINVAL, "bad chain");
   const Model& m = b->models[c];
   out.job = b->jobs[c];
-  out.kernel = b->kernel[c];
-  out.shared_smem = out.kernel == kSharedField ? b->field_smem[c] : b->gather_smem[c];
+  out.kernel = b->field_smem[c] > 0 ? kSharedField : b->kernel[c];
+  out.gather_smem = b->gather_smem[c];
+  out.field_smem = b->field_smem[c];
   out.smem_lat_bytes = smem_layout(m.g, true).total;
   out.smem_glob_bytes = smem_layout(m.g, false).total;
   out.use_D = smem_layout(m.g, false).use_D;

@@ -101,7 +101,7 @@ struct HaloGeom {
   // the same at every site.
   int32_t kSY, kSZ, korg, kcells;
   int32_t kx, ky, kz;     // index step of one period along each axis
-  uint32_t near_c[3], near_2c[3];  // near test on the words of z, x, y (pair_near_words)
+  uint32_t near_c[3], near_2c[3];  // near test on the words of z, x, y (words_near)
 };
 
 // Displacement classes of an fcc/bcc lattice (see field_engine.cuh): two
@@ -110,7 +110,8 @@ struct HaloGeom {
 struct FieldGeom {
   int32_t dm[3], side[3];   // per axis: offsets run to +-dm, values of (d + dm) mod W looked up
   int32_t n_class;
-  int32_t pad;
+  int32_t distinct;         // no two entries lead to the same site
+  uint32_t both_c[3], both_2c[3];  // the words' test of HaloGeom::near_c for twice the offsets
   const uint8_t* dtab;      // class by displacement, side[0] fastest
   const uint8_t* sig;       // per class and shell: entries of site 1, of site 2, that meet the other site
 };

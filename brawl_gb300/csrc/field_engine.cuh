@@ -22,27 +22,44 @@
 namespace brawl {
 
 // A position's static record (the trial that would start there):
-//   at   coordinates of site 1, of site 2 (x | y << 10 | z << 20), index of
-//        site 1 | index of site 2 << 16, displacement class (0: no entry)
-//   th   the larger of rej_above and the band; acc_below
-constexpr int kFieldRing = 4 * kWin;  // positions held: two halves of two windows
+//   A  index of site 1, of site 2; byte address of the neighbours' constants
+//      of its displacement class; the larger of rej_above and the band
+//   B  coordinates of site 1, of site 2 (x | y << 10 | z << 20); acc_below;
+//      whether a site may have both as neighbours
+// Four warps make them, a window each of a part of four; two parts are held.
+constexpr int kFieldMakers = 4;
+constexpr int kFieldPart = kFieldMakers * kWin, kFieldRing = 2 * kFieldPart;
+// Words generated before the first part, and ahead of the stream at most (the
+// stream in a part, the next one made, the words of one more).
+constexpr int kFieldAhead = 5 * kWin;
+using FieldWords = StreamRing<kFieldAhead + 2 * kFieldPart>;
 
 // Shared memory of a chain with fields: the stream's rings, the records, then
 // V, the update table U, the neighbours' constants C, W and F, the entries,
 // the axis tables, the displacement classes, the exact tier's codes, the
 // fields and the compact lattice.
 struct FieldLayout {
-  static constexpr uint32_t kAt = kRollWords * 4;
-  static constexpr uint32_t kTh = kAt + kFieldRing * 16;
-  static constexpr uint32_t kV = kTh + kFieldRing * 8;
+  static constexpr uint32_t kA = FieldWords::kWords * 4;
+  static constexpr uint32_t kB = kA + kFieldRing * 16;
+  static constexpr uint32_t kV = kB + kFieldRing * 16;
   uint32_t U, C, W, F, ents, tabs[3], sstart, dtab, codes, g, lat, total;
 };
-static_assert(FieldLayout::kAt % 16 == 0 && FieldLayout::kV % 16 == 0, "16-byte records, tables of doubles");
+static_assert(FieldLayout::kA % 16 == 0 && FieldLayout::kV % 16 == 0, "16-byte records, tables of doubles");
+
+// Fields a site keeps: ns - 1, three padded to four so that a site's are read
+// and written as one vector.
+__host__ __device__ __forceinline__ int field_stride(int ns) { return ns == 4 ? 4 : ns - 1; }
+
+// The kernel's variant: one, two or four fields a site as a vector, or 0.
+__host__ __device__ __forceinline__ int field_variant(int ns) {
+  const int r = field_stride(ns);
+  return r == 1 || r == 2 || r == 4 ? r : 0;
+}
 
 __host__ __device__ inline FieldLayout field_layout(const Geom& g, const FieldGeom& f) {
   FieldLayout L;
-  const uint32_t ns = (uint32_t)g.ns, r = ns - 1, nsh = (uint32_t)g.nsh;
-  L.U = FieldLayout::kV + ns * ns * nsh * 8;
+  const uint32_t ns = (uint32_t)g.ns, r = (uint32_t)field_stride(g.ns), nsh = (uint32_t)g.nsh;
+  L.U = align_up(FieldLayout::kV + ns * ns * nsh * 8, 16);
   L.C = L.U + ns * ns * nsh * r * 4;
   L.W = L.C + (uint32_t)f.n_class * ns * ns * 4;
   L.F = L.W + nsh * ns * r * 4;
@@ -59,11 +76,12 @@ __host__ __device__ inline FieldLayout field_layout(const Geom& g, const FieldGe
   return L;
 }
 
-// Tables, lattice and fields from the job, by all the block's threads.  Ends
-// with a __syncthreads.
+// Tables, lattice (4 (species - 1) a site: a byte offset into rows by species)
+// and fields from the job, by all the block's threads.  Ends with a
+// __syncthreads.
 __device__ inline void field_stage(const ChainJob& J, const Geom& g, const FieldLayout& L, unsigned char* smem, int tid,
                                    int nt) {
-  const int ns = g.ns, nsp = ns + 1, r = ns - 1, nsh = g.nsh;
+  const int ns = g.ns, nsp = ns + 1, r = field_stride(ns), nsh = g.nsh;
   double* V = reinterpret_cast<double*>(smem + FieldLayout::kV);
   int32_t* U = reinterpret_cast<int32_t*>(smem + L.U);
   int32_t* C = reinterpret_cast<int32_t*>(smem + L.C);
@@ -73,7 +91,7 @@ __device__ inline void field_stage(const ChainJob& J, const Geom& g, const Field
   int16_t* sstart = reinterpret_cast<int16_t*>(smem + L.sstart);
   uint8_t* dtab = smem + L.dtab;
   int32_t* G = reinterpret_cast<int32_t*>(smem + L.g);
-  int8_t* lat = reinterpret_cast<int8_t*>(smem + L.lat);
+  uint8_t* lat = smem + L.lat;
   const FieldGeom& f = J.fg;
   for (int i = tid; i < ns * ns * nsh; i += nt) V[i] = J.V[i];
   for (int i = tid; i < nsp * nsh * nsp; i += nt) F[i] = J.F[i];
@@ -92,23 +110,24 @@ __device__ inline void field_stage(const ChainJob& J, const Geom& g, const Field
     }
   }
   {
-    const int n16 = g.n_sites >> 4;
-    const uint4* src = reinterpret_cast<const uint4*>(J.lat);
-    uint4* dst = reinterpret_cast<uint4*>(lat);
-    for (int i = tid; i < n16; i += nt) dst[i] = src[i];
-    for (int i = (n16 << 4) + tid; i < g.n_sites; i += nt) lat[i] = J.lat[i];
+    // 4 (species - 1) a site, four sites at a time
+    const int n4 = g.n_sites >> 2;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(J.lat);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(smem + L.lat);
+    for (int i = tid; i < n4; i += nt) dst[i] = (src[i] - 0x01010101u) << 2;
+    for (int i = (n4 << 2) + tid; i < g.n_sites; i += nt) lat[i] = (uint8_t)((J.lat[i] - 1) << 2);
   }
   __syncthreads();
   auto Fv = [&](int a, int sh, int b) { return F[(a * nsh + sh) * nsp + b]; };
   // W[sh][s - 1][s2 - 2]: a neighbour of species s in shell sh, to g(., s2)
   for (int i = tid; i < nsh * ns * r; i += nt) {
     const int s2 = i % r + 2, s = (i / r) % ns + 1, sh = i / (r * ns);
-    W[i] = Fv(s2, sh, s) - Fv(1, sh, s);
+    W[i] = s2 <= ns ? Fv(s2, sh, s) - Fv(1, sh, s) : 0;
   }
   // U[old - 1][new - 1][sh][s2 - 2]: a neighbour changing from old to new
   for (int i = tid; i < ns * ns * nsh * r; i += nt) {
     const int s2 = i % r + 2, sh = (i / r) % nsh, sn = (i / (r * nsh)) % ns + 1, so = i / (r * nsh * ns) + 1;
-    U[i] = (Fv(s2, sh, sn) - Fv(1, sh, sn)) - (Fv(s2, sh, so) - Fv(1, sh, so));
+    U[i] = s2 <= ns ? (Fv(s2, sh, sn) - Fv(1, sh, sn)) - (Fv(s2, sh, so) - Fv(1, sh, so)) : 0;
   }
   // C[class][sa - 1][sb - 1]: an entry that meets the other site finds our old
   // species there after the swap, not the other site's own
@@ -123,30 +142,42 @@ __device__ inline void field_stage(const ChainJob& J, const Geom& g, const Field
     C[i] = v;
   }
   __syncthreads();
-  // The fields: per shell the neighbours are counted by species (a byte each
-  // of a 64-bit word, eight species at a time), then weighted.
-  const int32_t* tx = reinterpret_cast<const int32_t*>(smem + L.tabs[0]) + kHalo;
-  const int32_t* ty = reinterpret_cast<const int32_t*>(smem + L.tabs[1]) + kHalo;
-  const int32_t* tz = reinterpret_cast<const int32_t*>(smem + L.tabs[2]) + kHalo;
+  // The fields: per shell the neighbours are counted by species (six bits each,
+  // a shell has at most 48; five species at a time), then weighted.
+  const unsigned char* tx = smem + L.tabs[0] + kHalo * 4;
+  const unsigned char* ty = smem + L.tabs[1] + kHalo * 4;
+  const unsigned char* tz = smem + L.tabs[2] + kHalo * 4;
   for (int i = tid; i < g.n_sites; i += nt) {
     int x, y, z;
     decode_site(g, i, x, y, z);
+    const unsigned char *bx = tx + 4 * x, *by = ty + 4 * y, *bz = tz + 4 * z;
     for (int sh = 0; sh < nsh; ++sh) {
-      for (int s0 = 0; s0 < ns; s0 += 8) {
-        unsigned long long n8 = 0;
-        const int k1 = sstart[sh + 1];
-#pragma unroll 4
-        for (int k = sstart[sh]; k < k1; ++k) {
-          int dx, dy, dz, s_;
-          unpack_entry(ents[k], dx, dy, dz, s_);
-          const int s = lat[tx[x + dx] + ty[y + dy] + tz[z + dz]] - 1 - s0;
-          n8 += (unsigned)s < 8u ? 1ull << (8 * s) : 0ull;
+      const int k0 = sstart[sh], k1 = sstart[sh + 1];
+      for (int s0 = 0; s0 < ns; s0 += 5) {
+        unsigned n5 = 0;
+        auto count = [&](int k) {
+          const uint32_t e = ents[k];
+          const int dx = (int)(e << 24) >> 24, dy = (int)(e << 16) >> 24, dz = (int)(e << 8) >> 24;
+          const int at = *reinterpret_cast<const int32_t*>(bx + 4 * dx) + *reinterpret_cast<const int32_t*>(by + 4 * dy) +
+                         *reinterpret_cast<const int32_t*>(bz + 4 * dz);
+          const unsigned s = (unsigned)((lat[at] >> 2) - s0);
+          return s < 5u ? 1u << (6u * s) : 0u;
+        };
+        int k = k0;
+        for (; k + 6 <= k1; k += 6) {
+          unsigned c[6];
+#pragma unroll
+          for (int u = 0; u < 6; ++u) c[u] = count(k + u);
+#pragma unroll
+          for (int u = 0; u < 6; ++u) n5 += c[u];
         }
+        for (; k < k1; ++k) n5 += count(k);
         for (int p = 0; p < r; ++p) {
-          int v = sh == 0 && s0 == 0 ? 0 : G[p * g.n_sites + i];
-          for (int s = s0; s < min(ns, s0 + 8); ++s)
-            v += (int)((n8 >> (8 * (s - s0))) & 0xffull) * W[(sh * ns + s) * r + p];
-          G[p * g.n_sites + i] = v;
+          int v = sh == 0 && s0 == 0 ? 0 : G[i * r + p];
+          const int32_t* w = W + (sh * ns + s0) * r + p;
+          unsigned m = n5;
+          for (int s = s0; s < min(ns, s0 + 5); ++s, m >>= 6, w += r) v += (int)(m & 63u) * *w;
+          G[i * r + p] = v;
         }
       }
     }
@@ -154,65 +185,106 @@ __device__ inline void field_stage(const ChainJob& J, const Geom& g, const Field
   __syncthreads();
 }
 
-// This lane's share of an update: lanes 0-15 the sites that have site 1 as a
-// neighbour, 16-31 site 2; entry (lane & 15) + 16 j of such a site leads back
-// to it, so the site lies one entry before it.
+// A thread's share of an update by the team: the first half of it takes the
+// sites around swapped site 1, the second half around site 2; entries (tid mod
+// half) + half j.  Entry e of a site leads to the swapped site when the site lies
+// one entry before it.
 template <int NJ>
 struct FieldPlan {
   int ex[NJ], ey[NJ], ez[NJ];  // byte addresses of the axis tables at -entry
   int ush[NJ];                 // the entry's shell in a row of U, bytes
-  unsigned valid;
+  int valid;                   // bit j: entry j exists
+};
+
+// The team that decides trials and updates fields: four of a block's warps.
+constexpr int kFieldTeam = 128, kFieldHalf = kFieldTeam / 2;
+__device__ __forceinline__ void team_sync() { asm volatile("bar.sync 6, 128;" ::: "memory"); }
+
+template <int R>
+struct FieldVec;
+template <>
+struct FieldVec<1> {
+  using T = int;
+  static __device__ __forceinline__ T add(T a, T b) { return a + b; }
+};
+template <>
+struct FieldVec<2> {
+  using T = int2;
+  static __device__ __forceinline__ T add(T a, T b) { return make_int2(a.x + b.x, a.y + b.y); }
+};
+template <>
+struct FieldVec<4> {
+  using T = int4;
+  static __device__ __forceinline__ T add(T a, T b) { return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 };
 
 template <int NJ>
-__device__ __forceinline__ void field_plan(const Geom& g, const FieldLayout& L, const unsigned char* smem, int lane,
+__device__ __forceinline__ void field_plan(const Geom& g, const FieldLayout& L, const unsigned char* smem, int tid,
                                            FieldPlan<NJ>& P) {
   const uint32_t* ents = reinterpret_cast<const uint32_t*>(smem + L.ents);
   P.valid = 0;
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const int k = (lane & 15) + 16 * j;
+    const int k = (tid & (kFieldHalf - 1)) + kFieldHalf * j;
     int dx = 0, dy = 0, dz = 0, sh = 0;
     if (k < g.z) {
       unpack_entry(ents[k], dx, dy, dz, sh);
-      P.valid |= 1u << j;
+      P.valid |= 1 << j;
     }
     P.ex[j] = (int)L.tabs[0] + (kHalo - dx) * 4;
     P.ey[j] = (int)L.tabs[1] + (kHalo - dy) * 4;
     P.ez[j] = (int)L.tabs[2] + (kHalo - dz) * 4;
-    P.ush[j] = sh * (g.ns - 1) * 4;
+    P.ush[j] = sh * field_stride(g.ns) * 4;
   }
 }
 
-// The swap of sites 1 and 2 (coordinates xyz1, xyz2, indices, species before):
-// the lattice and the fields.  All lanes of one warp; a __syncwarp follows
-// before either is read.  Sites can meet in several entries, so the adds are
-// atomic.
-template <int NJ>
-__device__ __forceinline__ void field_swap(const Geom& g, const FieldLayout& L, unsigned char* smem,
-                                           const FieldPlan<NJ>& P, int xyz1, int xyz2, int i1, int i2, int s1, int s2,
-                                           int lane) {
-  const bool second = lane >= 16;
-  const int c = second ? xyz2 : xyz1;
-  const int so = second ? s2 : s1, sn = second ? s1 : s2;
-  const int x4 = (c & 1023) << 2, y4 = (c >> 8) & 4092, z4 = (c >> 18) & 4092;
-  const int r = g.ns - 1;
-  const int row = (int)L.U + (((so - 1) * g.ns + (sn - 1)) * g.nsh * r) * 4;
+// This thread's share of the fields' update for a swap: its site's coordinates
+// and U's row of that site's change (byte address).  Plain loads, adds and
+// stores: an entry's sites are distinct for one swapped site, and where a site
+// may be around both, the halves go one after the other.  On lattices so small
+// that several entries of a site lead to one other (distinct = 0) the adds are
+// atomic.  R: fields a site keeps (1, 2 or 4 as one vector; 0: r of them).  The
+// team meets once more before the fields are read.
+template <int NJ, int R>
+__device__ __forceinline__ void field_update(const FieldLayout& L, unsigned char* smem, const FieldPlan<NJ>& P,
+                                             int distinct, int r, int xyz, int row, bool both, bool second) {
+  using F = FieldVec<R == 0 ? 1 : R>;
+  using T = typename F::T;
+  const int rs = R == 0 ? r : R;
+  const int x = (xyz & 1023) << 2, y = (xyz >> 8) & 4092, z = (xyz >> 18) & 4092;
+  auto tab = [&](int at) { return *reinterpret_cast<const int32_t*>(smem + at); };
   int at[NJ];
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
-    at[j] = *reinterpret_cast<const int32_t*>(smem + P.ex[j] + x4) +
-            *reinterpret_cast<const int32_t*>(smem + P.ey[j] + y4) +
-            *reinterpret_cast<const int32_t*>(smem + P.ez[j] + z4);
-  if (lane == 0) smem[L.lat + i1] = (unsigned char)s2;
-  if (lane == 16) smem[L.lat + i2] = (unsigned char)s1;
-  for (int p = 0; p < r; ++p) {
-    int32_t* G = reinterpret_cast<int32_t*>(smem + L.g) + p * g.n_sites;
+    at[j] = (int)L.g + 4 * rs * (tab(P.ex[j] + x) + tab(P.ey[j] + y) + tab(P.ez[j] + z));
+  if (!distinct) {
+    for (int p = 0; p < rs; ++p)
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int u = *reinterpret_cast<const int32_t*>(smem + row + P.ush[j] + 4 * p);
-      if ((P.valid >> j) & 1u) atomicAdd(G + at[j], u);
+      for (int j = 0; j < NJ; ++j)
+        if ((P.valid >> j) & 1)
+          atomicAdd(reinterpret_cast<int32_t*>(smem + at[j] + 4 * p),
+                    *reinterpret_cast<const int32_t*>(smem + row + P.ush[j] + 4 * p));
+    return;
+  }
+  auto add = [&]() {
+    for (int p = 0; p < (R == 0 ? r : 1); ++p) {
+      T d[NJ], v[NJ];
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        d[j] = *reinterpret_cast<const T*>(smem + row + P.ush[j] + 4 * p);
+        v[j] = *reinterpret_cast<const T*>(smem + at[j] + 4 * p);
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        if ((P.valid >> j) & 1) *reinterpret_cast<T*>(smem + at[j] + 4 * p) = F::add(v[j], d[j]);
     }
+  };
+  if (both) {
+    if (!second) add();
+    team_sync();
+    if (second) add();
+  } else {
+    add();
   }
 }
 
@@ -250,7 +322,7 @@ static __device__ __noinline__ double field_exact_delta(const FieldExact X, int 
     int dx, dy, dz, sh;
     unpack_entry(ents[k], dx, dy, dz, sh);
     const int i = tx[dx] + ty[dy] + tz[dz];
-    codes[(second ? z : 0) + k] = (uint8_t)(smem[X.lat + i] | (i == other ? kOther : 0));
+    codes[(second ? z : 0) + k] = (uint8_t)((smem[X.lat + i] >> 2) + 1 + (i == other ? kOther : 0));
   }
   __syncwarp();
   const int nc = 4 * nsh;

@@ -123,7 +123,7 @@ __host__ __device__ inline HaloLayout halo_layout(const Geom& g, const HaloGeom&
 // stream's rings (trial_window.cuh), the positions' records and the lattice
 // with its halo (halo_shear.cuh) at fixed places, then the tables.
 struct WindowLayout {
-  static constexpr uint32_t kRec = kRollWords * 4;           // kRecRing records of 16 bytes
+  static constexpr uint32_t kRec = GatherRing::kWords * 4;           // kRecRing records of 16 bytes
   static constexpr uint32_t kFlags = kRec + kRecRing * 16;   // and a word of flags each
   static constexpr uint32_t kLat = kFlags + kRecRing * 4;
   uint32_t V, I, D, edelta, ecan, dnbr, sstart, total;
@@ -177,23 +177,36 @@ enum shared_kernel : int {
   kSharedField = 2,   // the sites' fields there too (metropolis_field.cu)
 };
 
+// Whether a set of chains that could run with fields should.  A chain with
+// fields takes eight warps and its fields' shared memory, so two at most share an
+// SM (field_load: the part of an SM it takes); with the lattice alone it is one
+// warp, and six or more share one.  Cycles per trial and chain, with fields and
+// gathered (GB300, 900 K, four species, six shells): 116 and 572 on bcc 8^3 at
+// one chain per SM, 273 and 590 at four, 527 and 658 at eight; 153 and 396 on
+// bcc 16^3 (one per SM) at one, 308 and 402 at two, 456 and 407 at three; on fcc
+// 8^3 with two species 310 and 368 at four, 456 and 414 at six.  So: fields
+// while they take two rounds of the SMs at most.
+inline double field_load(uint32_t smem) { return 2u * (smem + 1024u) <= 228u * 1024u ? 0.5 : 1.0; }
+inline bool fields_pay(double load, int n_sm) { return load <= 2.0 * n_sm; }
+
 // One launch of them: `count` chains from `first` in launch order, the largest
-// shared memory, neighbour count and lattice among them, and the trials per
+// shared memory and neighbour count among them, and the trials per
 // round of the gather kernel (1: kGatherDefault).
 struct LaunchGroup {
   int kernel = kSharedNone, depth = 1, first = -1, count = 0;
   uint32_t smem = 0;
-  int max_z = 0, max_sites = 0;
+  int max_z = 0;
+  int ns = 0;        // species of one of them (field kernel: all are of its field_variant)
   int64_t most = 0;  // the most trials of one chain
 };
 constexpr int kGatherDefault = 4;
 void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int depth,
                             cudaStream_t stream);
-void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_sites, int max_z,
+void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int ns,
                              cudaStream_t stream);
 inline void launch_shared_chains(const ChainJob* d_jobs, int n_jobs, const LaunchGroup& G, cudaStream_t stream) {
   if (G.kernel == kSharedField)
-    launch_metropolis_field(d_jobs, n_jobs, G.smem, G.max_sites, G.max_z, stream);
+    launch_metropolis_field(d_jobs, n_jobs, G.smem, G.max_z, G.ns, stream);
   else
     launch_metropolis_halo(d_jobs, n_jobs, G.smem, G.max_z, G.depth, stream);
 }

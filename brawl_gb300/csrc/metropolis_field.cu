@@ -10,38 +10,29 @@ namespace brawl {
 
 namespace {
 
-// Named hardware barriers of the block's first two warps, per half h of the
-// record ring: its records are made (1, 2); they have been used (3, 4).  The
-// numbers are literals: a number in a register would reserve all sixteen.
-__device__ __forceinline__ void made_arrive(int h) {
-  if (h) asm volatile("bar.arrive 2, 64;" ::: "memory");
-  else asm volatile("bar.arrive 1, 64;" ::: "memory");
-}
-__device__ __forceinline__ void made_wait(int h) {
-  if (h) asm volatile("bar.sync 2, 64;" ::: "memory");
-  else asm volatile("bar.sync 1, 64;" ::: "memory");
-}
-__device__ __forceinline__ void used_arrive(int h) {
-  if (h) asm volatile("bar.arrive 4, 64;" ::: "memory");
-  else asm volatile("bar.arrive 3, 64;" ::: "memory");
-}
-__device__ __forceinline__ void used_wait(int h) {
-  if (h) asm volatile("bar.sync 4, 64;" ::: "memory");
-  else asm volatile("bar.sync 3, 64;" ::: "memory");
-}
+// Named hardware barriers of the team's warps and the makers', per part h of
+// the record ring: its records are made (1 + h); they have been used (3 + h);
+// and of the makers alone (5).
+__device__ __forceinline__ void made_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(1 + h) : "memory"); }
+__device__ __forceinline__ void made_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory"); }
+__device__ __forceinline__ void used_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(3 + h) : "memory"); }
+__device__ __forceinline__ void used_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(3 + h) : "memory"); }
+__device__ __forceinline__ void makers_meet() { asm volatile("bar.sync 5, 128;" ::: "memory"); }
 
-// What the walking warp tells the stream's warp at the end.
+// What the team tells the makers at the end.
 struct FieldEnd {
   unsigned long long words;
   int done;
 };
 
-// Warp 1: the windows' static records, two windows ahead of warp 0 at most
-// four.
+// A making warp (`mine` of kFieldMakers): its window's static records of every
+// part, two parts at most before the team has used one, and its 32 words of the
+// stream one part further on.
 __device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, const FieldLayout& L,
-                                              unsigned char* smem, FieldEnd* end, int lane) {
+                                              unsigned char* smem, FieldEnd* end, int mine, int lane) {
+  using Ring = FieldWords;
   uint32_t* mt = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* tw = mt + kMtRing + kMtMirror;
+  uint32_t* tw = mt + Ring::kTwAt;
   const FieldGeom f = J.fg;
   const uint8_t* dtab = smem + L.dtab;
   const bool bcc = g.lattice == kBcc;
@@ -50,67 +41,108 @@ __device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, 
   const float inv_k = 1.0f / J.beta_q_l2, band_f = (float)band;
   const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
   const int pos0 = (int)J.rng[kMTN];
-  mt_roll_load(J.rng, mt, pos0, lane);
-  __syncwarp();
   MtRoll R = {pos0, 0, 0};
-  mt_roll(mt, tw, R, lane);
-  __syncwarp();
-  mt_roll(mt, tw, R, lane);
-  __syncwarp();
-  unsigned long long made = 2 * kWin;
-  int at = 0;  // the window's place in the ring of tempered words
-  for (unsigned i = 0;; ++i) {
-    const int h = (int)(i & 1u);
-    if (i >= 2) used_wait(h);
-    if (*(volatile int*)&end->done) break;
+  if (mine == 0) {
+    mt_roll_load<Ring>(J.rng, mt, pos0, lane);
+    __syncwarp();
 #pragma unroll 1
-    for (int k = 0; k < 2; ++k) {
-      const uint32_t* w = tw + at + lane;
-      int ax, ay, az, Ya, Xa, bx, by, bz, Yb, Xb;
-      draw_site_halo(g, bcc, w[0], w[1], w[2], ax, ay, az, Ya, Xa);
-      if (nbr) {
-        // draw_nbr's neighbour; its steps are -1, 0, 1
-        const int8_t* v = cNbrSwap[g.lattice][umulhi32(w[3], (uint32_t)g.nbr_k)];
-        bx = wrap_fast(ax + v[0], W1);
-        by = wrap_fast(ay + v[1], W2);
-        bz = wrap_fast(az + v[2], W3);
-        Yb = by >> g.ys;
-        Xb = bx >> 1;
-      } else {
-        draw_site_halo(g, bcc, w[3], w[4], w[5], bx, by, bz, Yb, Xb);
-      }
-      const AcceptThresholds th = accept_thresholds(w[nbr ? 4 : 6], inv_k, band_f);
-      const int t1 = wrap_fast(bx - ax + f.dm[0], W1), t2 = wrap_fast(by - ay + f.dm[1], W2),
-                t3 = wrap_fast(bz - az + f.dm[2], W3);
-      int cls = 0;
-      if (t1 < f.side[0] && t2 < f.side[1] && t3 < f.side[2]) cls = dtab[(t3 * f.side[1] + t2) * f.side[0] + t1];
-      const int ia = az * g.sz + Ya * g.sy + Xa, ib = bz * g.sz + Yb * g.sy + Xb;
-      const int slot = (2 * h + k) * kWin + lane;
-      *reinterpret_cast<int4*>(smem + FieldLayout::kAt + slot * 16) =
-          make_int4(ax | ay << 10 | az << 20, bx | by << 10 | bz << 20, ia | ib << 16, cls);
-      *reinterpret_cast<int2*>(smem + FieldLayout::kTh + slot * 8) = make_int2(max(band, th.rej_above), th.acc_below);
-      mt_roll(mt, tw, R, lane);
-      made += kWin;
+    for (int k = 0; k < kFieldAhead / kWin; ++k) {
+      mt_roll<Ring>(mt, tw, R, lane);
       __syncwarp();
-      at = at + kWin == kTwRing ? 0 : at + kWin;
     }
+  }
+  // this warp's rows of the stream: the first after those, then every fourth
+  R = {pos0 + kFieldAhead + mine * kWin, kFieldAhead + mine * kWin, kFieldAhead + mine * kWin};
+  unsigned long long made = kFieldAhead;
+  int at = mine * kWin;  // the window's place in the ring of tempered words
+  const int ns4 = 4 * g.ns, c_at = (int)L.C;
+  bool wrapped = false;  // two parts have been made
+  for (int h = 0;; h ^= 1) {
+    if (wrapped) used_wait(h);
+    wrapped = wrapped || h == 1;
+    if (*(volatile int*)&end->done) break;
+    makers_meet();  // the words of the part before
+    const uint32_t* w = tw + at + lane;
+    int ax, ay, az, Ya, Xa, bx, by, bz, Yb, Xb;
+    draw_site_halo(g, bcc, w[0], w[1], w[2], ax, ay, az, Ya, Xa);
+    if (nbr) {
+      // draw_nbr's neighbour; its steps are -1, 0, 1
+      const int8_t* v = cNbrSwap[g.lattice][umulhi32(w[3], (uint32_t)g.nbr_k)];
+      bx = wrap_fast(ax + v[0], W1);
+      by = wrap_fast(ay + v[1], W2);
+      bz = wrap_fast(az + v[2], W3);
+      Yb = by >> g.ys;
+      Xb = bx >> 1;
+    } else {
+      draw_site_halo(g, bcc, w[3], w[4], w[5], bx, by, bz, Yb, Xb);
+    }
+    const AcceptThresholds th = accept_thresholds(w[nbr ? 4 : 6], inv_k, band_f);
+    const int t1 = wrap_fast(bx - ax + f.dm[0], W1), t2 = wrap_fast(by - ay + f.dm[1], W2),
+              t3 = wrap_fast(bz - az + f.dm[2], W3);
+    const int both = nbr || words_near(f.both_c, f.both_2c, w);  // a site may be around both
+    int cls = 0;
+    if (t1 < f.side[0] && t2 < f.side[1] && t3 < f.side[2]) cls = dtab[(t3 * f.side[1] + t2) * f.side[0] + t1];
+    const int ia = az * g.sz + Ya * g.sy + Xa, ib = bz * g.sz + Yb * g.sy + Xb;
+    const int slot = (kFieldMakers * h + mine) * kWin + lane;
+    *reinterpret_cast<int4*>(smem + FieldLayout::kA + slot * 16) =
+        make_int4(ia, ib, c_at + cls * g.ns * ns4, max(band, th.rej_above));
+    *reinterpret_cast<int4*>(smem + FieldLayout::kB + slot * 16) =
+        make_int4(ax | ay << 10 | az << 20, bx | by << 10 | bz << 20, th.acc_below, both);
+    mt_roll<Ring>(mt, tw, R, lane, kFieldMakers - 1);
+    made += kFieldPart;
+    at = at + kFieldPart >= Ring::kTw ? at + kFieldPart - Ring::kTw : at + kFieldPart;
     made_arrive(h);
   }
-  mt_roll_store(mt, tw, R, pos0, end->words, made, J.rng, lane);
+  if (mine == 0) mt_roll_store<Ring>(mt, tw, R, pos0, end->words, made, J.rng, lane);
 }
 
 }  // namespace
 
-// One chain per block.  All warps stage the tables and sum the fields; then
-// warp 1 makes the windows' records and warp 0 decides the trials.  What
-// bounds it: the chain's dependent sequence -- per window of 32 positions two
-// dependent shared loads (species, fields), two ballots and the stepping
-// through the outcomes, per accepted trial the update of 2z sites' fields and
-// the window again -- times the longest chain's trials.
-template <int NJ>
-__global__ void __launch_bounds__(256) metropolis_field_kernel(const ChainJob* __restrict__ jobs) {
+// The walk through a window of decided positions from this lane's position: like
+// pairs (accepted without an energy evaluation or a draw) and certain
+// rejections are passed, up to a trial that is neither or past the window.
+// Bits 0-7: that position (32 and more: past the window), 8-15: trials passed,
+// 16-23: rejections among them.
+__device__ __forceinline__ unsigned field_walk(unsigned like, unsigned rej, int lane, int n_base, bool nbr) {
+  unsigned path = 1u << lane;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
+  if (nbr) {  // eight trials can start in a window, six otherwise
+    path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
+    path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
+  }
+  // the positions passed, by n_base words each and one more per rejection
+  const unsigned passed = __popc(path & (like | rej)), n_rej = __popc(path & rej);
+  return ((unsigned)lane + passed * (unsigned)n_base + n_rej) | passed << 8 | n_rej << 16;
+}
+
+// What the team shares of two windows (twice: one pair is written while the
+// other is read): the walk from every position, each position's change and
+// species (as stored, site 2's from bit 8), and the masks of rejections.
+struct FieldShare {
+  unsigned walk[2][2 * kWin];
+  int2 pos[2][2 * kWin];
+  unsigned rej[2][2];
+  int verdict;  // the exact tier's: bit 0 accepted, bit 1 uniform drawn
+};
+
+// One chain per block.  All warps stage the tables and sum the fields; then four
+// make the windows' records and the team of four decides the trials.  The team
+// goes in step: two of its warps decide a window each (32 positions, one per
+// lane, on the lattice as it stands) and walk through it from every position; all
+// four then follow the walk to the first trial that is not certainly rejected,
+// and update the fields together when it is accepted.
+//
+// What bounds it: the chain's dependent sequence times the longest chain's
+// trials.  A pair of windows (nine or ten trials) costs the latency of two
+// dependent shared loads, a ballot, a barrier and the walk; an accepted trial
+// that of an update shared by 128 threads.  On one chain the other schedulers
+// of the SM are idle, so the team's repeated work costs nothing.
+template <int NJ, int R>
+__global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob* __restrict__ jobs) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ FieldEnd end;
+  __shared__ __align__(16) FieldShare S;
   const ChainJob& J = jobs[blockIdx.x];
   if (J.status && *J.status != 0) return;  // the chain's input was flagged: no trial runs
   const Geom g = J.g;
@@ -119,145 +151,156 @@ __global__ void __launch_bounds__(256) metropolis_field_kernel(const ChainJob* _
   const FieldLayout L = field_layout(g, J.fg);
   if (tid == 0) end.done = 0;
   field_stage(J, g, L, smem, tid, blockDim.x);
-  if (warp == 1) {
-    field_produce(J, g, L, smem, &end, lane);
-  } else if (warp == 0) {
+  // Warps 2, 3, 6 and 7 are the team (the schedulers take every fourth warp, so
+  // it has two of them to itself), 0, 1, 4 and 5 the makers.
+  if (warp < 8 && (warp & 2) == 0) {
+    field_produce(J, g, L, smem, &end, (warp & 1) + (warp >> 1), lane);
+  } else if (warp < 8) {
+    const int who = (warp & 1) + (warp >> 2) * 2, tt = who * 32 + lane;
+    const bool second = tt >= kFieldHalf;
     FieldPlan<NJ> P;
-    field_plan<NJ>(g, L, smem, lane, P);
-    const int n_base = J.nbr_swap ? 4 : 6;
-    const int hops = J.nbr_swap ? 7 : 5;  // trials that start in a window, less one
+    field_plan<NJ>(g, L, smem, tt, P);
+    const int distinct = J.fg.distinct;
+    const bool nbr = J.nbr_swap != 0;
+    const int n_base = nbr ? 4 : 6;
     const int nt = (int)J.n_trials;
-    const int band = J.band, ns = g.ns, n4 = 4 * g.n_sites;
-    const uint32_t* tw = reinterpret_cast<const uint32_t*>(smem) + kMtRing + kMtMirror;
+    const int band = J.band, ns = g.ns, r = field_stride(ns), stride = 4 * r, per = g.nsh * stride;
     // 32-bit tallies (a launch runs fewer than 2^31 trials per chain); the
     // uniforms follow from the words consumed
-    unsigned b_eval = 0, b_acc = 0, b_exact = 0, c_fp64 = 0, c_cr = 0;
-    const FieldExact X = field_exact_setup(g, L);
-    unsigned n_win = 0;  // windows passed
-    int o = 0, t = 0;    // the next trial's position in the window; trials done
-    int4 at;             // this lane's position
-    int2 th;
-    unsigned like = 0, rej = 0;  // positions: two like species; certainly rejected
-    int outcome = 0;             // sa | sb << 4 | certainly accepted << 8 | certainly downhill << 9
-    auto window = [&]() {
-      const int slot = (int)(n_win & 3u) * kWin + lane;
-      at = *reinterpret_cast<const int4*>(smem + FieldLayout::kAt + slot * 16);
-      th = *reinterpret_cast<const int2*>(smem + FieldLayout::kTh + slot * 8);
-    };
-    auto decide = [&]() {
-      const int ia = at.z & 0xffff, ib = (int)((unsigned)at.z >> 16);
-      const int sa = smem[L.lat + ia], sb = smem[L.lat + ib];
-      const unsigned char* ga = smem + L.g + 4 * ia - 2 * n4;
-      const unsigned char* gb = smem + L.g + 4 * ib - 2 * n4;
-      int dE = 0;
-      if (sb > 1) dE += *reinterpret_cast<const int32_t*>(ga + sb * n4) - *reinterpret_cast<const int32_t*>(gb + sb * n4);
-      if (sa > 1) dE += *reinterpret_cast<const int32_t*>(gb + sa * n4) - *reinterpret_cast<const int32_t*>(ga + sa * n4);
-      if (at.w) dE += *reinterpret_cast<const int32_t*>(smem + L.C + ((at.w * ns + sa - 1) * ns + sb - 1) * 4);
-      const bool same = sa == sb;
-      const bool down = dE < -band;
-      const bool sure = down || (dE > band && dE < th.y);
-      // (rej_above >= acc_below: a trial above rej_above is not also below it)
-      like = __ballot_sync(kFull, same);
-      rej = __ballot_sync(kFull, !same && dE > th.x);
-      outcome = sa | sb << 4 | (sure ? 1 << 8 : 0) | (down ? 1 << 9 : 0);
+    unsigned b_like = 0, b_rej = 0, b_event = 0, b_acc = 0, b_exact = 0, c_fp64 = 0, c_cr = 0;
+    unsigned n_win = 0;      // windows passed
+    int o = 0, t = 0;        // the next trial's position in the window; trials done
+    int slot = 0;            // the window's place in the record ring
+    unsigned have = 0;       // the last part waited for
+    int flip = 0;            // the shared pair in use
+    auto after = [&](int at, int by) { return at + by >= kFieldRing ? at + by - kFieldRing : at + by; };
+    // k = 0, 1 or 2 windows on; the window after the next one is at hand
+    auto pass_windows = [&](int k) {
+      const unsigned before = n_win / kFieldMakers;
+      n_win += k;
+      slot = after(slot, k * kWin);
+      if (n_win / kFieldMakers != before) used_arrive((int)(before & 1u));
+      if ((n_win + 1) / kFieldMakers != have) {
+        ++have;
+        made_wait((int)(have & 1u));
+      }
     };
     made_wait(0);
-    window();
-    decide();
     while (t < nt) {
-      if (o >= kWin) {
-        o -= kWin;
-        ++n_win;
-        if ((n_win & 1u) == 0u) {
-          const int h = (int)((n_win >> 1) & 1u);
-          used_arrive(h ^ 1);
-          made_wait(h);
-        }
-        window();
-        decide();
+      if (who < 2) {
+        const int4 a = *reinterpret_cast<const int4*>(smem + FieldLayout::kA + (after(slot, kWin * who) + lane) * 16);
+        const int sa = smem[L.lat + a.x], sb = smem[L.lat + a.y];
+        // species 1 (0 as stored) has no field: its loads are read past
+        const unsigned char* ga = smem + L.g - 4 + a.x * stride;
+        const unsigned char* gb = smem + L.g - 4 + a.y * stride;
+        const int ab = *reinterpret_cast<const int32_t*>(ga + sb), bb = *reinterpret_cast<const int32_t*>(gb + sb);
+        const int ba = *reinterpret_cast<const int32_t*>(gb + sa), aa = *reinterpret_cast<const int32_t*>(ga + sa);
+        const int met = *reinterpret_cast<const int32_t*>(smem + a.z + sa * ns + sb);
+        const int dE = (sb ? ab - bb : 0) + (sa ? ba - aa : 0) + met;
+        // (rej_above >= acc_below: a trial above rej_above is not also below it)
+        const unsigned like = __ballot_sync(kFull, sa == sb);
+        const unsigned rej = __ballot_sync(kFull, sa != sb && dE > a.w);
+        S.pos[flip][tt] = make_int2(dE, sa | sb << 8);
+        S.walk[flip][tt] = field_walk(like, rej, lane, n_base, nbr);
+        if (lane == 0) S.rej[flip][who] = rej;
       }
-      // the positions the chain steps through from o: like pairs (accepted
-      // without an energy evaluation or a draw) and certain rejections, up to
-      // the first other trial or the window's end
-      unsigned path = 1u << o;
-      const unsigned pass = like | rej;
-#pragma unroll
-      for (int i = 0; i < 5; ++i) path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
-      if (hops > 5) {
-        path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
-        path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
-      }
-      const int passed = __popc(path & pass);
+      team_sync();
+      const unsigned w0 = S.walk[flip][o];
+      const int o0 = (int)(w0 & 0xffu);
+      const unsigned w1 = o0 >= kWin ? S.walk[flip][o0] : 0u;
+      const unsigned w = w0 + w1;  // (the counts; the positions apart)
+      const int passed = (int)((w >> 8) & 0xffu), n_rej = (int)(w >> 16);
       if (passed >= nt - t) {
-        // the run ends among them, at its last trial
-        unsigned m = path & pass;
-        for (int i = nt - t; i < passed; ++i) m &= ~(0x80000000u >> __clz(m));
-        const int last = 31 - __clz(m);
-        b_acc += __popc(m & like);
-        b_eval += __popc(m & rej);
-        o = last + n_base + (int)((rej >> last) & 1u);
-        t = nt;
+        // the run ends among the passed trials
+        int k = 0;
+        for (; t < nt; ++t) {
+          const unsigned re = (S.rej[flip][k] >> o) & 1u;
+          b_like += 1u - re;
+          b_rej += re;
+          o += n_base + (int)re;
+          if (o >= kWin) {
+            o -= kWin;
+            ++k;
+          }
+        }
+        pass_windows(k);
         break;
       }
       t += passed;
-      b_acc += __popc(path & like);
-      b_eval += __popc(path & rej);
-      const unsigned stop = path & ~pass;
-      if (stop == 0u) {
-        const int last = 31 - __clz(path);
-        o = last + n_base + (int)((rej >> last) & 1u);
+      b_rej += n_rej;
+      b_like += passed - n_rej;
+      const int e = o0 >= kWin;
+      const int p = e ? (int)(w1 & 0xffu) : o0;
+      if (p >= kWin) {
+        flip ^= 1;
+        o = p - kWin;
+        pass_windows(2);
         continue;
       }
       // ---- a trial that is not certainly rejected ---------------------------
-      const int p = __ffs(stop) - 1;
-      const int out = __shfl_sync(kFull, outcome, p);
-      const int4 q = *reinterpret_cast<const int4*>(smem + FieldLayout::kAt + ((int)(n_win & 3u) * kWin + p) * 16);
-      const int s1 = out & 15, s2 = (out >> 4) & 15;
-      const int i1 = q.z & 0xffff, i2 = (int)((unsigned)q.z >> 16);
+      const int at = after(slot, kWin * e) + p;
+      const int4 a = *reinterpret_cast<const int4*>(smem + FieldLayout::kA + at * 16);
+      const int4 q = *reinterpret_cast<const int4*>(smem + FieldLayout::kB + at * 16);
+      const int2 v = S.pos[flip][kWin * e + p];
+      const int s1 = v.y & 0xff, s2 = v.y >> 8;
       ++t;
-      ++b_eval;
-      int accept = 1;
-      if (out & (1 << 8)) {
-        o = p + n_base + ((out >> 9) & 1 ? 0 : 1);
-      } else {
+      ++b_event;
+      o = p + n_base + (v.x > band);
+      int accept = v.x < -band || (v.x > band && v.x < q.z) ? 1 : -1;
+      if (accept < 0) {
         // inside the band, or too near its threshold: the reference's FP64
         // sums, in its order
         ++b_exact;
-        const double delta_e = field_exact_delta(X, q.x, q.y, i1, i2, s1, s2, lane);
-        o = p + n_base;
-        if (!(delta_e < 0.0)) {
-          DecideStats st = {0u, 0u};
-          const uint32_t wu = tw[(int)(n_win & (kTwRing / kWin - 1)) * kWin + p + n_base];
-          accept = u_lt_exp(wu, __dmul_rn(-J.beta, delta_e), st);
-          ++o;
-          c_fp64 += st.fp64;
-          c_cr += st.cr;
+        if (who == 0) {
+          const double delta_e = field_exact_delta(field_exact_setup(g, L), q.x, q.y, a.x, a.y, (s1 >> 2) + 1,
+                                                   (s2 >> 2) + 1, lane);
+          int verdict = 1;
+          if (!(delta_e < 0.0)) {
+            DecideStats st = {0u, 0u};
+            const uint32_t* tw = reinterpret_cast<const uint32_t*>(smem) + FieldWords::kTwAt;
+            const uint32_t wu = tw[((n_win + e) % (FieldWords::kTw / kWin)) * kWin + p + n_base];
+            verdict = u_lt_exp(wu, __dmul_rn(-J.beta, delta_e), st) | 2;
+            c_fp64 += st.fp64;
+            c_cr += st.cr;
+          }
+          if (lane == 0) S.verdict = verdict;
         }
+        team_sync();
+        const int verdict = *(volatile int*)&S.verdict;
+        accept = verdict & 1;
+        o = p + n_base + (verdict >> 1);
       }
       if (accept) {
         ++b_acc;
-        field_swap<NJ>(g, L, smem, P, q.x, q.y, i1, i2, s1, s2, lane);
-        __syncwarp();
-        if (o < kWin) decide();
+        if (tt == 0) {
+          smem[L.lat + a.x] = (unsigned char)s2;
+          smem[L.lat + a.y] = (unsigned char)s1;
+        }
+        // U's rows by (old - 1) ns + new - 1
+        const int row = (int)L.U + ((second ? s2 * ns + s1 : s1 * ns + s2) >> 2) * per;
+        field_update<NJ, R>(L, smem, P, distinct, r, second ? q.y : q.x, row, q.w != 0, second);
       }
+      pass_windows(e + (o >= kWin));
+      o &= kWin - 1;
+      team_sync();
     }
+    // the makers have made, or are making, the part after this one and then wait
+    // for this one to be used
+    const unsigned part = n_win / kFieldMakers;
+    if (have == part) made_wait((int)((part + 1) & 1u));
     const unsigned long long words = (unsigned long long)kWin * n_win + (unsigned long long)o;
-    // the stream's warp: it has made, or is making, the half after this one and
-    // then waits for this one to be used
-    const int h = (int)((n_win >> 1) & 1u);
-    made_wait(h ^ 1);
-    if (lane == 0) {
+    if (tt == 0) {
       end.words = words;
       end.done = 1;
     }
     __syncwarp();
-    used_arrive(h);
-    if (lane == 0) {
+    used_arrive((int)(part & 1u));
+    if (tt == 0) {
       unsigned long long* c = J.counters;
       c[kCntTrials] += (unsigned long long)nt;
-      c[kCntEvaluated] += b_eval;
+      c[kCntEvaluated] += b_rej + b_event;
       c[kCntDraws] += words;
-      c[kCntAccepted] += b_acc;
+      c[kCntAccepted] += b_like + b_acc;
       c[kCntExpTests] += words - (unsigned long long)n_base * (unsigned long long)nt;
       c[kCntExactPath] += b_exact;
       c[kCntExpFp64] += c_fp64;
@@ -266,44 +309,68 @@ __global__ void __launch_bounds__(256) metropolis_field_kernel(const ChainJob* _
   }
   __syncthreads();
   // ---- write back -----------------------------------------------------------
-  const int8_t* lat = reinterpret_cast<const int8_t*>(smem + L.lat);
-  const int n16 = g.n_sites >> 4;
-  const uint4* src = reinterpret_cast<const uint4*>(lat);
-  uint4* dst = reinterpret_cast<uint4*>(J.lat);
-  for (int i = tid; i < n16; i += blockDim.x) dst[i] = src[i];
-  for (int i = (n16 << 4) + tid; i < g.n_sites; i += blockDim.x) J.lat[i] = lat[i];
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(smem + L.lat);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(J.lat);
+  const int n4 = g.n_sites >> 2;
+  for (int i = tid; i < n4; i += blockDim.x) dst[i] = ((src[i] >> 2) & 0x3f3f3f3fu) + 0x01010101u;
+  for (int i = (n4 << 2) + tid; i < g.n_sites; i += blockDim.x) J.lat[i] = (int8_t)((smem[L.lat + i] >> 2) + 1);
   if (tid == 0 && J.t_ns) *J.t_ns = global_ns() - t_start;
 }
 
-int field_threads(int n_sites) { return n_sites <= 512 ? 64 : n_sites <= 4096 ? 128 : 256; }
-
-template <int NJ>
-static void launch_field_nj(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int threads, cudaStream_t stream) {
-  cudaFuncSetAttribute(metropolis_field_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  BRAWL_CARVEOUT(metropolis_field_kernel<NJ>);
-  metropolis_field_kernel<NJ><<<n_jobs, threads, smem_bytes, stream>>>(d_jobs);
+// Threads per chain: eight warps run the trials; the others share the staging and
+// the fields' first sums.  Chains that have an SM to themselves take 16 warps
+// (four on each scheduler).
+static int field_threads(int n_jobs) {
+  static int n_sm = 0;
+  if (n_sm == 0) {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    n_sm = n;
+  }
+  return n_jobs <= n_sm ? 512 : 256;
 }
 
-void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_sites, int max_z,
+template <int NJ, int R>
+static void launch_field_r(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, cudaStream_t stream) {
+  cudaFuncSetAttribute(metropolis_field_kernel<NJ, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+  BRAWL_CARVEOUT(metropolis_field_kernel<NJ, R>);
+  metropolis_field_kernel<NJ, R><<<n_jobs, field_threads(n_jobs), smem_bytes, stream>>>(d_jobs);
+}
+
+template <int NJ>
+static void launch_field_nj(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int ns, cudaStream_t stream) {
+  switch (field_variant(ns)) {
+    case 1: launch_field_r<NJ, 1>(d_jobs, n_jobs, smem_bytes, stream); break;
+    case 2: launch_field_r<NJ, 2>(d_jobs, n_jobs, smem_bytes, stream); break;
+    case 4: launch_field_r<NJ, 4>(d_jobs, n_jobs, smem_bytes, stream); break;
+    default: launch_field_r<NJ, 0>(d_jobs, n_jobs, smem_bytes, stream); break;
+  }
+}
+
+// The chains are of ns's variant (field_variant), their neighbour counts up to
+// max_z.
+void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int ns,
                              cudaStream_t stream) {
   if (n_jobs <= 0) return;
-  const int threads = field_threads(max_sites);
-  switch (lane_entries_for(max_z)) {
-    case 2: launch_field_nj<2>(d_jobs, n_jobs, smem_bytes, threads, stream); break;
-    case 4: launch_field_nj<4>(d_jobs, n_jobs, smem_bytes, threads, stream); break;
-    case 6: launch_field_nj<6>(d_jobs, n_jobs, smem_bytes, threads, stream); break;
-    case 8: launch_field_nj<8>(d_jobs, n_jobs, smem_bytes, threads, stream); break;
-    default: launch_field_nj<11>(d_jobs, n_jobs, smem_bytes, threads, stream); break;
-  }
+  if (max_z <= kFieldHalf) launch_field_nj<1>(d_jobs, n_jobs, smem_bytes, ns, stream);
+  else if (max_z <= 2 * kFieldHalf) launch_field_nj<2>(d_jobs, n_jobs, smem_bytes, ns, stream);
+  else launch_field_nj<3>(d_jobs, n_jobs, smem_bytes, ns, stream);
+}
+
+template <int NJ>
+static void preload_field_nj(cudaFuncAttributes& a) {
+  cudaFuncGetAttributes(&a, metropolis_field_kernel<NJ, 1>);
+  cudaFuncGetAttributes(&a, metropolis_field_kernel<NJ, 2>);
+  cudaFuncGetAttributes(&a, metropolis_field_kernel<NJ, 4>);
+  cudaFuncGetAttributes(&a, metropolis_field_kernel<NJ, 0>);
 }
 
 void preload_field_kernels() {
   cudaFuncAttributes a;
-  cudaFuncGetAttributes(&a, metropolis_field_kernel<2>);
-  cudaFuncGetAttributes(&a, metropolis_field_kernel<4>);
-  cudaFuncGetAttributes(&a, metropolis_field_kernel<6>);
-  cudaFuncGetAttributes(&a, metropolis_field_kernel<8>);
-  cudaFuncGetAttributes(&a, metropolis_field_kernel<11>);
+  preload_field_nj<1>(a);
+  preload_field_nj<2>(a);
+  preload_field_nj<3>(a);
 }
 
 }  // namespace brawl

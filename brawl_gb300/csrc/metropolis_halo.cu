@@ -85,14 +85,6 @@ __device__ __forceinline__ int image_codes(const HaloGeom& H, int X, int Y, int 
   return cx | cy | cz;
 }
 
-// Whether the sites of two word triples may be within interaction range, from
-// the words alone (never false for a pair that is; make_halo has the margin).
-__device__ __forceinline__ bool pair_near_words(const HaloGeom& H, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t b0,
-                                                uint32_t b1, uint32_t b2) {
-  return (b0 - a0 + H.near_c[0] <= H.near_2c[0]) & (b1 - a1 + H.near_c[1] <= H.near_2c[1]) &
-         (b2 - a2 + H.near_c[2] <= H.near_2c[2]);
-}
-
 constexpr int kNoTrial = 0x40;  // no further trial known: past the two windows, or too many like pairs between
 constexpr int kRun = 5;         // like pairs a step passes over at most, plus one
 
@@ -150,7 +142,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   if (lane == 0) s_t_start = global_ns();
   const WindowLayout L = window_layout(g, H);
   uint32_t* mt = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* tw = mt + kMtRing + kMtMirror;
+  uint32_t* tw = mt + GatherRing::kTwAt;
   int4* rec = reinterpret_cast<int4*>(smem + WL::kRec);
   int32_t* flags = reinterpret_cast<int32_t*>(smem + WL::kFlags);
   uint8_t* lat = smem + WL::kLat;
@@ -169,7 +161,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   const int nF = nsp * g.nsh * nsp, nV = g.ns * g.ns * g.nsh;
   const uint32_t* rng = Jg->rng;
   const int pos0 = (int)rng[kMTN];
-  mt_roll_load(rng, mt, pos0, lane);
+  mt_roll_load<GatherRing>(rng, mt, pos0, lane);
   for (int i = lane; i < nF; i += 32) F[i] = Jg->F[i];
   {
     // the difference table, each pair's rows followed by a row of zeros (for
@@ -229,11 +221,11 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   MtRoll R = {pos0, 0, 0};
 #pragma unroll 1
   for (int i = 0; i < kLookAhead / kWin; ++i) {
-    mt_roll(mt, tw, R, lane);
+    mt_roll<GatherRing>(mt, tw, R, lane);
     __syncwarp();
   }
   unsigned int n_win = 0;   // windows passed
-  int tb = kTwRing - 2 * kWin;  // the first window's place in the ring of tempered words
+  int tb = GatherRing::kTw - 2 * kWin;  // the first window's place in the ring of tempered words
   int half = 0;             // its half of the record ring: 0 or kWin
   // this lane's sites: of the two windows, and of the next one (species not
   // read yet, the pair's flags in nf)
@@ -245,7 +237,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
     draw_site_halo(g, bcc, w[0], w[1], w[2], x, y, z, Y, X);
     if (!nbr_swap) {
       draw_site_halo(g, bcc, w[3], w[4], w[5], x2, y2, z2, Y2, X2);
-      nf = pair_near_words(H, w[0], w[1], w[2], w[3], w[4], w[5]) ? kFlagNear : 0;
+      nf = words_near(H.near_c, H.near_2c, w) ? kFlagNear : 0;
     } else {
       // draw_nbr's neighbour; its steps are -1, 0, 1
       const int k = (int)umulhi32(w[3], (uint32_t)g.nbr_k);
@@ -271,7 +263,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   // one window on: the second becomes the first, the next one's species are
   // read, the one after is decoded and 32 more words are generated
   auto advance = [&]() {
-    tb = tb + kWin == kTwRing ? 0 : tb + kWin;
+    tb = tb + kWin == GatherRing::kTw ? 0 : tb + kWin;
     ca0 = ca1;
     cb0 = cb1;
     lo = hi;
@@ -280,8 +272,8 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
     const int f = nf;
     const int sa = lat[na], sb = lat[nb];
     const int ahead = tb + 2 * kWin;
-    decode(ahead >= kTwRing ? ahead - kTwRing : ahead);
-    mt_roll(mt, tw, R, lane);
+    decode(ahead >= GatherRing::kTw ? ahead - GatherRing::kTw : ahead);
+    mt_roll<GatherRing>(mt, tw, R, lane);
     put(half + lane, ca1, cb1, sa, sb, f);  // the half the window that ended held
     half ^= kWin;
     hi = __ballot_sync(kFull, sa != sb);
@@ -329,7 +321,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
     }
     const int fl = flags[(half + pl) & (kRecRing - 1)];
     int wat = tb + pl + n_base;
-    wat -= wat >= kTwRing ? kTwRing : 0;
+    wat -= wat >= GatherRing::kTw ? GatherRing::kTw : 0;
     const AcceptThresholds th = accept_thresholds(tw[wat], inv_k, band_f);
     int acc[kSpec];
 #pragma unroll
@@ -348,7 +340,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
       // the displacement of the pair at position p
       if (nbr_swap) return dnbr[(f >> kFlagNbr) & 15];
       int ax, ay, az, bx, by, bz;
-      const uint32_t* w = tw + (tb + p >= kTwRing ? tb + p - kTwRing : tb + p);
+      const uint32_t* w = tw + (tb + p >= GatherRing::kTw ? tb + p - GatherRing::kTw : tb + p);
       draw_site(g, w[0], w[1], w[2], ax, ay, az);
       draw_site(g, w[3], w[4], w[5], bx, by, bz);
       return displacement(g, bx - ax, by - ay, bz - az);
@@ -407,7 +399,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
     } else {
       ++b_exact;
       const int d = (f & kFlagNear) ? pair_d(p, f) : -2;
-      const int at = tb + p >= kTwRing ? tb + p - kTwRing : tb + p;
+      const int at = tb + p >= GatherRing::kTw ? tb + p - GatherRing::kTw : tb + p;
       const int r = window_exact(Jg, V, edelta, ecan, epad, sstart, lat, q.x, q.z, s1 >> 2, s2 >> 2, d, g.ns, g.nsh,
                                  tw[at + n_base], lane);
       accept = r & 1;
@@ -452,7 +444,7 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
   __syncwarp();
   const unsigned long long words = (unsigned long long)kWin * n_win + (unsigned long long)o;
   shear_store(g, H, lat, Jg->lat, lane);
-  mt_roll_store(mt, tw, R, pos0, words, (unsigned long long)kWin * (n_win + 2) + kLookAhead, Jg->rng, lane);
+  mt_roll_store<GatherRing>(mt, tw, R, pos0, words, (unsigned long long)kWin * (n_win + 2) + kLookAhead, Jg->rng, lane);
   if (lane == 0) {
     unsigned long long* c = Jg->counters;
     c[kCntTrials] += (unsigned long long)nt;

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "api_internal.h"
+#include "field_engine.cuh"
 
 using namespace brawl;
 
@@ -176,7 +177,7 @@ __global__ void ns_unstage_kernel(const NsRun* __restrict__ from, NsRun* const* 
 // others on side streams forked from it and joined back: one launch sized
 // for the largest lattice would give every small one the same shared
 // memory and leave most of each SM's slots empty.
-constexpr int kSide = 3;
+constexpr int kSide = 7;
 
 struct Pipe {
   cudaStream_t s = nullptr;
@@ -298,9 +299,23 @@ struct Group {
   int first, count;
 };
 
+// The kernel a chain takes in a round where fields pay (or do not), its shared
+// memory, and what the chains of one launch have alike: the kernel, with fields
+// their number per site.
+int round_kernel(const ChainSlot& s, bool fields) {
+  return s.kernel == kSharedField && !fields && s.gather_smem > 0 ? (int)kSharedGather : s.kernel;
+}
+uint32_t round_smem(const ChainSlot& s, bool fields) {
+  return round_kernel(s, fields) == kSharedField ? s.field_smem : s.gather_smem;
+}
+int round_kind(const ChainSlot& s, bool fields) {
+  const int k = round_kernel(s, fields);
+  return k == kSharedField ? 8 + field_variant(s.job.g.ns) : k;
+}
+
 std::vector<Group> smem_groups(const std::vector<uint32_t>& smem, const std::vector<int>* kind = nullptr) {
   std::vector<Group> gs;
-  const int most = kind ? kSide - 1 : kSide;  // room for the change of kind
+  const int most = kind ? 3 : kSide;  // room for the changes of kind (at most four)
   for (int i = 0; i < (int)smem.size(); ++i) {
     const bool other = kind && i > 0 && (*kind)[i] != (*kind)[i - 1];
     if (gs.empty() || other ||
@@ -334,7 +349,7 @@ int launch_groups(Pipe& P, const std::vector<Group>& gs, F launch) {
 struct brawl_server {
   brawl_server_opts o;
   int device = 0;
-  int max_optin = 0;
+  int max_optin = 0, n_sm = 0;
   std::chrono::steady_clock::time_point t0;
   std::mutex mu;
   // cv_work: workers wait for admissible or ended jobs; cv_sched: the
@@ -651,9 +666,14 @@ int launch_anneal(brawl_server* S, Pipe& P) {
   bool use_D = true;
   SV_TRY(grow(P.d_tns, P.tns_cap, std::max<size_t>(P.jobs.size(), 1), P.s));
   const double t_round = round_ns(S, P.jobs);
-  std::stable_sort(P.jobs.begin(), P.jobs.end(), [](const JobP& a, const JobP& b) {
-    if (a->slot.kernel != b->slot.kernel) return a->slot.kernel > b->slot.kernel;
-    return a->slot.shared_smem > b->slot.shared_smem;
+  double load = 0.0;
+  for (const auto& j : P.jobs)
+    if (j->slot.kernel == kSharedField) load += field_load(j->slot.field_smem);
+  const bool fields = fields_pay(load, S->n_sm);
+  std::stable_sort(P.jobs.begin(), P.jobs.end(), [fields](const JobP& a, const JobP& b) {
+    const int ka = round_kind(a->slot, fields), kb = round_kind(b->slot, fields);
+    if (ka != kb) return ka > kb;
+    return round_smem(a->slot, fields) > round_smem(b->slot, fields);
   });
   for (int pass = 0; pass < 2; ++pass)
     for (auto& j : P.jobs) {
@@ -685,17 +705,15 @@ int launch_anneal(brawl_server* S, Pipe& P) {
     std::vector<uint32_t> sm(nh);
     std::vector<int> kind(nh);
     for (int k = 0; k < nh; ++k) {
-      sm[k] = P.launched[k]->slot.shared_smem;
-      kind[k] = P.launched[k]->slot.kernel;
+      sm[k] = round_smem(P.launched[k]->slot, fields);
+      kind[k] = round_kind(P.launched[k]->slot, fields);
     }
     SV_TRY(launch_groups(P, smem_groups(sm, &kind), [&](int first, int count, cudaStream_t st) {
       LaunchGroup G;
-      G.kernel = kind[first];
+      G.kernel = round_kernel(P.launched[first]->slot, fields);
+      G.ns = staged[first].g.ns;
       G.smem = sm[first];
-      for (int k = first; k < first + count; ++k) {
-        G.max_z = std::max(G.max_z, (int)staged[k].g.z);
-        G.max_sites = std::max(G.max_sites, (int)staged[k].g.n_sites);
-      }
+      for (int k = first; k < first + count; ++k) G.max_z = std::max(G.max_z, (int)staged[k].g.z);
       launch_shared_chains(P.d_chain + first, count, G, st);
     }));
   }
@@ -1202,6 +1220,7 @@ int brawl_serve_create(const brawl_server_opts* opts, brawl_server** out) {
   if (S->o.max_trials < 0) S->o.max_trials = 0;
   if (S->o.max_iterations < 0) S->o.max_iterations = 0;
   cudaDeviceGetAttribute(&S->max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S->device);
+  cudaDeviceGetAttribute(&S->n_sm, cudaDevAttrMultiProcessorCount, S->device);
   // every kernel a round may launch is loaded now: a round that first used
   // a variant would otherwise wait for every round in flight
   preload_metropolis_kernels();
