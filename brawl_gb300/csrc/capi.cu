@@ -228,6 +228,18 @@ bool make_field(const Geom& g, FieldTabs& T) {
         v[2 * sh + side] += 1;
       }
   T.fg.distinct = 1;
+  T.fg.symmetric = 1;
+  for (int sh = 0; sh < g.nsh; ++sh) {
+    // the shell's entries and their opposites, as sets with repeats
+    std::map<int, int> count;
+    auto key = [](int x, int y, int z) { return (x + 64) + 128 * ((y + 64) + 128 * (z + 64)); };
+    for (int k = st[sh]; k < st[sh + 1]; ++k) {
+      count[key(offs[k][0], offs[k][1], offs[k][2])] += 1;
+      count[key(-offs[k][0], -offs[k][1], -offs[k][2])] -= 1;
+    }
+    for (const auto& e : count)
+      if (e.second != 0) T.fg.symmetric = 0;
+  }
   for (const auto& e : met) {
     int once = 0;
     for (int sh = 0; sh < g.nsh; ++sh) once += e.second[2 * sh];
@@ -2254,6 +2266,11 @@ struct brawl_wl {
   uint32_t smem = 0;
   int max_z = 0;        // the kernel variant: entries per lane and D staged
   bool all_D = true;
+  // with the sites' fields (wl_field.cu): its shared memory and field_variant,
+  // when every walker can take it (wl_plan_fields)
+  bool fields = false;
+  uint32_t field_smem = 0;
+  int variant = 0;
   // radial-density samples (brawl_wl_radial_enable)
   int rad_wc = 0, rad_n_off = 0, rad_n_class = 0;
   WlRadial* d_rad = nullptr;
@@ -2305,6 +2322,29 @@ int batch_genrand(brawl_batch* b, int c, int64_t n, double* out) {
   return BRAWL_OK;
 }
 }  // namespace
+
+// The walkers' sweeps with fields: when all have displacement classes, lists
+// that hold every entry's opposite (the log and the update share a plan) and one
+// field_variant, their fields, window and a log of sixteen moves fit (fewer, and
+// the flushes would cost more than the fields save), and no radial samples are
+// taken (those need every trial's bin).  Both sides' times: wl_field_kernel.
+static void wl_plan_fields(brawl_wl* wl) {
+  int max_optin = 0;
+  cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, wl->b->device);
+  wl->fields = wl->d_rad == nullptr;
+  wl->field_smem = 0;
+  wl->variant = field_variant(wl->w[0].job.g.ns);
+  for (WlWalker& W : wl->w) {
+    const Geom& g = W.job.g;
+    const int nb = W.end - W.start + 1;
+    W.field_cap = 0;
+    if (W.job.fg.n_class > 0 && W.job.fg.symmetric)
+      W.field_cap = lazy_cap_for(g, wl_field_smem_bytes(g, W.job.fg, nb, 0), (uint32_t)max_optin);
+    if (W.field_cap < std::min(16, W.lazy_cap) || field_variant(g.ns) != wl->variant) wl->fields = false;
+    if (W.field_cap > 0)
+      wl->field_smem = std::max(wl->field_smem, wl_field_smem_bytes(g, W.job.fg, nb, W.field_cap));
+  }
+}
 
 extern "C" int brawl_wl_destroy(brawl_wl* wl) {
   if (!wl) return BRAWL_OK;
@@ -2408,6 +2448,7 @@ extern "C" int brawl_wl_create(const brawl_wl_desc* walkers, int n, int bins,
     return cleanup(fail(BRAWL_ENOMEM, "exchange buffers"));
   cudaMemcpyAsync(wl->d_groups, wl->groups.data(), wl->groups.size() * sizeof(WlGroup), cudaMemcpyHostToDevice, ws);
   if (stream_wait(ws) != cudaSuccess) return cleanup(fail(BRAWL_ECUDA, "walker set-up"));
+  wl_plan_fields(wl);
   *out = wl;
   return BRAWL_OK;
 }
@@ -2426,7 +2467,10 @@ extern "C" int brawl_wl_sweeps(brawl_wl* wl, int64_t n_trials, double wl_f, int 
     W.hist_period = hist_period;
   }
   CUDA_TRY(cudaMemcpyAsync(wl->d_w, wl->w.data(), n * sizeof(WlWalker), cudaMemcpyHostToDevice, b->stream));
-  launch_wl_sweeps(wl->d_w, n, wl->smem, wl->max_z, wl->all_D, b->stream);
+  if (wl->fields)
+    launch_wl_field(wl->d_w, n, wl->field_smem, wl->max_z, wl->variant, b->stream);
+  else
+    launch_wl_sweeps(wl->d_w, n, wl->smem, wl->max_z, wl->all_D, b->stream);
   launch_wl_average(wl->d_groups, (int)wl->groups.size(), wl->d_w, wl->bins, 1, b->stream);
   CUDA_TRY(cudaGetLastError());
   std::vector<WlWalker> res(n);
@@ -2644,6 +2688,7 @@ extern "C" int brawl_wl_radial_enable(brawl_wl* wl, int wc_range, const double* 
   wl->rad_wc = wc_range;
   wl->rad_n_off = n_off;
   wl->rad_n_class = n_class;
+  wl_plan_fields(wl);
   wl->smem = std::max(wl->smem, smem);
   for (int c = 0; c < n; ++c) {
     WlWalker& W = wl->w[c];
@@ -2837,6 +2882,7 @@ extern "C" int brawl_wl_set_windows(brawl_wl* wl, const int* start_idx, const in
   }
   wl->smem = smem;
   wl->all_D = all_D;
+  wl_plan_fields(wl);
   CUDA_TRY(stream_wait(s));
   return BRAWL_OK;
 }
@@ -2951,7 +2997,8 @@ int api_batch_set_rng(brawl_batch* b, int c, const uint32_t state[625]) {
 cudaStream_t api_batch_stream(brawl_batch* b) { return b->stream; }
 brawl_batch* api_wl_batch(brawl_wl* wl) { return wl->b; }
 std::vector<WlWalker>& api_wl_walkers(brawl_wl* wl) { return wl->w; }
-uint32_t api_wl_smem(brawl_wl* wl) { return wl->smem; }
+uint32_t api_wl_smem(brawl_wl* wl) { return wl->fields ? wl->field_smem : wl->smem; }
+int api_wl_kind(brawl_wl* wl) { return wl->fields ? 8 + wl->variant : 0; }
 void api_wl_variant(brawl_wl* wl, int* max_z, bool* all_D) {
   *max_z = wl->max_z;
   *all_D = wl->all_D;

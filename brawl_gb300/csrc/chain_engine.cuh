@@ -111,6 +111,8 @@ struct FieldGeom {
   int32_t dm[3], side[3];   // per axis: offsets run to +-dm, values of (d + dm) mod W looked up
   int32_t n_class;
   int32_t distinct;         // no two entries lead to the same site
+  int32_t symmetric;        // every entry's opposite is an entry of its shell
+  int32_t pad;
   uint32_t both_c[3], both_2c[3];  // the words' test of HaloGeom::near_c for twice the offsets
   const uint8_t* dtab;      // class by displacement, side[0] fastest
   const uint8_t* sig;       // per class and shell: entries of site 1, of site 2, that meet the other site

@@ -17,15 +17,16 @@
 // gives.
 #pragma once
 
+#include "halo_engine.cuh"
 #include "kernels.cuh"
 
 namespace brawl {
 
 // A position's static record (the trial that would start there):
 //   A  index of site 1, of site 2; byte address of the neighbours' constants
-//      of its displacement class; the larger of rej_above and the band
-//   B  coordinates of site 1, of site 2 (x | y << 10 | z << 20); acc_below;
-//      whether a site may have both as neighbours
+//      of its displacement class; the caller's, from the acceptance word
+//   B  coordinates of site 1, of site 2 (x | y << 10 | z << 20); the caller's,
+//      from the acceptance word; whether a site may have both as neighbours
 // Four warps make them, a window each of a part of four; two parts are held.
 constexpr int kFieldMakers = 4;
 constexpr int kFieldPart = kFieldMakers * kWin, kFieldRing = 2 * kFieldPart;
@@ -218,9 +219,11 @@ struct FieldVec<4> {
   static __device__ __forceinline__ T add(T a, T b) { return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 };
 
+// sign = 1: the sites one entry after it instead, the same sites with the same
+// shells when every entry's opposite is an entry of its shell.
 template <int NJ>
 __device__ __forceinline__ void field_plan(const Geom& g, const FieldLayout& L, const unsigned char* smem, int tid,
-                                           FieldPlan<NJ>& P) {
+                                           FieldPlan<NJ>& P, int sign = -1) {
   const uint32_t* ents = reinterpret_cast<const uint32_t*>(smem + L.ents);
   P.valid = 0;
 #pragma unroll
@@ -231,11 +234,20 @@ __device__ __forceinline__ void field_plan(const Geom& g, const FieldLayout& L, 
       unpack_entry(ents[k], dx, dy, dz, sh);
       P.valid |= 1 << j;
     }
-    P.ex[j] = (int)L.tabs[0] + (kHalo - dx) * 4;
-    P.ey[j] = (int)L.tabs[1] + (kHalo - dy) * 4;
-    P.ez[j] = (int)L.tabs[2] + (kHalo - dz) * 4;
+    P.ex[j] = (int)L.tabs[0] + (kHalo + sign * dx) * 4;
+    P.ey[j] = (int)L.tabs[1] + (kHalo + sign * dy) * 4;
+    P.ez[j] = (int)L.tabs[2] + (kHalo + sign * dz) * 4;
     P.ush[j] = sh * field_stride(g.ns) * 4;
   }
+}
+
+// The plan's sites around the site at coordinates xyz (compact indices).
+template <int NJ>
+__device__ __forceinline__ void field_sites(const unsigned char* smem, const FieldPlan<NJ>& P, int xyz, int* at) {
+  const int x = (xyz & 1023) << 2, y = (xyz >> 8) & 4092, z = (xyz >> 18) & 4092;
+  auto tab = [&](int a) { return *reinterpret_cast<const int32_t*>(smem + a); };
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) at[j] = tab(P.ex[j] + x) + tab(P.ey[j] + y) + tab(P.ez[j] + z);
 }
 
 // This thread's share of the fields' update for a swap: its site's coordinates
@@ -251,12 +263,10 @@ __device__ __forceinline__ void field_update(const FieldLayout& L, unsigned char
   using F = FieldVec<R == 0 ? 1 : R>;
   using T = typename F::T;
   const int rs = R == 0 ? r : R;
-  const int x = (xyz & 1023) << 2, y = (xyz >> 8) & 4092, z = (xyz >> 18) & 4092;
-  auto tab = [&](int at) { return *reinterpret_cast<const int32_t*>(smem + at); };
   int at[NJ];
+  field_sites<NJ>(smem, P, xyz, at);
 #pragma unroll
-  for (int j = 0; j < NJ; ++j)
-    at[j] = (int)L.g + 4 * rs * (tab(P.ex[j] + x) + tab(P.ey[j] + y) + tab(P.ez[j] + z));
+  for (int j = 0; j < NJ; ++j) at[j] = (int)L.g + 4 * rs * at[j];
   if (!distinct) {
     for (int p = 0; p < rs; ++p)
 #pragma unroll
@@ -288,7 +298,7 @@ __device__ __forceinline__ void field_update(const FieldLayout& L, unsigned char
   }
 }
 
-// The reference-order FP64 pair energies' difference e_swapped - e_unswapped
+// The reference-order FP64 pair energies before and after a swap
 // (exact_pair_energies: same values, same order): the neighbours' species of
 // both sites are gathered by all lanes, then lane c < 4 nsh adds, in list order
 // from 0.0, the terms of shell c % nsh of evaluation c / nsh (site 1 before,
@@ -303,7 +313,7 @@ __device__ __forceinline__ FieldExact field_exact_setup(const Geom& g, const Fie
           L.codes, L.lat};
 }
 
-static __device__ __noinline__ double field_exact_delta(const FieldExact X, int xyz1, int xyz2, int i1, int i2, int s1,
+static __device__ __noinline__ double2 field_exact_pair(const FieldExact X, int xyz1, int xyz2, int i1, int i2, int s1,
                                                         int s2, int lane) {
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t* ents = reinterpret_cast<const uint32_t*>(smem + X.ents);
@@ -350,7 +360,107 @@ static __device__ __noinline__ double field_exact_delta(const FieldExact X, int 
   }
   double e_un, e_sw;
   combine_pair_energies(part, nsh, lane, e_un, e_sw);
-  return __dsub_rn(e_sw, e_un);
+  return make_double2(e_un, e_sw);
+}
+
+// Named hardware barriers of the team's warps and the makers', per part h of
+// the record ring: its records are made (1 + h); they have been used (3 + h);
+// and of the makers alone (5).
+__device__ __forceinline__ void made_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(1 + h) : "memory"); }
+__device__ __forceinline__ void made_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory"); }
+__device__ __forceinline__ void used_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(3 + h) : "memory"); }
+__device__ __forceinline__ void used_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(3 + h) : "memory"); }
+__device__ __forceinline__ void makers_meet() { asm volatile("bar.sync 5, 128;" ::: "memory"); }
+
+// What the team tells the makers at the end.
+struct FieldEnd {
+  unsigned long long words;
+  int done;
+};
+
+// A making warp (`mine` of kFieldMakers): its window's static records of every
+// part, two parts at most before the team has used one, and its 32 words of the
+// stream one part further on.  test(w): the records' last word of A and third of
+// B from the acceptance word.
+template <class Test>
+__device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, const FieldLayout& L,
+                                              unsigned char* smem, FieldEnd* end, int mine, int lane, Test test) {
+  using Ring = FieldWords;
+  uint32_t* mt = reinterpret_cast<uint32_t*>(smem);
+  uint32_t* tw = mt + Ring::kTwAt;
+  const FieldGeom f = J.fg;
+  const uint8_t* dtab = smem + L.dtab;
+  const bool bcc = g.lattice == kBcc;
+  const bool nbr = J.nbr_swap != 0;
+  const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
+  const int pos0 = (int)J.rng[kMTN];
+  MtRoll R = {pos0, 0, 0};
+  if (mine == 0) {
+    mt_roll_load<Ring>(J.rng, mt, pos0, lane);
+    __syncwarp();
+#pragma unroll 1
+    for (int k = 0; k < kFieldAhead / kWin; ++k) {
+      mt_roll<Ring>(mt, tw, R, lane);
+      __syncwarp();
+    }
+  }
+  // this warp's rows of the stream: the first after those, then every fourth
+  R = {pos0 + kFieldAhead + mine * kWin, kFieldAhead + mine * kWin, kFieldAhead + mine * kWin};
+  unsigned long long made = kFieldAhead;
+  int at = mine * kWin;  // the window's place in the ring of tempered words
+  const int ns4 = 4 * g.ns, c_at = (int)L.C;
+  bool wrapped = false;  // two parts have been made
+  for (int h = 0;; h ^= 1) {
+    if (wrapped) used_wait(h);
+    wrapped = wrapped || h == 1;
+    if (*(volatile int*)&end->done) break;
+    makers_meet();  // the words of the part before
+    const uint32_t* w = tw + at + lane;
+    int ax, ay, az, Ya, Xa, bx, by, bz, Yb, Xb;
+    draw_site_halo(g, bcc, w[0], w[1], w[2], ax, ay, az, Ya, Xa);
+    if (nbr) {
+      // draw_nbr's neighbour; its steps are -1, 0, 1
+      const int8_t* v = cNbrSwap[g.lattice][umulhi32(w[3], (uint32_t)g.nbr_k)];
+      bx = wrap_fast(ax + v[0], W1);
+      by = wrap_fast(ay + v[1], W2);
+      bz = wrap_fast(az + v[2], W3);
+      Yb = by >> g.ys;
+      Xb = bx >> 1;
+    } else {
+      draw_site_halo(g, bcc, w[3], w[4], w[5], bx, by, bz, Yb, Xb);
+    }
+    const int2 th = test(w[nbr ? 4 : 6]);
+    const int t1 = wrap_fast(bx - ax + f.dm[0], W1), t2 = wrap_fast(by - ay + f.dm[1], W2),
+              t3 = wrap_fast(bz - az + f.dm[2], W3);
+    const int both = nbr || words_near(f.both_c, f.both_2c, w);  // a site may be around both
+    int cls = 0;
+    if (t1 < f.side[0] && t2 < f.side[1] && t3 < f.side[2]) cls = dtab[(t3 * f.side[1] + t2) * f.side[0] + t1];
+    const int ia = az * g.sz + Ya * g.sy + Xa, ib = bz * g.sz + Yb * g.sy + Xb;
+    const int slot = (kFieldMakers * h + mine) * kWin + lane;
+    *reinterpret_cast<int4*>(smem + FieldLayout::kA + slot * 16) =
+        make_int4(ia, ib, c_at + cls * g.ns * ns4, th.x);
+    *reinterpret_cast<int4*>(smem + FieldLayout::kB + slot * 16) =
+        make_int4(ax | ay << 10 | az << 20, bx | by << 10 | bz << 20, th.y, both);
+    mt_roll<Ring>(mt, tw, R, lane, kFieldMakers - 1);
+    made += kFieldPart;
+    at = at + kFieldPart >= Ring::kTw ? at + kFieldPart - Ring::kTw : at + kFieldPart;
+    made_arrive(h);
+  }
+  if (mine == 0) mt_roll_store<Ring>(mt, tw, R, pos0, end->words, made, J.rng, lane);
+}
+
+// Threads per chain: eight warps run the trials; the others share the staging and
+// the fields' first sums.  Chains that have an SM to themselves take 16 warps
+// (four on each scheduler).
+inline int field_threads(int n_jobs) {
+  static int n_sm = 0;
+  if (n_sm == 0) {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    n_sm = n;
+  }
+  return n_jobs <= n_sm ? 512 : 256;
 }
 
 }  // namespace brawl

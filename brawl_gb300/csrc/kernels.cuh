@@ -168,6 +168,7 @@ void preload_halo_kernels();
 void preload_field_kernels();
 void preload_ns_kernels();
 void preload_wl_kernels();
+void preload_wl_field_kernels();
 void preload_lattice_kernels();
 
 // Kernels of the chains that run in shared memory (fcc/bcc).

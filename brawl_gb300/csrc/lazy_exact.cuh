@@ -213,9 +213,9 @@ __device__ __forceinline__ bool in_quanta(double E, double E0, long long lo, lon
 // coordinate, the offsets within 1.8e-7 |offset| (three roundings), their
 // sums within 6e-8 |t|, and the reference's own t within 5e-16 |t|; m
 // doubles that.  Far outside (|t| >= 5e8) is left to the exact path.
-__device__ __forceinline__ bool bin_from_quanta(float t0, float qrf, long long lo, long long hi,
-                                                int& bin) {
-  const float plo = __fmul_rn(__ll2float_rn(lo), qrf), phi = __fmul_rn(__ll2float_rn(hi), qrf);
+// bin_from_floats takes lo and hi rounded to floats.
+__device__ __forceinline__ bool bin_from_floats(float t0, float qrf, float lo, float hi, int& bin) {
+  const float plo = __fmul_rn(lo, qrf), phi = __fmul_rn(hi, qrf);
   const float tlo = __fadd_rn(t0, plo), thi = __fadd_rn(t0, phi);
   if (!(fabsf(tlo) < 5.0e8f && fabsf(thi) < 5.0e8f)) return false;
   const float m = (fabsf(t0) + fmaxf(fabsf(tlo), fabsf(thi))) * 1.2e-7f +
@@ -226,33 +226,16 @@ __device__ __forceinline__ bool bin_from_quanta(float t0, float qrf, long long l
   return true;
 }
 
+__device__ __forceinline__ bool bin_from_quanta(float t0, float qrf, long long lo, long long hi, int& bin) {
+  return bin_from_floats(t0, qrf, __ll2float_rn(lo), __ll2float_rn(hi), bin);
+}
+
 enum LazyFold : int {
   kFoldWangLandau = 0,  // e = (e - pair_before) + pair_after
   kFoldNested = 1,      // e = e + (pair_after - pair_before)
 };
 
 constexpr int kLazyIlp = 8;  // chains per lane in flight
-
-// The species a chain's logged neighbour holds at its evaluation (before or
-// after the move).
-__device__ __forceinline__ int lazy_species(const LazyLog& L, int at, int s_before, int s_after,
-                                            bool after) {
-  const int code = (int)L.codes[at];
-  int s = code & 0x3f;
-  if (after) {
-    if (code & kLazyPartner) s = s_before;  // the partner now holds our old species
-    else if (code & kLazySelf) s = s_after;
-  }
-  return s;
-}
-
-// One logged neighbour's term V(cs, s, shell) of a chain (0 for a lane's
-// chain slot past the last chain: adding 0.0 to the unused sums).
-__device__ __forceinline__ double lazy_term(const LazyLog& L, const double* Vsh, int at, int cs,
-                                            int s_before, int s_after, bool after, bool on, int ns) {
-  if (!on) return 0.0;
-  return Vsh[(cs - 1) + ns * (lazy_species(L, at, s_before, s_after, after) - 1)];
-}
 
 // bar.sync on named barrier `id` for `count` threads (a multiple of 32):
 // the warps of a block that share a deferred-energy log meet there.
@@ -274,51 +257,76 @@ __device__ __forceinline__ void lazy_sites(const Geom& g, const double* V, const
                                            const LazyLog& L, int n, int fold, int tid, int nthreads) {
   const int z = g.z, nsh = g.nsh, ns = g.ns;
   const int nch = 4 * n;
+  constexpr int kAhead = ILP <= 2 ? 8 : 4;  // terms loaded ahead of their adds
   for (int c0 = 0; c0 < nch; c0 += nthreads * ILP) {
-    int row[ILP], cs[ILP], s_before[ILP], s_after[ILP];
-    bool on[ILP], after[ILP];
+    const uint8_t* row[ILP];  // the chain's neighbour codes
+    int cs[ILP], met[ILP];    // its centre's species; what it finds at the other site
+    bool on[ILP];
     double site[ILP];
 #pragma unroll
     for (int i = 0; i < ILP; ++i) {
       const int c = c0 + nthreads * i + tid;
       on[i] = c < nch;
       const int m = on[i] ? c >> 2 : 0, ev = c & 3;
-      const bool site2 = ev & 1;
-      after[i] = ev >= 2;
+      const bool site2 = ev & 1, after = ev >= 2;
       const int sa = L.spec[2 * m], sb = L.spec[2 * m + 1];
-      s_before[i] = site2 ? sb : sa;  // the site's own species before the move
-      s_after[i] = site2 ? sa : sb;
-      cs[i] = after[i] ? s_after[i] : s_before[i];
-      row[i] = m * 2 * z + (site2 ? z : 0);
+      const int before = site2 ? sb : sa, then = site2 ? sa : sb;
+      cs[i] = after ? then : before;
+      // after the move the partner holds our old species, a site that is its
+      // own neighbour its new one; before it the codes' own
+      met[i] = after ? (before | then << 8) : 0;
+      row[i] = L.codes + m * 2 * z + (site2 ? z : 0);
       site[i] = 0.0;
     }
     for (int sh = 0; sh < nsh; ++sh) {
       const int k0 = sstart[sh], len = sstart[sh + 1] - k0;
-      const double* Vsh = V + ns * ns * sh;
+      const double* Vr[ILP];
       double sum[ILP];
 #pragma unroll
-      for (int i = 0; i < ILP; ++i) sum[i] = 0.0;
+      for (int i = 0; i < ILP; ++i) {
+        Vr[i] = V + ns * ns * sh + (cs[i] - 1) - ns;  // + ns * species
+        sum[i] = 0.0;
+      }
+      auto term = [&](int i, int code) {
+        int s = code & 0x3f;
+        if (code & (kLazyPartner | kLazySelf))
+          if (met[i]) s = (code & kLazyPartner) ? (met[i] & 0xff) : (met[i] >> 8);
+        return on[i] ? Vr[i][ns * s] : 0.0;
+      };
       int k = 0;
-      // the terms of four neighbours of every chain are loaded before
-      // their adds, so the loads overlap and the adds issue back to back;
-      // each chain still adds its terms in list order
-      for (; k + 4 <= len; k += 4) {
-        double t[ILP][4];
+      // the terms of kAhead neighbours of every chain are loaded before their
+      // adds, so the loads overlap and the adds issue back to back; each chain
+      // still adds its terms in list order
+      for (; k + kAhead <= len; k += kAhead) {
+        int code[ILP][kAhead];
+        double t[ILP][kAhead];
 #pragma unroll
         for (int i = 0; i < ILP; ++i)
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            t[i][u] = lazy_term(L, Vsh, row[i] + k0 + k + u, cs[i], s_before[i], s_after[i], after[i], on[i], ns);
+          for (int u = 0; u < kAhead; ++u) code[i][u] = row[i][k0 + k + u];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int i = 0; i < ILP; ++i)
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) t[i][u] = term(i, code[i][u]);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
 #pragma unroll
           for (int i = 0; i < ILP; ++i) sum[i] = __dadd_rn(sum[i], t[i][u]);
       }
-      for (; k < len; ++k) {
+      for (; k + 2 <= len; k += 2) {
+        double t[ILP][2];
 #pragma unroll
         for (int i = 0; i < ILP; ++i)
-          sum[i] = __dadd_rn(sum[i], lazy_term(L, Vsh, row[i] + k0 + k, cs[i], s_before[i], s_after[i],
-                                               after[i], on[i], ns));
+#pragma unroll
+          for (int u = 0; u < 2; ++u) t[i][u] = term(i, row[i][k0 + k + u]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int i = 0; i < ILP; ++i) sum[i] = __dadd_rn(sum[i], t[i][u]);
+      }
+      if (k < len) {
+#pragma unroll
+        for (int i = 0; i < ILP; ++i) sum[i] = __dadd_rn(sum[i], term(i, row[i][k0 + k]));
       }
       // site energy: shell 1 + shell 2 + ... left to right
 #pragma unroll

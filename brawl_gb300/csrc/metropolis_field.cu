@@ -4,99 +4,8 @@
 // src/metropolis.F90:751-891) on the chain's own mt19937ar stream.
 #include "accept_thresholds.cuh"
 #include "field_engine.cuh"
-#include "halo_engine.cuh"
 
 namespace brawl {
-
-namespace {
-
-// Named hardware barriers of the team's warps and the makers', per part h of
-// the record ring: its records are made (1 + h); they have been used (3 + h);
-// and of the makers alone (5).
-__device__ __forceinline__ void made_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(1 + h) : "memory"); }
-__device__ __forceinline__ void made_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory"); }
-__device__ __forceinline__ void used_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(3 + h) : "memory"); }
-__device__ __forceinline__ void used_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(3 + h) : "memory"); }
-__device__ __forceinline__ void makers_meet() { asm volatile("bar.sync 5, 128;" ::: "memory"); }
-
-// What the team tells the makers at the end.
-struct FieldEnd {
-  unsigned long long words;
-  int done;
-};
-
-// A making warp (`mine` of kFieldMakers): its window's static records of every
-// part, two parts at most before the team has used one, and its 32 words of the
-// stream one part further on.
-__device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, const FieldLayout& L,
-                                              unsigned char* smem, FieldEnd* end, int mine, int lane) {
-  using Ring = FieldWords;
-  uint32_t* mt = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* tw = mt + Ring::kTwAt;
-  const FieldGeom f = J.fg;
-  const uint8_t* dtab = smem + L.dtab;
-  const bool bcc = g.lattice == kBcc;
-  const bool nbr = J.nbr_swap != 0;
-  const int band = J.band;
-  const float inv_k = 1.0f / J.beta_q_l2, band_f = (float)band;
-  const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
-  const int pos0 = (int)J.rng[kMTN];
-  MtRoll R = {pos0, 0, 0};
-  if (mine == 0) {
-    mt_roll_load<Ring>(J.rng, mt, pos0, lane);
-    __syncwarp();
-#pragma unroll 1
-    for (int k = 0; k < kFieldAhead / kWin; ++k) {
-      mt_roll<Ring>(mt, tw, R, lane);
-      __syncwarp();
-    }
-  }
-  // this warp's rows of the stream: the first after those, then every fourth
-  R = {pos0 + kFieldAhead + mine * kWin, kFieldAhead + mine * kWin, kFieldAhead + mine * kWin};
-  unsigned long long made = kFieldAhead;
-  int at = mine * kWin;  // the window's place in the ring of tempered words
-  const int ns4 = 4 * g.ns, c_at = (int)L.C;
-  bool wrapped = false;  // two parts have been made
-  for (int h = 0;; h ^= 1) {
-    if (wrapped) used_wait(h);
-    wrapped = wrapped || h == 1;
-    if (*(volatile int*)&end->done) break;
-    makers_meet();  // the words of the part before
-    const uint32_t* w = tw + at + lane;
-    int ax, ay, az, Ya, Xa, bx, by, bz, Yb, Xb;
-    draw_site_halo(g, bcc, w[0], w[1], w[2], ax, ay, az, Ya, Xa);
-    if (nbr) {
-      // draw_nbr's neighbour; its steps are -1, 0, 1
-      const int8_t* v = cNbrSwap[g.lattice][umulhi32(w[3], (uint32_t)g.nbr_k)];
-      bx = wrap_fast(ax + v[0], W1);
-      by = wrap_fast(ay + v[1], W2);
-      bz = wrap_fast(az + v[2], W3);
-      Yb = by >> g.ys;
-      Xb = bx >> 1;
-    } else {
-      draw_site_halo(g, bcc, w[3], w[4], w[5], bx, by, bz, Yb, Xb);
-    }
-    const AcceptThresholds th = accept_thresholds(w[nbr ? 4 : 6], inv_k, band_f);
-    const int t1 = wrap_fast(bx - ax + f.dm[0], W1), t2 = wrap_fast(by - ay + f.dm[1], W2),
-              t3 = wrap_fast(bz - az + f.dm[2], W3);
-    const int both = nbr || words_near(f.both_c, f.both_2c, w);  // a site may be around both
-    int cls = 0;
-    if (t1 < f.side[0] && t2 < f.side[1] && t3 < f.side[2]) cls = dtab[(t3 * f.side[1] + t2) * f.side[0] + t1];
-    const int ia = az * g.sz + Ya * g.sy + Xa, ib = bz * g.sz + Yb * g.sy + Xb;
-    const int slot = (kFieldMakers * h + mine) * kWin + lane;
-    *reinterpret_cast<int4*>(smem + FieldLayout::kA + slot * 16) =
-        make_int4(ia, ib, c_at + cls * g.ns * ns4, max(band, th.rej_above));
-    *reinterpret_cast<int4*>(smem + FieldLayout::kB + slot * 16) =
-        make_int4(ax | ay << 10 | az << 20, bx | by << 10 | bz << 20, th.acc_below, both);
-    mt_roll<Ring>(mt, tw, R, lane, kFieldMakers - 1);
-    made += kFieldPart;
-    at = at + kFieldPart >= Ring::kTw ? at + kFieldPart - Ring::kTw : at + kFieldPart;
-    made_arrive(h);
-  }
-  if (mine == 0) mt_roll_store<Ring>(mt, tw, R, pos0, end->words, made, J.rng, lane);
-}
-
-}  // namespace
 
 // The walk through a window of decided positions from this lane's position: like
 // pairs (accepted without an energy evaluation or a draw) and certain
@@ -154,7 +63,13 @@ __global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob
   // Warps 2, 3, 6 and 7 are the team (the schedulers take every fourth warp, so
   // it has two of them to itself), 0, 1, 4 and 5 the makers.
   if (warp < 8 && (warp & 2) == 0) {
-    field_produce(J, g, L, smem, &end, (warp & 1) + (warp >> 1), lane);
+    // A's last word: the larger of rej_above and the band; B's third: acc_below
+    const int band = J.band;
+    const float inv_k = 1.0f / J.beta_q_l2, band_f = (float)band;
+    field_produce(J, g, L, smem, &end, (warp & 1) + (warp >> 1), lane, [=](uint32_t w) {
+      const AcceptThresholds th = accept_thresholds(w, inv_k, band_f);
+      return make_int2(max(band, th.rej_above), th.acc_below);
+    });
   } else if (warp < 8) {
     const int who = (warp & 1) + (warp >> 2) * 2, tt = who * 32 + lane;
     const bool second = tt >= kFieldHalf;
@@ -252,8 +167,9 @@ __global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob
         // sums, in its order
         ++b_exact;
         if (who == 0) {
-          const double delta_e = field_exact_delta(field_exact_setup(g, L), q.x, q.y, a.x, a.y, (s1 >> 2) + 1,
-                                                   (s2 >> 2) + 1, lane);
+          const double2 pair = field_exact_pair(field_exact_setup(g, L), q.x, q.y, a.x, a.y, (s1 >> 2) + 1,
+                                                (s2 >> 2) + 1, lane);
+          const double delta_e = __dsub_rn(pair.y, pair.x);
           int verdict = 1;
           if (!(delta_e < 0.0)) {
             DecideStats st = {0u, 0u};
@@ -315,20 +231,6 @@ __global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob
   for (int i = tid; i < n4; i += blockDim.x) dst[i] = ((src[i] >> 2) & 0x3f3f3f3fu) + 0x01010101u;
   for (int i = (n4 << 2) + tid; i < g.n_sites; i += blockDim.x) J.lat[i] = (int8_t)((smem[L.lat + i] >> 2) + 1);
   if (tid == 0 && J.t_ns) *J.t_ns = global_ns() - t_start;
-}
-
-// Threads per chain: eight warps run the trials; the others share the staging and
-// the fields' first sums.  Chains that have an SM to themselves take 16 warps
-// (four on each scheduler).
-static int field_threads(int n_jobs) {
-  static int n_sm = 0;
-  if (n_sm == 0) {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    n_sm = n;
-  }
-  return n_jobs <= n_sm ? 512 : 256;
 }
 
 template <int NJ, int R>

@@ -741,10 +741,14 @@ int launch_wl(brawl_server* S, Pipe& P) {
   std::vector<int> ej_walker;
   std::vector<uint32_t> w_smem;
   std::vector<int> w_z;
+  std::vector<int> w_kind;
   std::vector<char> w_D;
   int max_bins = 0;
   std::stable_sort(P.jobs.begin(), P.jobs.end(),
-                   [](const JobP& a, const JobP& b) { return api_wl_smem(a->wl) > api_wl_smem(b->wl); });
+                   [](const JobP& a, const JobP& b) {
+                     const int ka = api_wl_kind(a->wl), kb = api_wl_kind(b->wl);
+                     return ka != kb ? ka > kb : api_wl_smem(a->wl) > api_wl_smem(b->wl);
+                   });
   P.launched = P.jobs;
   P.call_ends.assign(P.launched.size(), 0);
   size_t n_all = 0;
@@ -784,6 +788,7 @@ int launch_wl(brawl_server* S, Pipe& P) {
     api_wl_variant(j.wl, &jz, &jd);
     w_smem.insert(w_smem.end(), w.size(), api_wl_smem(j.wl));
     w_z.insert(w_z.end(), w.size(), jz);
+    w_kind.insert(w_kind.end(), w.size(), api_wl_kind(j.wl));
     w_D.insert(w_D.end(), w.size(), jd ? 1 : 0);
     max_bins = std::max(max_bins, j.d.wl_bins);
   }
@@ -798,14 +803,17 @@ int launch_wl(brawl_server* S, Pipe& P) {
   SV_TRY(grow_host(P.h_flat, P.h_flat_cap, (size_t)n));
   SV_TRY(stage_copy(P, P.d_wl, staged.data(), n * sizeof(WlWalker)));
   if (!groups.empty()) SV_TRY(stage_copy(P, P.d_groups, groups.data(), groups.size() * sizeof(WlGroup)));
-  SV_TRY(launch_groups(P, smem_groups(w_smem), [&](int first, int count, cudaStream_t st) {
+  SV_TRY(launch_groups(P, smem_groups(w_smem, &w_kind), [&](int first, int count, cudaStream_t st) {
     int max_z = 0;
     bool all_D = true;
     for (int k = first; k < first + count; ++k) {
       max_z = std::max(max_z, w_z[k]);
       all_D = all_D && w_D[k];
     }
-    launch_wl_sweeps(P.d_wl + first, count, w_smem[first], max_z, all_D, st);
+    if (w_kind[first])
+      launch_wl_field(P.d_wl + first, count, w_smem[first], max_z, w_kind[first] - 8, st);
+    else
+      launch_wl_sweeps(P.d_wl + first, count, w_smem[first], max_z, all_D, st);
   }));
   if (!groups.empty()) launch_wl_average(P.d_groups, (int)groups.size(), P.d_wl, max_bins, 1, P.s);
   launch_wl_flatness(P.d_wl, n, P.d_flat, P.s);
@@ -1228,6 +1236,7 @@ int brawl_serve_create(const brawl_server_opts* opts, brawl_server** out) {
   preload_field_kernels();
   preload_ns_kernels();
   preload_wl_kernels();
+  preload_wl_field_kernels();
   preload_lattice_kernels();
   {
     cudaFuncAttributes a;

@@ -37,6 +37,8 @@ struct WlWalker {
   double* e_state;
   int32_t S;             // fixed-point shift of the chain's F table
   int32_t lazy_cap;      // moves the deferred-energy log holds (>= 1)
+  int32_t field_cap;     // the same with fields (wl_field.cu); 0: they do not fit
+  int32_t pad;
   // radial-density samples (all null when off): the plan, this walker's
   // radial_record (bins), rho_of_E (bins x wc x ns x ns, rho(i, j, l, bin)
   // with i fastest) and radial_mc_steps
@@ -82,6 +84,10 @@ uint32_t wl_smem_bytes(const Geom& g, int nb, int lazy_cap, int rad_bins = 0, in
 // difference table D is staged (walker_layout's use_D).
 void launch_wl_sweeps(WlWalker* d_walkers, int n, uint32_t smem, int max_z, bool all_D,
                       cudaStream_t stream);
+// The same with the sites' fields in shared memory (wl_field.cu), for walkers
+// with a field_cap, of one field_variant and without radial samples.
+uint32_t wl_field_smem_bytes(const Geom& g, const FieldGeom& f, int nb, int cap);
+void launch_wl_field(WlWalker* d_walkers, int n, uint32_t smem, int max_z, int variant, cudaStream_t stream);
 void launch_wl_average(const WlGroup* d_groups, int n_groups, WlWalker* d_walkers, int bins,
                        int with_hist, cudaStream_t stream);
 uint32_t wl_exchange_smem_bytes(int per_window);

@@ -1,0 +1,96 @@
+"""The kernels that keep a chain in shared memory (fields of the sites, or
+gathered sums in rounds) at the edges of what they take: neighbour counts on
+both sides of 64 and 128, lattices that an offset spans (a site met by two
+offsets), shells without every offset's opposite, one to five fields a site,
+nbr_swap, and calls of none, one and a few trials.  Against the oracle, bit for
+bit: configurations, accepted moves, streams, ln g and histograms."""
+import numpy as np
+import pytest
+
+import brawl_gb300 as B
+from oracle import oracle as O
+from tests.test_gpu_metropolis import conc_vector, random_V
+from tests.test_gpu_wang_landau import _emulate
+
+pytestmark = pytest.mark.gpu
+
+# lattice, n, ns, nsh, nbr_swap
+EDGES = [
+    ("fcc", (2, 2, 2), 2, 2, False),    # offsets of n: a site is met twice
+    ("bcc", (2, 3, 2), 3, 2, True),
+    ("fcc", (3, 5, 7), 3, 3, True),
+    ("bcc", (4, 4, 4), 5, 6, False),
+    ("fcc", (4, 5, 4), 6, 6, False),    # five fields: no vector variant
+    ("bcc", (5, 4, 4), 2, 10, False),   # z > 128, not every shell symmetric
+    ("bcc", (4, 4, 5), 4, 8, False),
+]
+
+
+def _chain(case, k):
+    lattice, n, ns, nsh, nbr = case
+    V = random_V(np.random.default_rng(100 + k), ns, nsh)
+    mod = O.OracleModel(lattice, *n, V)
+    r = O.OracleRng(7000 + k)
+    cfg, _ = mod.initial_setup(r, conc_vector(ns))
+    return V, mod, r, cfg
+
+
+@pytest.mark.parametrize("depth", [1, 2, 3, 4])
+def test_chains_at_the_edges_match_oracle(depth):
+    chains, ref = [], []
+    for k, case in enumerate(EDGES):
+        V, mod, r, cfg = _chain(case, k)
+        T = (300.0, 1500.0, 6000.0)[k % 3]
+        chains.append(dict(setup=B.Setup(case[0], *case[1], case[2], case[3]), V=V, seed=7000 + k,
+                           beta=1.0 / (T * B.K_B_IN_RY), nbr_swap=case[4],
+                           species_concentrations=conc_vector(case[2])))
+        ref.append((mod, r, cfg, chains[-1]["beta"], case[4]))
+    b = B.Batch(chains)
+    b.set_speculation(depth)
+    for trials in (0, 1, 2, 5, 64, 3001):
+        acc = b.metropolis(trials)
+        for k, (mod, r, cfg, beta, nbr) in enumerate(ref):
+            a, _ = mod.mc_run(cfg, r, beta, trials, nbr)
+            assert acc[k] == a, (EDGES[k], trials)
+            assert np.array_equal(b.config(k), cfg), (EDGES[k], trials)
+            assert _same_stream(b.rng_state(k), r), (EDGES[k], trials)
+
+
+def _same_stream(words, r):
+    g, h = O.OracleRng(1), O.OracleRng(1)
+    g.set_state_words(words)
+    h.set_state_words(r.state_words())
+    return [g.u32() for _ in range(640)] == [h.u32() for _ in range(640)]
+
+
+@pytest.mark.parametrize("wl_f,period", [(0.0, 1), (2.0 ** -31, 3), (0.05, 7), (1.5, 1), (1.0e5, 40)])
+def test_wang_landau_at_the_edges_matches_oracle(wl_f, period):
+    """ln f of none, below the fixed point of ln g, and beyond it."""
+    for k, case in enumerate(EDGES):
+        lattice, n, ns, nsh, nbr = case
+        V, mod, r, cfg = _chain(case, k)
+        bins = 24
+        e0 = mod.total_energy(cfg)
+        step = 0.004 * (1 + k % 3)
+        edges = e0 - step * bins / 2 + np.arange(bins + 1) * step
+        walkers, cfgs, rngs = [], [], []
+        for w, (lo, hi) in enumerate([(1, bins), (9, 17), (12, 14)]):
+            walkers.append(dict(setup=B.Setup(lattice, *n, ns, nsh), V=V, seed=50 + w, config=cfg.copy(),
+                                start_idx=lo, end_idx=hi, window=w, nbr_swap=nbr))
+            cfgs.append(cfg.copy())
+            rngs.append(O.OracleRng(50 + w))
+        mods = [O.OracleModel(lattice, *n, V) for _ in walkers]
+        lngs = [np.zeros(bins) for _ in walkers]
+        hists = [np.zeros(w["end_idx"] - w["start_idx"] + 1) for w in walkers]
+        wl = B.WangLandauWalkers(walkers, edges)
+        # (where a shell lacks an offset's opposite, a walk's energy is not the
+        # configuration's, from which the next call starts: one call)
+        for trials in (1, 2, 37, 1500) if nsh < 10 else (1500,):
+            acc_o = _emulate(mods, cfgs, rngs, walkers, edges, lngs, hists, trials, wl_f, period)
+            assert list(wl.sweeps(trials, wl_f, period)) == acc_o, (case, trials)
+            for w in range(len(walkers)):
+                assert np.array_equal(wl.lng(w), lngs[w]), (case, trials)
+                assert np.array_equal(wl.hist(w), hists[w]), (case, trials)
+                assert np.array_equal(wl.config(w), cfgs[w]), (case, trials)
+        for w in range(len(walkers)):
+            assert np.array_equal(wl.genrand(w, 20), np.array([rngs[w].uniform() for _ in range(20)]))
