@@ -363,13 +363,25 @@ static __device__ __noinline__ double2 field_exact_pair(const FieldExact X, int 
   return make_double2(e_un, e_sw);
 }
 
-// Named hardware barriers of the team's warps and the makers', per part h of
-// the record ring: its records are made (1 + h); they have been used (3 + h);
-// and of the makers alone (5).
-__device__ __forceinline__ void made_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(1 + h) : "memory"); }
-__device__ __forceinline__ void made_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory"); }
-__device__ __forceinline__ void used_arrive(int h) { asm volatile("bar.arrive %0, 256;" ::"r"(3 + h) : "memory"); }
-__device__ __forceinline__ void used_wait(int h) { asm volatile("bar.sync %0, 256;" ::"r"(3 + h) : "memory"); }
+// Named hardware barriers of the team's warps and the makers' (N threads
+// together), per part h of the record ring: its records are made (1 + h); they
+// have been used (3 + h); and of the makers alone (5).
+template <int N = kFieldTeam + 32 * kFieldMakers>
+__device__ __forceinline__ void made_arrive(int h) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1 + h), "n"(N) : "memory");
+}
+template <int N = kFieldTeam + 32 * kFieldMakers>
+__device__ __forceinline__ void made_wait(int h) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + h), "n"(N) : "memory");
+}
+template <int N = kFieldTeam + 32 * kFieldMakers>
+__device__ __forceinline__ void used_arrive(int h) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(3 + h), "n"(N) : "memory");
+}
+template <int N = kFieldTeam + 32 * kFieldMakers>
+__device__ __forceinline__ void used_wait(int h) {
+  asm volatile("bar.sync %0, %1;" ::"r"(3 + h), "n"(N) : "memory");
+}
 __device__ __forceinline__ void makers_meet() { asm volatile("bar.sync 5, 128;" ::: "memory"); }
 
 // What the team tells the makers at the end.
@@ -380,23 +392,18 @@ struct FieldEnd {
 
 // A making warp (`mine` of kFieldMakers): its window's static records of every
 // part, two parts at most before the team has used one, and its 32 words of the
-// stream one part further on.  test(w): the records' last word of A and third of
-// B from the acceptance word.
-template <class Test>
-__device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, const FieldLayout& L,
-                                              unsigned char* smem, FieldEnd* end, int mine, int lane, Test test) {
+// stream one part further on.  make(w, slot): the record at place `slot` of the
+// ring, of the position of words w[0], w[1], ...  N: the threads of the barriers.
+template <int N = kFieldTeam + 32 * kFieldMakers, class Make>
+__device__ __forceinline__ void stream_produce(uint32_t* rng, unsigned char* smem, FieldEnd* end, int mine, int lane,
+                                               Make make) {
   using Ring = FieldWords;
   uint32_t* mt = reinterpret_cast<uint32_t*>(smem);
   uint32_t* tw = mt + Ring::kTwAt;
-  const FieldGeom f = J.fg;
-  const uint8_t* dtab = smem + L.dtab;
-  const bool bcc = g.lattice == kBcc;
-  const bool nbr = J.nbr_swap != 0;
-  const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
-  const int pos0 = (int)J.rng[kMTN];
+  const int pos0 = (int)rng[kMTN];
   MtRoll R = {pos0, 0, 0};
   if (mine == 0) {
-    mt_roll_load<Ring>(J.rng, mt, pos0, lane);
+    mt_roll_load<Ring>(rng, mt, pos0, lane);
     __syncwarp();
 #pragma unroll 1
     for (int k = 0; k < kFieldAhead / kWin; ++k) {
@@ -408,14 +415,33 @@ __device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, 
   R = {pos0 + kFieldAhead + mine * kWin, kFieldAhead + mine * kWin, kFieldAhead + mine * kWin};
   unsigned long long made = kFieldAhead;
   int at = mine * kWin;  // the window's place in the ring of tempered words
-  const int ns4 = 4 * g.ns, c_at = (int)L.C;
   bool wrapped = false;  // two parts have been made
   for (int h = 0;; h ^= 1) {
-    if (wrapped) used_wait(h);
+    if (wrapped) used_wait<N>(h);
     wrapped = wrapped || h == 1;
     if (*(volatile int*)&end->done) break;
     makers_meet();  // the words of the part before
-    const uint32_t* w = tw + at + lane;
+    make(tw + at + lane, (kFieldMakers * h + mine) * kWin + lane);
+    mt_roll<Ring>(mt, tw, R, lane, kFieldMakers - 1);
+    made += kFieldPart;
+    at = at + kFieldPart >= Ring::kTw ? at + kFieldPart - Ring::kTw : at + kFieldPart;
+    made_arrive<N>(h);
+  }
+  if (mine == 0) mt_roll_store<Ring>(mt, tw, R, pos0, end->words, made, rng, lane);
+}
+
+// stream_produce for trials (records A and B).  test(w): the records' last word
+// of A and third of B from the acceptance word.
+template <class Test>
+__device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, const FieldLayout& L,
+                                              unsigned char* smem, FieldEnd* end, int mine, int lane, Test test) {
+  const FieldGeom f = J.fg;
+  const uint8_t* dtab = smem + L.dtab;
+  const bool bcc = g.lattice == kBcc;
+  const bool nbr = J.nbr_swap != 0;
+  const int W1 = 2 * g.n1, W2 = 2 * g.n2, W3 = 2 * g.n3;
+  const int ns4 = 4 * g.ns, c_at = (int)L.C;
+  stream_produce(J.rng, smem, end, mine, lane, [&](const uint32_t* w, int slot) {
     int ax, ay, az, Ya, Xa, bx, by, bz, Yb, Xb;
     draw_site_halo(g, bcc, w[0], w[1], w[2], ax, ay, az, Ya, Xa);
     if (nbr) {
@@ -436,17 +462,11 @@ __device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, 
     int cls = 0;
     if (t1 < f.side[0] && t2 < f.side[1] && t3 < f.side[2]) cls = dtab[(t3 * f.side[1] + t2) * f.side[0] + t1];
     const int ia = az * g.sz + Ya * g.sy + Xa, ib = bz * g.sz + Yb * g.sy + Xb;
-    const int slot = (kFieldMakers * h + mine) * kWin + lane;
     *reinterpret_cast<int4*>(smem + FieldLayout::kA + slot * 16) =
         make_int4(ia, ib, c_at + cls * g.ns * ns4, th.x);
     *reinterpret_cast<int4*>(smem + FieldLayout::kB + slot * 16) =
         make_int4(ax | ay << 10 | az << 20, bx | by << 10 | bz << 20, th.y, both);
-    mt_roll<Ring>(mt, tw, R, lane, kFieldMakers - 1);
-    made += kFieldPart;
-    at = at + kFieldPart >= Ring::kTw ? at + kFieldPart - Ring::kTw : at + kFieldPart;
-    made_arrive(h);
-  }
-  if (mine == 0) mt_roll_store<Ring>(mt, tw, R, pos0, end->words, made, J.rng, lane);
+  });
 }
 
 // Threads per chain: eight warps run the trials; the others share the staging and

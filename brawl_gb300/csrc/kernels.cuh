@@ -167,6 +167,7 @@ void preload_metropolis_kernels();
 void preload_halo_kernels();
 void preload_field_kernels();
 void preload_ns_kernels();
+void preload_ns_rounds_kernels();
 void preload_wl_kernels();
 void preload_wl_field_kernels();
 void preload_lattice_kernels();

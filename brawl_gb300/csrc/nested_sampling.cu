@@ -63,35 +63,6 @@ __global__ void ns_jitter_kernel(NsRun* __restrict__ runs, int n_runs) {
   }
 }
 
-// Order-preserving integer key of a double (larger double, larger key).
-__device__ __forceinline__ unsigned long long dkey(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-
-// Fixed-point lower bound of the room under the ceiling: Gdn <= (pred(limit)
-// - E) * 2^S, pred(limit) the largest double below it; a step with
-// dE + band <= Gdn certainly lands strictly below the ceiling.
-__device__ __forceinline__ long long gap_dn(double limit, double E, int S) {
-  const double gd = __dsub_rd(nextafter(limit, -__longlong_as_double(0x7ff0000000000000LL)), E);
-  const double m = __dsub_rd(gd, __dmul_ru(fabs(gd), 8.881784197001252e-16));  // - |gd| 2^-50
-  const double s = ldexp(m, S);
-  if (!(s > -9.0e18)) return -0x7fffffffffffffffll;
-  if (s > 9.0e18) return 0x7fffffffffffffffll;
-  return (long long)floor(s);
-}
-
-// Fixed-point upper bound of the ceiling gap: Gup >= (limit - E) * 2^S.
-__device__ __forceinline__ long long gap_up(double limit, double E, int S) {
-  const double gd = __dsub_rn(limit, E);
-  const double m = __dadd_rn(gd, __dmul_rn(fabs(gd), 8.881784197001252e-16));  // + |gd| 2^-50
-  const double s = ldexp(m, S);
-  if (!(s < 9.0e18)) return 0x7fffffffffffffffll;
-  if (s < -9.0e18) return -0x7fffffffffffffffll;
-  return (long long)ceil(s);
-}
-
-
 // site-2 redraws tried at once, one per lane (3 words each, within the
 // ring's mirror)
 constexpr int kRedraws = 32;
@@ -163,7 +134,7 @@ __global__ void __launch_bounds__(32 * kNsWarps, 1) ns_iterate_kernel(NsRun* __r
     unsigned long long best = 0;
     int bidx = 0x7fffffff;
     for (int w = lane; w < K; w += 32) {
-      const unsigned long long k = dkey(R.energies[w]);
+      const unsigned long long k = ns_dkey(R.energies[w]);
       if (k > best || (k == best && w < bidx)) {
         best = k;
         bidx = w;
@@ -204,8 +175,8 @@ __global__ void __launch_bounds__(32 * kNsWarps, 1) ns_iterate_kernel(NsRun* __r
     int n_log = 0;
     __syncwarp();
     auto rebase = [&]() {
-      gup = gap_up(limit, E, S);
-      gdn = gap_dn(limit, E, S);
+      gup = ns_gap_up(limit, E, S);
+      gdn = ns_gap_dn(limit, E, S);
       Eq = quanta_bound(E, S);
       Dlo = Dhi = Rs = 0;
     };

@@ -1235,6 +1235,7 @@ int brawl_serve_create(const brawl_server_opts* opts, brawl_server** out) {
   preload_halo_kernels();
   preload_field_kernels();
   preload_ns_kernels();
+  preload_ns_rounds_kernels();
   preload_wl_kernels();
   preload_wl_field_kernels();
   preload_lattice_kernels();
