@@ -2597,6 +2597,12 @@ extern "C" int brawl_wl_enter_windows(brawl_wl* wl, double energy_min, double en
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
   std::vector<WlEnterJob> jobs(n);
   uint32_t smem = 0;
+  // with the sites' fields (wl_enter.cu): where wl_plan_fields would have the
+  // sweeps so, but for the window's tables
+  bool fields = true;
+  uint32_t field_smem = 0;
+  int max_z = 0;
+  const int variant = field_variant(b->models[0].g.ns);
   int64_t scratch = 0;
   std::vector<int64_t> off(n);
   for (int c = 0; c < n; ++c) {
@@ -2641,11 +2647,20 @@ extern "C" int brawl_wl_enter_windows(brawl_wl* wl, double energy_min, double en
     E.max_steps = max_steps;
     E.site_e = d_site_e + off[c];
     E.initial = initial ? 1 : 0;
+    E.S = m.S;
+    E.job.nbr_swap = 0;  // two sites are drawn, whatever the walker's sweeps do
     smem = std::max(smem, wl_enter_smem_bytes(m.g));
+    max_z = std::max(max_z, (int)m.g.z);
+    const FieldGeom& f = E.job.fg;
+    if (f.n_class > 0 && f.symmetric)
+      E.field_cap = lazy_cap_for(m.g, wl_enter_field_smem_bytes(m.g, f, 0), (uint32_t)max_optin);
+    if (E.field_cap < 16 || field_variant(m.g.ns) != variant) fields = false;
+    else field_smem = std::max(field_smem, wl_enter_field_smem_bytes(m.g, f, E.field_cap));
   }
   if (smem > (uint32_t)max_optin) return cleanup(fail(BRAWL_EINVAL, "lattice too large for the burn-in kernel"));
   CUDA_TRY(cudaMemcpyAsync(d_jobs, jobs.data(), (size_t)n * sizeof(WlEnterJob), cudaMemcpyHostToDevice, s));
-  launch_wl_enter(d_jobs, n, smem, s);
+  if (fields) launch_wl_enter_field(d_jobs, n, field_smem, max_z, variant, s);
+  else launch_wl_enter(d_jobs, n, smem, s);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(jobs.data(), d_jobs, (size_t)n * sizeof(WlEnterJob), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(stream_wait(s));

@@ -384,6 +384,24 @@ __device__ __forceinline__ void used_wait(int h) {
 }
 __device__ __forceinline__ void makers_meet() { asm volatile("bar.sync 5, 128;" ::: "memory"); }
 
+// The walk through a window of decided positions from this lane's position: like
+// pairs (accepted without an energy evaluation or a draw) and certain
+// rejections are passed, up to a trial that is neither or past the window.
+// Bits 0-7: that position (32 and more: past the window), 8-15: trials passed,
+// 16-23: rejections among them.
+__device__ __forceinline__ unsigned field_walk(unsigned like, unsigned rej, int lane, int n_base, bool nbr) {
+  unsigned path = 1u << lane;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
+  if (nbr) {  // eight trials can start in a window, six otherwise
+    path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
+    path |= ((path & like) << n_base) | ((path & rej) << (n_base + 1));
+  }
+  // the positions passed, by n_base words each and one more per rejection
+  const unsigned passed = __popc(path & (like | rej)), n_rej = __popc(path & rej);
+  return ((unsigned)lane + passed * (unsigned)n_base + n_rej) | passed << 8 | n_rej << 16;
+}
+
 // What the team tells the makers at the end.
 struct FieldEnd {
   unsigned long long words;

@@ -170,6 +170,7 @@ void preload_ns_kernels();
 void preload_ns_rounds_kernels();
 void preload_wl_kernels();
 void preload_wl_field_kernels();
+void preload_wl_enter_kernels();
 void preload_lattice_kernels();
 
 // Kernels of the chains that run in shared memory (fcc/bcc).

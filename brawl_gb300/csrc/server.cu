@@ -1238,6 +1238,7 @@ int brawl_serve_create(const brawl_server_opts* opts, brawl_server** out) {
   preload_ns_rounds_kernels();
   preload_wl_kernels();
   preload_wl_field_kernels();
+  preload_wl_enter_kernels();
   preload_lattice_kernels();
   {
     cudaFuncAttributes a;

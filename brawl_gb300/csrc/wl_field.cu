@@ -57,7 +57,7 @@ struct WlShare {
   int verdict;
 };
 
-// field_walk (metropolis_field.cu) for the masks of trials that draw n_base + 1
+// field_walk (field_engine.cuh) for the masks of trials that draw n_base + 1
 // words and n_base words.
 __device__ __forceinline__ unsigned wl_walk(unsigned like, unsigned long_m, unsigned short_m, int lane, int n_base,
                                             bool nbr) {

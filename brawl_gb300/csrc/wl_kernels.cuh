@@ -65,11 +65,17 @@ struct WlEnterJob {
   int64_t steps;         // out: loop iterations, -1 when max_steps ran out
   double energy;         // out: the final full_energy
   int32_t initial;       // draw the starting configuration with initial_setup first
+  int32_t S;             // fixed-point shift of F
+  int32_t field_cap;     // moves the deferred-energy log holds beside the fields (wl_enter.cu)
   int32_t pad;
 };
 
 uint32_t wl_enter_smem_bytes(const Geom& g);
 void launch_wl_enter(WlEnterJob* d_jobs, int n, uint32_t smem, cudaStream_t stream);
+// The same with the sites' fields in shared memory (wl_enter.cu), for walkers with
+// a field_cap, of one field_variant.
+uint32_t wl_enter_field_smem_bytes(const Geom& g, const FieldGeom& f, int cap);
+void launch_wl_enter_field(WlEnterJob* d_jobs, int n, uint32_t smem, int max_z, int variant, cudaStream_t stream);
 
 // Walkers first..first+count-1 share a window and are averaged together.
 struct WlGroup {

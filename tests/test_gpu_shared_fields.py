@@ -94,3 +94,39 @@ def test_wang_landau_at_the_edges_matches_oracle(wl_f, period):
                 assert np.array_equal(wl.config(w), cfgs[w]), (case, trials)
         for w in range(len(walkers)):
             assert np.array_equal(wl.genrand(w, 20), np.array([rngs[w].uniform() for _ in range(20)]))
+
+
+@pytest.mark.parametrize("scale", [1.0, 30.0])
+def test_enter_windows_at_the_edges_matches_oracle(scale):
+    """Walks into windows below, above and around the likely energies, one that
+    is entered at the start and one that is out of reach (the configuration is
+    drawn again every 250 steps a site, until max_steps), sharply biased and
+    not."""
+    for k, case in enumerate(EDGES):
+        lattice, n, ns, nsh, _ = case
+        if nsh == 10:
+            continue  # (shells without every opposite: the energies never agree)
+        V, mod, r, cfg = _chain(case, k)
+        conc = conc_vector(ns)
+        E = np.array([mod.total_energy(mod.initial_setup(O.OracleRng(s), conc)[0]) for s in range(12)])
+        mid, spread = float(E.mean()), max(float(np.ptp(E)), 0.02)
+        edges = mid + spread * np.array([-400.0, -399.0, -1.6, -1.0, -0.5, 0.5, 1.0, 1.6])
+        walkers = [dict(setup=B.Setup(lattice, *n, ns, nsh), V=V, seed=900 + 3 * w, config=cfg.copy(), start_idx=b,
+                        end_idx=b, window=w) for w, b in enumerate((1, 3, 5, 7))]
+        max_steps = 250 * mod.n_atoms * 2 + 77
+        lo_mev, hi_mev = 0.0, scale * spread * 13605.693122 / mod.n_atoms
+        W = B.WangLandauWalkers(walkers, edges)
+        try:
+            W.enter_windows(lo_mev, hi_mev, conc, None, initial=True, max_steps=max_steps)
+            assert False, "a window is out of reach"
+        except B.BrawlError:
+            pass
+        f32 = np.float32
+        x = float((f32(0.0025) * abs(f32(hi_mev) - f32(lo_mev))) * f32(mod.n_atoms)) / (13.605693122 * 1000.0)
+        for w, d in enumerate(walkers):
+            s = O.OracleRng(d["seed"])
+            c, _ = mod.initial_setup(s, conc)
+            mod.wl_enter_window(c, s, conc, None, edges[d["start_idx"] - 1], edges[d["end_idx"]], 2.0 * (x * x),
+                                max_steps)
+            assert np.array_equal(W.config(w), c), (case, w)
+            assert np.array_equal(W.genrand(w, 10), np.array([s.uniform() for _ in range(10)])), (case, w)
