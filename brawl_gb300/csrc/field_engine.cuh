@@ -250,8 +250,8 @@ __device__ __forceinline__ void field_sites(const unsigned char* smem, const Fie
   for (int j = 0; j < NJ; ++j) at[j] = tab(P.ex[j] + x) + tab(P.ey[j] + y) + tab(P.ez[j] + z);
 }
 
-// This thread's share of the fields' update for a swap: its site's coordinates
-// and U's row of that site's change (byte address).  Plain loads, adds and
+// This thread's share of the fields' update for a swap: the plan's sites around
+// its site (field_sites) and U's row of that site's change (byte address).  Plain loads, adds and
 // stores: an entry's sites are distinct for one swapped site, and where a site
 // may be around both, the halves go one after the other.  On lattices so small
 // that several entries of a site lead to one other (distinct = 0) the adds are
@@ -259,14 +259,14 @@ __device__ __forceinline__ void field_sites(const unsigned char* smem, const Fie
 // team meets once more before the fields are read.
 template <int NJ, int R>
 __device__ __forceinline__ void field_update(const FieldLayout& L, unsigned char* smem, const FieldPlan<NJ>& P,
-                                             int distinct, int r, int xyz, int row, bool both, bool second) {
+                                             int distinct, int r, const int (&sites)[NJ], int row, bool both,
+                                             bool second) {
   using F = FieldVec<R == 0 ? 1 : R>;
   using T = typename F::T;
   const int rs = R == 0 ? r : R;
   int at[NJ];
-  field_sites<NJ>(smem, P, xyz, at);
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) at[j] = (int)L.g + 4 * rs * at[j];
+  for (int j = 0; j < NJ; ++j) at[j] = (int)L.g + 4 * rs * sites[j];
   if (!distinct) {
     for (int p = 0; p < rs; ++p)
 #pragma unroll

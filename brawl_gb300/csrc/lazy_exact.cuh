@@ -261,6 +261,7 @@ __device__ __forceinline__ void lazy_sites(const Geom& g, const double* V, const
   for (int c0 = 0; c0 < nch; c0 += nthreads * ILP) {
     const uint8_t* row[ILP];  // the chain's neighbour codes
     int cs[ILP], met[ILP];    // its centre's species; what it finds at the other site
+    int keep[ILP];            // the codes' bits it looks at
     bool on[ILP];
     double site[ILP];
 #pragma unroll
@@ -274,7 +275,8 @@ __device__ __forceinline__ void lazy_sites(const Geom& g, const double* V, const
       cs[i] = after ? then : before;
       // after the move the partner holds our old species, a site that is its
       // own neighbour its new one; before it the codes' own
-      met[i] = after ? (before | then << 8) : 0;
+      met[i] = before | then << 8;
+      keep[i] = after ? 0xff : 0x3f;
       row[i] = L.codes + m * 2 * z + (site2 ? z : 0);
       site[i] = 0.0;
     }
@@ -288,10 +290,10 @@ __device__ __forceinline__ void lazy_sites(const Geom& g, const double* V, const
         sum[i] = 0.0;
       }
       auto term = [&](int i, int code) {
-        int s = code & 0x3f;
-        if (code & (kLazyPartner | kLazySelf))
-          if (met[i]) s = (code & kLazyPartner) ? (met[i] & 0xff) : (met[i] >> 8);
-        return on[i] ? Vr[i][ns * s] : 0.0;
+        int s = code & keep[i];
+        s = s & kLazyPartner ? met[i] & 0xff : s;
+        s = s & kLazySelf ? met[i] >> 8 : s;
+        return Vr[i][ns * s];
       };
       int k = 0;
       // the terms of kAhead neighbours of every chain are loaded before their
@@ -360,7 +362,63 @@ static __device__ __noinline__ void lazy_sites_any(const Geom& g, const double* 
 
 // The walker's energy e folded with the n moves' pair energies (one warp;
 // every lane returns the same value).
+//
+// One by one the adds are a chain of 64 cycles each.  While the energy and what
+// it passes through stay in one binade they are multiples of that binade's ulp,
+// and an add rounds its term to such a multiple, the same whatever the energy,
+// unless the term lies halfway between two: so the terms are rounded by
+// themselves (to whole ulps, the difference of the doubles' bits), added up as
+// integers in parallel, and every value passed through is checked to lie inside
+// the binade (lane l: moves 2 l and 2 l + 1).  Where one does not, one by one.  A
+// log of 64 moves is 128 dependent adds of 64 cycles one by one (Wang-Landau), and
+// twelve in parallel.
 static __device__ __noinline__ double lazy_fold(LazyLog L, int n, double e, int fold) {
+  const int lane = threadIdx.x & 31;
+  const long long eb = __double_as_longlong(e);
+  const int hi = (int)(eb >> 32) & 0xfff00000, ex = hi & 0x7ff00000;
+  if (n > 2 && n <= 64 && ex > (60 << 20) && ex < 0x7ff00000) {
+    // half an ulp of e, compared by the bits
+    const long long half = (long long)(ex - (53 << 20)) << 32;
+    bool ok = true;
+    // (not the binade's first value: a sum just under it rounds more finely)
+    auto inside = [&](long long b) {
+      ok = ok && ((int)(b >> 32) & 0xfff00000) == hi && (b & 0xfffffffffffffll) != 0;
+    };
+    auto ulps = [&](double t) {
+      const double x = __dadd_rn(e, t), off = __dsub_rn(t, __dsub_rn(x, e));
+      const long long b = __double_as_longlong(x);
+      inside(b);
+      ok = ok && (__double_as_longlong(off) & 0x7fffffffffffffffll) < half;
+      return b - eb;
+    };
+    long long r[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int m = 2 * lane + k;
+      if (m < n) {
+        if (fold == kFoldWangLandau) {
+          r[k][0] = ulps(-L.pair[2 * m]);
+          r[k][1] = ulps(L.pair[2 * m + 1]);
+        } else {
+          r[k][0] = ulps(L.part[m]);
+        }
+      }
+    }
+    const long long first = r[0][0] + r[0][1], both = first + r[1][0] + r[1][1];
+    long long sum = both;  // with the lanes before
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long v = __shfl_up_sync(kFull, sum, o);
+      sum += lane >= o ? v : 0ll;
+    }
+    const long long x0 = eb + sum - both;
+    if (lane > 0) inside(x0);
+    inside(x0 + r[0][0]);
+    inside(x0 + first);
+    inside(x0 + first + r[1][0]);
+    inside(x0 + both);
+    if (__all_sync(kFull, ok)) return __longlong_as_double(eb + __shfl_sync(kFull, sum, 31));
+  }
   if (fold == kFoldWangLandau) {
     // e = (e - pair_before) + pair_after, two dependent adds per move
     for (int m = 0; m < n; ++m) e = __dadd_rn(__dsub_rn(e, L.pair[2 * m]), L.pair[2 * m + 1]);

@@ -176,7 +176,9 @@ __global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob
         }
         // U's rows by (old - 1) ns + new - 1
         const int row = (int)L.U + ((second ? s2 * ns + s1 : s1 * ns + s2) >> 2) * per;
-        field_update<NJ, R>(L, smem, P, distinct, r, second ? q.y : q.x, row, q.w != 0, second);
+        int sites[NJ];
+        field_sites<NJ>(smem, P, second ? q.y : q.x, sites);
+        field_update<NJ, R>(L, smem, P, distinct, r, sites, row, q.w != 0, second);
       }
       pass_windows(e + (o >= kWin));
       o &= kWin - 1;

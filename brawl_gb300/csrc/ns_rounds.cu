@@ -105,37 +105,6 @@ __device__ __forceinline__ void sums_end_arrive() { asm volatile("bar.arrive 8, 
 __device__ __forceinline__ void sums_end_wait() { asm volatile("bar.sync 8, 384;" ::: "memory"); }
 __device__ __forceinline__ void sums_sync() { asm volatile("bar.sync 9, 128;" ::: "memory"); }
 
-// lazy_fold's nested sum (one add per step, each rounded) by a warp.  While the
-// sum stays in one binade it is a multiple of that binade's ulp and every add
-// rounds its term to such a multiple, the same whatever the sum, unless the
-// term lies halfway between two: then the rounded terms add up exactly in any
-// order.  Otherwise one by one.
-__device__ double nested_fold(const LazyLog& L, int n, double e, int lane) {
-  double sum = 0.0, most = 0.0;
-  const int ex = __double2hiint(e) & 0x7ff00000;
-  bool ok = ex > (60 << 20) && ex < 0x7ff00000;
-  // half an ulp of e, compared by the bits
-  const long long half = (long long)(ex - (53 << 20)) << 32;
-  for (int m = lane; m < n; m += 32) {
-    const double d = L.part[m];
-    const double r = __dsub_rn(__dadd_rn(e, d), e), off = __dsub_rn(d, r);
-    ok = ok && (__double_as_longlong(off) & 0x7fffffffffffffffll) < half;
-    sum = __dadd_rn(sum, r);
-    most = __dadd_rn(most, fabs(r));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    sum = __dadd_rn(sum, __shfl_xor_sync(kFull, sum, o));
-    most = __dadd_ru(most, __shfl_xor_sync(kFull, most, o));
-  }
-  // no partial sum (nor the first of a term's two roundings) leaves the binade
-  const int up = __double2hiint(__dadd_ru(e, most)), dn = __double2hiint(__dsub_rd(e, most));
-  ok = ok && (up & 0xfff00000) == (__double2hiint(e) & 0xfff00000) && (dn & 0xfff00000) == (up & 0xfff00000);
-  if (__all_sync(kFull, ok)) return __dadd_rn(e, sum);
-  for (int m = 0; m < n; ++m) e = __dadd_rn(e, L.part[m]);
-  return e;
-}
-
 // This lane's neighbour entries (lanes 0 to 15: site 1's, 16 to 31: site 2's),
 // every 16th: the axis tables' byte
 // addresses of the entry's offset, and its shell's of F's rows.
@@ -182,7 +151,7 @@ __device__ __noinline__ void ns_sums(const Geom& g, unsigned char* smem, const N
     lazy_sites_any<2>(g, V, sstart, LG, n, kFoldNested, 32 * mine + lane, 128);
     sums_sync();
     const double E0 = vs->E, limit = vs->limit;
-    const double E = nested_fold(LG, n, E0, lane);  // (each of the four)
+    const double E = lazy_fold(LG, n, E0, kFoldNested);  // (each of the four)
     if (mine == 0) {
       const double q = ldexp(1.0, -St);
       const int ok = in_quanta(E, E0, vs->Dlo, vs->Dhi, q);

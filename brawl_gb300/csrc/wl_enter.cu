@@ -324,6 +324,8 @@ __global__ void __launch_bounds__(256, 1) wl_enter_field_kernel(WlEnterJob* __re
         }
         const int next_o = p + n_base + 1;
         if (verdict > 0) {
+          int at_n[NJ];
+          field_sites<NJ>(smem, P, second ? q.y : q.x, at_n);
           if (exact) {
             e_ex = e_sw;  // the log is empty here
             rebase();
@@ -332,8 +334,6 @@ __global__ void __launch_bounds__(256, 1) wl_enter_field_kernel(WlEnterJob* __re
             // other site marked
             uint8_t* rec = LG.codes + (size_t)n_log * 2 * z + (second ? z : 0) + (tt & (kFieldHalf - 1));
             const int other = second ? a.x : a.y, s_other = second ? s1 : s2;
-            int at_n[NJ];
-            field_sites<NJ>(smem, P, second ? q.y : q.x, at_n);
 #pragma unroll
             for (int j = 0; j < NJ; ++j)
               if ((P.valid >> j) & 1) {
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256, 1) wl_enter_field_kernel(WlEnterJob* __re
             smem[L.lat + a.y] = (unsigned char)s1;
           }
           const int row = (int)L.U + ((second ? s2 * ns + s1 : s1 * ns + s2) >> 2) * per;
-          field_update<NJ, R>(L, smem, P, distinct, r, second ? q.y : q.x, row, q.w != 0, second);
+          field_update<NJ, R>(L, smem, P, distinct, r, at_n, row, q.w != 0, second);
         }
         team_sync();
         if (verdict > 0) {

@@ -107,7 +107,7 @@ __device__ __forceinline__ double add_times(double v, double f, int k) {
     // half an ulp of v (v a normal number well above the smallest), compared by
     // the bits
     const long long half = (long long)((ev & 0x7ff00000) - (53 << 20)) << 32;
-    if (ev == ee && (ev & 0x7ff00000) > (60 << 20) && (ev & 0x7ff00000) < 0x7ff00000 &&
+    if (__double2hiint(f) >= 0 && ev >= 0 && ev == ee && (ev & 0x7ff00000) > (60 << 20) && (ev & 0x7ff00000) < 0x7ff00000 &&
         (__double_as_longlong(off) & 0x7fffffffffffffffll) < half)
       return end;
   }
@@ -122,13 +122,13 @@ __device__ __forceinline__ double add_times(double v, double f, int k) {
 // time, in order (each add rounds), beside the other warps' next decisions.
 //
 // A walker's trials depend on one another, so its own chain of decisions bounds
-// it: a pair of windows takes 730 cycles to decide and walk and an accepted move
-// 1,000 more (its log entry, the fields' update and the books), against some
+// it: a pair of windows takes some 700 cycles to decide and walk and an accepted
+// move 800 more (its log entry, the fields' update), against some
 // 2,900 a trial in wl_sweep_kernel, which gathers both sites' neighbours for
 // each.  FP64 is kept out of the decisions (a dependent FP64 add takes a warp 64
 // cycles): bins from a float interval, tests from ln g's fixed-point copy.
 // Measured on 128 walkers of bcc 12^3, four species, four shells, 10^4 trials: a
-// call takes 11 to 12 ms with wl_sweep_kernel and 3.1 to 5.4 ms here (walkers
+// call takes 11 to 12 ms with wl_sweep_kernel and 2.7 to 4.7 ms here (walkers
 // that accept 38% to 55% of their trials).  16 warps a block would leave each too
 // few registers (spills), hence 8.
 template <int NJ, int R>
@@ -227,8 +227,7 @@ __global__ void __launch_bounds__(256, 1) wl_field_kernel(WlWalker* __restrict__
     // 1.8e-7 |p| and |wide| (the floats' products), 6e-8 of the sums; m is at
     // least that.  int() truncates: below zero, where t < 0, it is one up.
     auto bin_of = [&](int dE, int& b) {
-      const float p = small ? __fmul_rn(__int2float_rn(lo32 + dE), qrf)
-                            : __fmul_rn(__ll2float_rn(base_lo + dE), qrf);
+      const float p = __fmul_rn(__int2float_rn(lo32 + dE), qrf);
       const float t = __fadd_rn(t0_frac, p);
       const float m = __fmaf_rn(3.0e-7f, fabsf(p) + wide, 8.0e-7f);
       const float lo = floorf(__fsub_rd(t, m)), hi = floorf(__fadd_ru(t, wide + 2.0f * m));
@@ -447,9 +446,9 @@ __global__ void __launch_bounds__(256, 1) wl_field_kernel(WlWalker* __restrict__
       const long long l_from = li;
       li = plus(accept && jbin != ibin ? lq[jbin - start] : li, 1);
       if (accept) ibin = jbin;
-      // the books of the bin it was in, beside the update
-      if (who == 2) book(from, ibin == from ? k + 1 : k, h);
       if (accept && differ) {
+        int at_n[NJ];
+        field_sites<NJ>(smem, P, second ? q.y : q.x, at_n);
         if (exact_done) {
           e_ex = e_sw;  // the log is empty here
           rebase();
@@ -458,8 +457,6 @@ __global__ void __launch_bounds__(256, 1) wl_field_kernel(WlWalker* __restrict__
           // other site marked
           uint8_t* rec = LG.codes + (size_t)n_log * 2 * z + (second ? z : 0) + (tt & (kFieldHalf - 1));
           const int other = second ? a.x : a.y, s_other = second ? s1 : s2;
-          int at_n[NJ];
-          field_sites<NJ>(smem, P, second ? q.y : q.x, at_n);
 #pragma unroll
           for (int j = 0; j < NJ; ++j)
             if ((P.valid >> j) & 1) {
@@ -482,14 +479,23 @@ __global__ void __launch_bounds__(256, 1) wl_field_kernel(WlWalker* __restrict__
           smem[L.lat + a.y] = (unsigned char)s1;
         }
         const int row = (int)L.U + ((second ? s2 * ns + s1 : s1 * ns + s2) >> 2) * per;
-        field_update<NJ, R>(L, smem, P, distinct, r, second ? q.y : q.x, row, q.w != 0, second);
+        field_update<NJ, R>(L, smem, P, distinct, r, at_n, row, q.w != 0, second);
       }
       if (tt == kFieldHalf && ibin != from) lq[from - start] = l_from;
       team_sync();
       int h1 = 0;
       if (who == 2 || stored) h1 = ticks(1);
       if (stored && h1 > 0) store(ibin);
-      if (who == 2) book(ibin, ibin == from ? 0 : 1, h1);
+      // the books of the bin it was in and of the one it is in, beside the next
+      // decisions
+      if (who == 2) {
+        if (ibin != from) {
+          book(from, k, h);
+          book(ibin, 1, h1);
+        } else {
+          book(ibin, k + 1, h + h1);
+        }
+      }
       if (n_log == LG.cap) flush();
       pass_windows(e + (next_o >= kWin));
       o = next_o & (kWin - 1);
