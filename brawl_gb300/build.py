@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libbrawl_gpu.so")
-SOURCES = ["metropolis.cu", "metropolis_halo.cu", "metropolis_field.cu", "lattice_ops.cu", "asro.cu", "capi.cu", "noalloc.cu", "nested_sampling.cu", "ns_rounds.cu", "wang_landau.cu", "wl_field.cu", "wl_enter.cu", "server.cu",
+SOURCES = ["metropolis.cu", "metropolis_halo.cu", "metropolis_field.cu", "metropolis_rounds.cu", "lattice_ops.cu", "asro.cu", "capi.cu", "noalloc.cu", "nested_sampling.cu", "ns_rounds.cu", "wang_landau.cu", "wl_field.cu", "wl_enter.cu", "server.cu",
            "peaks.cu", "sampling.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",

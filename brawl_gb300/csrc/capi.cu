@@ -187,6 +187,14 @@ void make_halo(const Geom& g, HaloGeom& H, bool& ok) {
        dmz <= g.n3 && smem_layout(g, false).use_D;
 }
 
+// Whether an entry leads from a site to itself.
+bool meets_itself(const Geom& g) {
+  const int8_t(*offs)[3] = shell_offsets(g.lattice);
+  for (int k = 0; k < g.z; ++k)
+    if (offs[k][0] % g.W1 == 0 && offs[k][1] % g.W2 == 0 && offs[k][2] % g.W3 == 0) return true;
+  return false;
+}
+
 // Displacement classes (FieldGeom) of an fcc/bcc lattice: usable when no entry
 // leads back to its own site and no further than the opposite one (offsets
 // within n per axis), and the packed coordinates and indices fit.
@@ -450,6 +458,10 @@ struct brawl_batch {
   size_t scratch_cap = 0;
   cudaStream_t stream = nullptr;
   uint32_t smem_bytes = 0;
+  // the chains without a shared-memory kernel: in rounds of trials
+  // (metropolis_rounds.cu), their lattices as half bytes, its shared memory
+  bool rest_rounds = false, rest_nibbles = false;
+  uint32_t rest_smem = 0;
   bool smem_lat = true;
   bool use_D = true;
   int max_z = 0;
@@ -716,11 +728,18 @@ int run_metropolis(brawl_batch* b, const int64_t* n_trials, int64_t* accepted, b
 
 // Every chain's uploaded job (b->d_jobs) once on `stream`: the shared-memory
 // chains' launches, the others in one launch of the plain kernel.
+// Chains first .. first + n - 1 of the launch order, which no shared-memory group
+// takes.
+void launch_rest(brawl_batch* b, int first, int n, cudaStream_t stream) {
+  if (b->rest_rounds)
+    launch_metropolis_rounds(b->d_jobs + first, n, b->rest_nibbles, b->rest_smem, b->max_z, stream);
+  else
+    launch_metropolis(b->d_jobs + first, n, b->smem_lat, b->use_D, b->smem_bytes, b->max_z, stream);
+}
+
 int launch_sweep(brawl_batch* b, cudaStream_t stream) {
   const int n = (int)b->jobs.size();
-  if (n > b->n_shared)
-    launch_metropolis(b->d_jobs + b->n_shared, n - b->n_shared, b->smem_lat, b->use_D, b->smem_bytes, b->max_z,
-                      stream);
+  if (n > b->n_shared) launch_rest(b, b->n_shared, n - b->n_shared, stream);
   CUDA_TRY(cudaGetLastError());
   return launch_groups(b, stream);
 }
@@ -751,7 +770,7 @@ int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accept
         CUDA_TRY(stream_wait(stream));
       }
     for (int k = b->n_shared; k < n; ++k) {
-      launch_metropolis(b->d_jobs + k, 1, b->smem_lat, b->use_D, b->smem_bytes, b->max_z, stream);
+      launch_rest(b, k, 1, stream);
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(stream_wait(stream));
     }
@@ -802,6 +821,9 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
   b->max_optin = max_optin;
   uint32_t need_smem = 0, need_gmem = 0;
+  int n_rest = 0;  // chains the shared-memory kernels do not take
+  bool rest_fits = true;
+  uint32_t rest_bytes = 0, rest_nibbles = 0;
   b->kernel.assign(n_chains, kSharedNone);
   b->halo.assign(n_chains, 0);
   b->gather_smem.assign(n_chains, 0);
@@ -852,6 +874,10 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     }
     b->cls[c] = kind_class[k];
     if (b->kernel[c] != kSharedNone) continue;
+    n_rest += 1;
+    rest_fits = rest_fits && m.g.n1 <= 512 && m.g.n2 <= 512 && m.g.n3 <= 512 && !meets_itself(m.g);
+    rest_bytes = std::max(rest_bytes, round_smem_bytes(m.g, false));
+    rest_nibbles = std::max(rest_nibbles, round_smem_bytes(m.g, true));
     need_smem = std::max(need_smem, smem_layout(m.g, true).total);
     need_gmem = std::max(need_gmem, smem_layout(m.g, false).total);
     b->max_z = std::max(b->max_z, (int)m.g.z);
@@ -867,6 +893,9 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     if (!fields_pay(load, n_sm))
       for (int c = 0; c < n_chains; ++c)
         if (b->halo[c]) b->kernel[c] = kSharedGather;
+    b->rest_nibbles = rest_bytes > (uint32_t)max_optin;
+    b->rest_smem = b->rest_nibbles ? rest_nibbles : rest_bytes;
+    b->rest_rounds = n_rest > 0 && rest_fits && b->rest_smem <= (uint32_t)max_optin && rounds_pay(n_rest, n_sm);
   }
   b->smem_lat = need_smem <= (uint32_t)max_optin;
   b->smem_bytes = b->smem_lat ? need_smem : need_gmem;
@@ -2039,9 +2068,7 @@ struct brawl_ns {
 static bool ns_plan_rounds(const Geom& g, NsRun& R, uint32_t limit) {
   R.rounds_cap = 0;
   if (g.n_sites > 65535 || g.n1 > 512 || g.n2 > 512 || g.n3 > 512) return false;
-  const int8_t(*offs)[3] = shell_offsets(g.lattice);
-  for (int k = 0; k < g.z; ++k)
-    if (offs[k][0] % g.W1 == 0 && offs[k][1] % g.W2 == 0 && offs[k][2] % g.W3 == 0) return false;
+  if (meets_itself(g)) return false;
   for (R.rounds_cap = kLazyMaxCap; R.rounds_cap >= 16; R.rounds_cap >>= 1)
     if (ns_rounds_smem_bytes(g, R.rounds_cap) <= limit) return true;
   return false;

@@ -192,6 +192,16 @@ enum shared_kernel : int {
 inline double field_load(uint32_t smem) { return 2u * (smem + 1024u) <= 228u * 1024u ? 0.5 : 1.0; }
 inline bool fields_pay(double load, int n_sm) { return load <= 2.0 * n_sm; }
 
+// Chains in rounds of trials (metropolis_rounds.cu) where each has an SM to itself
+// (its sixteen warps' registers fill one): 152 chains take as long as one, 0.74 ms
+// (simple cubic 6^3, 4,000 trials) and 1.0 (8^3, two species), and twice as many
+// twice that, where metropolis_kernel, a warp a chain, takes 2.7 and 1.75 for
+// either.
+inline bool rounds_pay(int n_chains, int n_sm) { return n_chains <= n_sm; }
+uint32_t round_smem_bytes(const Geom& g, bool nibbles);
+void launch_metropolis_rounds(const ChainJob* d_jobs, int n_jobs, bool nibbles, uint32_t smem_bytes, int max_z,
+                              cudaStream_t stream);
+
 // One launch of them: `count` chains from `first` in launch order, the largest
 // shared memory and neighbour count among them, and the trials per
 // round of the gather kernel (1: kGatherDefault).

@@ -130,3 +130,32 @@ def test_enter_windows_at_the_edges_matches_oracle(scale):
                                 max_steps)
             assert np.array_equal(W.config(w), c), (case, w)
             assert np.array_equal(W.genrand(w, 10), np.array([s.uniform() for _ in range(10)])), (case, w)
+
+
+@pytest.mark.parametrize("case", [
+    ("simple_cubic", (2, 3, 4), 3, 2, False, 900),
+    ("simple_cubic", (6, 5, 7), 15, 2, True, 6000),
+    ("simple_cubic", (16, 3, 3), 2, 1, False, 5001),
+    ("fcc", (512, 3, 40), 3, 2, False, 4000),        # half bytes; the largest coordinates
+    ("bcc", (47, 47, 51), 4, 3, True, 4000),         # half bytes, a remainder of two sites
+    ("fcc", (38, 38, 38), 15, 6, False, 3000),
+    ("bcc", (48, 48, 50), 2, 10, False, 3000),
+], ids=lambda c: f"{c[0]}-{c[1]}-s{c[2]}-sh{c[3]}")
+def test_rounds_of_trials_match_oracle(case):
+    """Chains in rounds of trials (simple cubic, and lattices of more than 2^16
+    sites), hot and cold, in calls of none, one and many trials."""
+    lattice, n, ns, nsh, nbr, trials = case
+    V, mod, r, start = _chain(case[:5], ns + nsh)
+    setup = B.Setup(lattice, *n, ns, nsh)
+    b = B.Batch([dict(setup=setup, V=V, seed=7000 + ns + nsh, beta=1.0 / (T * B.K_B_IN_RY), nbr_swap=nbr,
+                      species_concentrations=conc_vector(ns)) for T in (200.0, 4000.0)])
+    cfgs, rngs = [start.copy(), start.copy()], [O.OracleRng(1), O.OracleRng(1)]
+    for g in rngs:
+        g.set_state_words(r.state_words())
+    for k in (0, 1, 3, trials):
+        acc = b.metropolis(k)
+        for c, T in enumerate((200.0, 4000.0)):
+            a, _ = mod.mc_run(cfgs[c], rngs[c], 1.0 / (T * B.K_B_IN_RY), k, nbr)
+            assert acc[c] == a, (T, k)
+            assert np.array_equal(b.config(c), cfgs[c]), (T, k)
+            assert _same_stream(b.rng_state(c), rngs[c]), (T, k)
