@@ -21,24 +21,24 @@ int make_asro_plan(const Geom& g, int wc_range, const double* shells, AsroPlan& 
   plan.class_mask.clear();
   const int W[3] = {2 * g.n1, 2 * g.n2, 2 * g.n3};
   const int m[3] = {std::min(g.n1, 5), std::min(g.n2, 5), std::min(g.n3, 5)};
+  // per axis and step, the square of the minimum image exactly as the reference
+  // forms it, for site 0: d = real(i - j); d = d - float(2n) * nint(d / float(2n))
+  double square[3][11];
+  for (int a = 0; a < 3; ++a)
+    for (int d = -m[a]; d <= m[a]; ++d) {
+      const int j = ((0 + d) % W[a] + W[a]) % W[a];
+      double v = (double)(float)(0 - j);
+      const float wf = (float)W[a];
+      v = v - (double)(wf * (float)nint_d(v / (double)wf));
+      square[a][d + 5] = v * v;
+    }
   std::map<uint64_t, int> classes;
   for (int dz = -m[2]; dz <= m[2]; ++dz)
     for (int dy = -m[1]; dy <= m[1]; ++dy)
       for (int dx = -m[0]; dx <= m[0]; ++dx) {
-        const int d[3] = {dx, dy, dz};
         if (g.lattice == kBcc && !((((dx - dz) & 1) == 0) && (((dy - dz) & 1) == 0))) continue;
         if (g.lattice == kFcc && ((dx + dy + dz) & 1)) continue;
-        // minimum image exactly as the reference forms it, for site 0:
-        // d = real(i - j); d = d - float(2n) * nint(d / float(2n))
-        double comp[3];
-        for (int a = 0; a < 3; ++a) {
-          int j = ((0 + d[a]) % W[a] + W[a]) % W[a];
-          double v = (double)(float)(0 - j);
-          const float wf = (float)W[a];
-          v = v - (double)(wf * (float)nint_d(v / (double)wf));
-          comp[a] = v;
-        }
-        const double dist = std::sqrt(comp[0] * comp[0] + comp[1] * comp[1] + comp[2] * comp[2]);
+        const double dist = std::sqrt(square[0][dx + 5] + square[1][dy + 5] + square[2][dz + 5]);
         uint64_t mask = 0;
         for (int l = 0; l < wc_range; ++l)
           if (std::fabs(dist - shells[l]) < 1e-3) mask |= 1ull << l;

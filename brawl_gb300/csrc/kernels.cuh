@@ -256,21 +256,114 @@ __device__ inline double site_energy_ref(const Geom& g, const int8_t* lat, const
   return total;
 }
 
+// The doubles of one binade are consecutive in their bits, and a sum that stays in
+// the binade rounds its term to a whole number of the binade's ulps, the same
+// whatever the sum, unless the term lies halfway between two.  That number for
+// term t (bits) and the binade of e (bits; a normal number), in the direction in
+// which e's bits grow; ok: not halfway, and not past what 63 bits hold.
+__host__ __device__ __forceinline__ long long ulps_of(long long t, long long e, bool& ok) {
+  const int et = (int)(t >> 52) & 0x7ff, s = ((int)(e >> 52) & 0x7ff) - (et > 0 ? et : 1);
+  const long long m = (t & 0xfffffffffffffll) | (et > 0 ? 1ll << 52 : 0ll);
+  long long k;
+  if (s <= 0) {
+    ok = ok && s >= -8;
+    k = m << (-s & 15);
+  } else {
+    const int r = s < 55 ? s : 55;  // (from 55 on it is under half an ulp)
+    const long long half = 1ll << (r - 1);
+    ok = ok && (m & (2 * half - 1)) != half;
+    k = (m + half) >> r;
+  }
+  return (t ^ e) < 0 ? -k : k;
+}
+
+// A value passed through: inside the binade of e, and not its first value (a sum
+// just under that one rounds more finely).
+__host__ __device__ __forceinline__ bool inside_binade(long long b, long long e) {
+  return ((b ^ e) >> 52) == 0 && (b & 0xfffffffffffffll) != 0;
+}
+
 // total_energy's ordered sum (src/bw_hamiltonian.f90:67-79): energy =
 // energy + e(site) over the sites in order, then 0.5 * energy, for one warp.
-// The warp loads 32 site energies at a time (the next 32 already in flight)
-// and every lane runs the same ordered chain of adds on them through
-// shuffles, so the chain waits on the adds, not on the loads.  Every lane
-// returns the result.
+// Every lane returns the result.
+//
+// One by one that is a chain of FP64 adds, 64 cycles each.  256 terms at a time
+// (eight a lane) are rounded to whole ulps of the sum so far, added as integers,
+// and every value passed through is checked to lie in its binade; the terms up to
+// the first that leaves it (or lies halfway between two ulps) are done, and that
+// one is added by itself.  A sum that keeps leaving its binade (one that stays
+// near zero) is added up one by one for a while, longer each time.  256 chains
+// of up to 27,648 sites: 1.12 ms one by one, 0.19 ms so.
 __device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int n, int lane) {
+  constexpr int kTerms = 8;
   double energy = 0.0;
-  double v = lane < n ? e[lane] : 0.0;
-  for (int base = 0; base < n; base += 32) {
-    const int nxt = base + 32 + lane;
-    const double v_next = nxt < n ? e[nxt] : 0.0;
-    const int m = min(32, n - base);
-    for (int k = 0; k < m; ++k) energy = __dadd_rn(energy, __shfl_sync(kFull, v, k));
-    v = v_next;
+  int base = 0, slow = n < 128 ? n : 32, run = 32;  // terms to add one by one; then how many
+  while (base < n) {
+    if (slow > 0) {
+      // 32 at a time, the next 32 already in flight
+      double v = base + lane < n ? e[base + lane] : 0.0;
+      for (; slow > 0 && base < n; slow -= 32) {
+        const int m = min(32, n - base), next = base + 32 + lane;
+        const double v_next = next < n ? e[next] : 0.0;
+        for (int k = 0; k < m; ++k) energy = __dadd_rn(energy, __shfl_sync(kFull, v, k));
+        v = v_next;
+        base += m;
+      }
+      continue;
+    }
+    const int first = base + kTerms * lane;
+    double v[kTerms];
+#pragma unroll
+    for (int j = 0; j < kTerms; ++j) v[j] = first + j < n ? e[first + j] : 0.0;
+    const long long eb = __double_as_longlong(energy);
+    const int ex = (int)(eb >> 52) & 0x7ff;
+    long long k[kTerms], sum = 0;
+    unsigned bad = ex > 60 && ex < 0x7ff ? 0u : 1u;  // bit j: term j is not settled
+#pragma unroll
+    for (int j = 0; j < kTerms; ++j) {
+      bool ok = true;
+      k[j] = ulps_of(__double_as_longlong(v[j]), eb, ok);
+      sum += k[j];
+      bad |= ok ? 0u : 1u << j;
+    }
+    long long upto = sum;  // with the lanes before
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(kFull, upto, o);
+      upto += lane >= o ? u : 0ll;
+    }
+    long long x = eb + upto - sum;
+    const long long x0 = x;
+#pragma unroll
+    for (int j = 0; j < kTerms; ++j) {
+      x += k[j];
+      bad |= inside_binade(x, eb) ? 0u : 1u << j;
+    }
+    // the first term that is not settled
+    const unsigned lanes = __ballot_sync(kFull, bad != 0);
+    const int m = min(kTerms * 32, n - base);
+    int at = m;
+    if (lanes) {
+      const int l = __ffs(lanes) - 1;
+      const int j = __ffs(__shfl_sync(kFull, bad, l)) - 1;
+      at = min(m, kTerms * l + j);
+      // the sum before it, and it
+      long long before = x0;
+#pragma unroll
+      for (int i = 0; i < kTerms; ++i) before += i < j ? k[i] : 0ll;
+      energy = __longlong_as_double(__shfl_sync(kFull, before, l));
+      if (at < m) {
+        energy = __dadd_rn(energy, e[base + at]);
+        base += at + 1;
+        slow = at < 16 ? run : 0;
+        run = at < 16 ? min(2 * run, 1024) : 32;
+        continue;
+      }
+    } else {
+      energy = __longlong_as_double(__shfl_sync(kFull, x, 31));
+    }
+    base += m;
+    run = 32;
   }
   return __dmul_rn(0.5, energy);
 }
@@ -289,7 +382,7 @@ void launch_initial_setup(const InitJob* d_jobs, int n_jobs, cudaStream_t stream
 
 // The site-by-site draw loop of initial_setup for one configuration
 // (src/initialise.F90:434-617), on the warp's stream (mt in shared memory at
-// position pos); check is shared scratch of kMaxSpecies counters.  Every
+// position pos).  Every
 // word of the stream is one draw: species l + 1 when it falls in the
 // interval of species l whose count is below its quota (the last such l,
 // as the reference's loop over l leaves it), else no species and the site
@@ -302,89 +395,85 @@ void launch_initial_setup(const InitJob* d_jobs, int n_jobs, cudaStream_t stream
 // the next sites in order (a ballot and a prefix count).  A batch where a
 // quota fills, or a word sits on two intervals, is decided word by word.
 // Returns false when a quota can never be met (guards against a corrupted
-// job; the host validates counts).
+// job; the host validates counts).  Lane l keeps species l + 1's interval (as
+// 32-bit words; empty: from above to), quota and count: read from memory and
+// counted in shared memory for every batch they took 1,600 cycles of it, now 980
+// (256 chains of up to 27,648 sites: 0.72 -> 0.44 ms).
 __device__ inline bool initial_setup_warp(const InitJob& J, int8_t* lat, uint32_t* mt, int& pos,
-                                          int64_t* check, unsigned long long& draws, int lane) {
-  if (lane < kMaxSpecies) check[lane] = 0;
-  __syncwarp();
+                                          unsigned long long& draws, int lane) {
   const int ns = J.ns;
   const int n_sites = J.n_sites;
   const unsigned long long limit = draws + (unsigned long long)n_sites * 4096ull + 1000000ull;
   const unsigned lt_mask = (1u << lane) - 1u;
+  uint32_t from = 1u, to = 0u;
+  int64_t quota = 0, check = 0;
+  if (lane < ns) {
+    const int64_t lo = J.lo_w[lane], hi = J.hi_w[lane];
+    if (lo <= 0xffffffffll && hi >= 0) {
+      from = (uint32_t)(lo < 0 ? 0 : lo);
+      to = (uint32_t)(hi > 0xffffffffll ? 0xffffffffll : hi);
+    }
+    quota = J.counts[lane];
+  }
   int site = 0;
   while (site < n_sites) {
     // the next n <= 32 words, none past the end of the current block
     const int avail = kMTN - pos;
     const int n = avail > 0 ? min(32, avail) : 32;
     const uint32_t w = mt_peek(mt, pos, n, lane);
-    const int64_t wl = (int64_t)w;
     int cand = 0, hits = 0;
-    if (lane < n)
-      for (int l = 0; l < ns; ++l)
-        if (wl >= J.lo_w[l] && wl <= J.hi_w[l]) {
-          cand = l + 1;
-          ++hits;
-        }
-    bool fast = !__any_sync(kFull, hits > 1);
+    for (int l = 0; l < ns; ++l) {
+      const uint32_t lo = __shfl_sync(kFull, from, l), hi = __shfl_sync(kFull, to, l);  // (all lanes take part)
+      const bool in = lane < n && w >= lo && w <= hi;
+      cand = in ? l + 1 : cand;
+      hits += in;
+    }
     // a candidate whose quota is already full is a plain rejection; one
     // whose quota fills inside the batch needs the word-by-word pass
-    bool open = false;
-    if (cand > 0) open = check[cand - 1] < J.counts[cand - 1];
+    const unsigned not_full = __ballot_sync(kFull, check < quota) << 1;  // by species
+    const bool open = (not_full >> cand) & 1u;
     unsigned acc = __ballot_sync(kFull, open);
     int need_mine = 0;  // lane l < ns: accepted words of species l + 1 in the batch
     for (int l = 0; l < ns; ++l) {
       const int c = __popc(__ballot_sync(kFull, open && cand == l + 1));
-      if (lane == l) need_mine = c;
+      need_mine = lane == l ? c : need_mine;
     }
-    if (lane < ns && check[lane] + need_mine > J.counts[lane]) fast = false;
-    fast = __all_sync(kFull, fast);
+    const bool fast = __all_sync(kFull, hits <= 1 && !(lane < ns && check + need_mine > quota));
     int consumed = n;
     if (fast) {
       const int r = n_sites - site;
-      if (__popc(acc) >= r) {
+      bool mine = open;
+      if (__popc(acc) > r) {
         // the configuration ends inside the batch: its r-th accepted word
         // is the last one consumed (the words after it are not drawn)
-        unsigned m = acc;
-        for (int k = 1; k < r; ++k) m &= m - 1u;
-        const int last = __ffs(m) - 1;
-        consumed = last + 1;
-        acc &= (last == 31) ? 0xffffffffu : ((1u << (last + 1)) - 1u);
+        mine = open && __popc(acc & lt_mask) < r;
+        acc = __ballot_sync(kFull, mine);
+        for (int l = 0; l < ns; ++l) {
+          const int c = __popc(__ballot_sync(kFull, mine && cand == l + 1));
+          need_mine = lane == l ? c : need_mine;
+        }
       }
-      const bool mine = (acc >> lane) & 1u;
+      if (__popc(acc) == r) consumed = 32 - __clz(acc);
       if (mine) lat[site + __popc(acc & lt_mask)] = (int8_t)cand;
-      int add = 0;
-      for (int l = 0; l < ns; ++l) {
-        const int c = __popc(__ballot_sync(kFull, mine && cand == l + 1));
-        if (lane == l) add = c;
-      }
-      __syncwarp();
-      if (lane < ns) check[lane] += add;
+      check += need_mine;
       site += __popc(acc);
     } else {
       for (int k = 0; k < n; ++k) {
-        const int64_t wk = (int64_t)__shfl_sync(kFull, w, k);
+        const uint32_t wk = __shfl_sync(kFull, w, k);
         // every species whose interval holds the word and whose quota is
         // open takes the site in turn and uses up one of its quota (a word
         // on the boundary of two intervals uses up both); the last one keeps it
-        int s = 0;
-        unsigned taken = 0u;
-        for (int l = 0; l < ns; ++l)
-          if (wk >= J.lo_w[l] && wk <= J.hi_w[l] && check[l] < J.counts[l]) {
-            s = l + 1;
-            taken |= 1u << l;
-          }
-        __syncwarp();
-        if (s > 0) {
-          if (lane < ns && ((taken >> lane) & 1u)) check[lane] += 1;
-          if (lane == 0) lat[site] = (int8_t)s;
+        const bool takes = wk >= from && wk <= to && check < quota;
+        const unsigned taken = __ballot_sync(kFull, takes);
+        if (taken) {
+          check += takes;
+          if (lane == 0) lat[site] = (int8_t)(32 - __clz(taken));
           ++site;
           if (site == n_sites) {
             consumed = k + 1;
-            __syncwarp();
             break;
           }
         }
-        __syncwarp();
       }
     }
     __syncwarp();

@@ -17,14 +17,13 @@ namespace brawl {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(32) initial_setup_kernel(const InitJob* __restrict__ jobs) {
   __shared__ uint32_t mt[kMTN];
-  __shared__ int64_t check[kMaxSpecies];
   const InitJob& J = jobs[blockIdx.x];
   const int lane = threadIdx.x;
   for (int i = lane; i < kMTN; i += 32) mt[i] = J.rng[i];
   int pos = (int)J.rng[kMTN];
   __syncwarp();
   unsigned long long draws = 0;
-  if (!initial_setup_warp(J, J.lat, mt, pos, check, draws, lane)) {
+  if (!initial_setup_warp(J, J.lat, mt, pos, draws, lane)) {
     if (lane == 0) *J.status = kStatusBadSpecies;
     return;
   }

@@ -23,7 +23,6 @@ namespace brawl {
 // draw for the 1e-8 energy jitter (nested_sampling.f90:86-96).
 __global__ void __launch_bounds__(32) ns_init_kernel(NsRun* __restrict__ runs) {
   __shared__ uint32_t mt[kMTN];
-  __shared__ int64_t check[kMaxSpecies];
   NsRun& R = runs[blockIdx.x];
   const int lane = threadIdx.x;
   uint32_t* rng = R.job.rng;
@@ -33,7 +32,7 @@ __global__ void __launch_bounds__(32) ns_init_kernel(NsRun* __restrict__ runs) {
   unsigned long long draws = 0;
   const int n = R.job.g.n_sites;
   for (int w = 0; w < R.K; ++w) {
-    if (!initial_setup_warp(R.init, R.walkers + (size_t)w * n, mt, pos, check, draws, lane)) {
+    if (!initial_setup_warp(R.init, R.walkers + (size_t)w * n, mt, pos, draws, lane)) {
       if (lane == 0) *R.job.status = kStatusBadSpecies;
       return;
     }

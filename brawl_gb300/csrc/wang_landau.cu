@@ -435,7 +435,6 @@ __device__ double full_energy_warp(const Geom& g, const int8_t* lat, const doubl
 // leaves it).  Bounded by max_steps.
 __global__ void __launch_bounds__(32, 1) wl_enter_kernel(WlEnterJob* __restrict__ jobs) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int64_t check[kMaxSpecies];
   WlEnterJob& E = jobs[blockIdx.x];
   const ChainJob& J = E.job;
   const Geom g = J.g;
@@ -458,7 +457,7 @@ __global__ void __launch_bounds__(32, 1) wl_enter_kernel(WlEnterJob* __restrict_
   __syncwarp();
   unsigned long long draws = 0;
   int status = kStatusOk;
-  if (E.initial && !initial_setup_warp(E.init, lat, mt, pos, check, draws, lane)) status = kStatusBadSpecies;
+  if (E.initial && !initial_setup_warp(E.init, lat, mt, pos, draws, lane)) status = kStatusBadSpecies;
   const double lo = E.min_e, hi = E.max_e;
   const double target = __ddiv_rn(__dadd_rn(lo, hi), 2.0);
   const double cond = __dmul_rn(fabs(__dsub_rn(hi, lo)), 0.1);
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(32, 1) wl_enter_kernel(WlEnterJob* __restrict_
   for (int64_t it = 1; it <= E.max_steps && status == kStatusOk; ++it) {
     if (++i_steps % reinit == 0) {
       i_steps = 0;
-      if (!initial_setup_warp(E.init, lat, mt, pos, check, draws, lane)) {
+      if (!initial_setup_warp(E.init, lat, mt, pos, draws, lane)) {
         status = kStatusBadSpecies;
         break;
       }

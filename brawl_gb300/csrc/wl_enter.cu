@@ -83,7 +83,6 @@ __global__ void __launch_bounds__(256, 1) wl_enter_field_kernel(WlEnterJob* __re
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ FieldEnd end;
   __shared__ __align__(16) EnterShare S;
-  __shared__ int64_t check[kMaxSpecies];
   WlEnterJob& E = jobs[blockIdx.x];
   const ChainJob& J = E.job;
   const Geom g = J.g;
@@ -105,7 +104,7 @@ __global__ void __launch_bounds__(256, 1) wl_enter_field_kernel(WlEnterJob* __re
       int pos = (int)J.rng[kMTN];
       unsigned long long draws = 0;
       __syncwarp();
-      const bool ok = initial_setup_warp(E.init, J.lat, mt, pos, check, draws, lane);
+      const bool ok = initial_setup_warp(E.init, J.lat, mt, pos, draws, lane);
       __syncwarp();
       for (int i = lane; i < kMTN; i += 32) J.rng[i] = mt[i];
       if (lane == 0) {

@@ -1,0 +1,41 @@
+"""total_energy's ordered sum and the initial configurations at the edges: sums
+that grow through many binades, that stay near zero (energies of both signs),
+that are exactly zero and of few bits (ties), lattices below, at and past the
+256 terms taken at once; quotas of one atom and intervals that share a word."""
+import numpy as np
+import pytest
+
+import brawl_gb300 as B
+from oracle import oracle as O
+from tests.test_gpu_metropolis import conc_vector, random_V
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["random", "one sign", "few bits", "zero", "tiny"])
+def test_energies_at_the_edges_match_oracle(kind):
+    rng = np.random.default_rng(3)
+    for lattice, n, ns, nsh in [("fcc", (1, 2, 1), 2, 1), ("bcc", (4, 4, 4), 3, 2), ("fcc", (4, 4, 4), 2, 3),
+                                ("bcc", (5, 5, 7), 4, 4), ("fcc", (9, 8, 11), 5, 2), ("simple_cubic", (4, 5, 6), 3, 2),
+                                ("bcc", (17, 16, 15), 2, 6)]:
+        V = random_V(rng, ns, nsh)
+        if kind == "one sign":
+            V = -np.abs(V)
+        elif kind == "few bits":
+            V = np.round(V * 4096.0) / 64.0
+        elif kind == "zero":
+            V = np.zeros_like(V)
+        elif kind == "tiny":
+            V = V * 1e-200
+        setup = B.Setup(lattice, *n, ns, nsh)
+        mod = O.OracleModel(lattice, *n, V)
+        few = np.full(ns, 1, dtype=np.int64)
+        few[-1] = setup.n_atoms - (ns - 1)
+        chains = [dict(setup=setup, V=V, seed=60 + k, beta=1.0, species_concentrations=conc_vector(ns),
+                       species_numbers=few if k == 2 else None) for k in range(3)]
+        b = B.Batch(chains)
+        E = b.total_energy()
+        for k, c in enumerate(chains):
+            cfg, _ = mod.initial_setup(O.OracleRng(60 + k), conc_vector(ns), c["species_numbers"])
+            assert np.array_equal(b.config(k), cfg), (lattice, n, k)
+            assert E[k] == mod.total_energy(cfg), (lattice, n, k)
