@@ -57,12 +57,19 @@ int make_asro_plan(const Geom& g, int wc_range, const double* shells, AsroPlan& 
                                ((uint32_t)(uint8_t)dz << 16) | ((uint32_t)cls << 24));
       }
   plan.n_class = std::max(1, (int)plan.class_mask.size());
+  // by class: a site's pairs of one class are counted together
+  std::stable_sort(plan.offsets.begin(), plan.offsets.end(), [](uint32_t a, uint32_t b) { return a >> 24 < b >> 24; });
   return 0;
 }
 
 // One grid-stride pass over the chain's sites; each block keeps a shared
-// histogram of (species_i, species_j, class) and merges it at the end.
-__global__ void asro_kernel(const AsroJob* __restrict__ jp) {
+// histogram of (species_i, species_j, class) and merges it at the end.  A
+// thread counts its site's neighbours of a class by species in the bytes of two
+// words (eight species each) and adds them to the histogram when the class ends
+// (or the bytes could be full): a shared atomic per class and species, not per
+// pair, and no two pairs wait for one another.
+constexpr int kAsroThreads = 128;
+__global__ void __launch_bounds__(kAsroThreads) asro_kernel(const AsroJob* __restrict__ jp) {
   extern __shared__ unsigned int hist[];
   const AsroJob J = *jp;
   const Geom& g = J.g;
@@ -79,13 +86,27 @@ __global__ void asro_kernel(const AsroJob* __restrict__ jp) {
     const int si = J.lat[site];
     atomicAdd(&pcs[si], 1u);
     const int row = si * nsp;
-    for (int o = 0; o < J.n_offsets; ++o) {
-      int dx, dy, dz, cls;
-      unpack_entry(J.offsets[o], dx, dy, dz, cls);
-      const int nx = wrap_general(x, dx, W1), ny = wrap_general(y, dy, W2),
-                nz = wrap_general(z, dz, W3);
-      const int sj = J.lat[compact_index(g, nx, ny, nz)];
-      atomicAdd(&hist[(row + sj) * J.n_class + cls], 1u);
+    int o = 0;
+    while (o < J.n_offsets) {
+      const int cls = (int)(J.offsets[o] >> 24);
+      unsigned long long lo = 0, hi = 0;  // by species: 0 to 7, 8 to 15
+      const int end = min(J.n_offsets, o + 255);
+#pragma unroll 4
+      for (; o < end; ++o) {
+        int dx, dy, dz, c;
+        unpack_entry(J.offsets[o], dx, dy, dz, c);
+        if (c != cls) break;
+        // (no offset is longer than half a period)
+        const int nx = wrap_fast(x + dx, W1), ny = wrap_fast(y + dy, W2), nz = wrap_fast(z + dz, W3);
+        const int sj = J.lat[compact_index(g, nx, ny, nz)];
+        const unsigned long long one = 1ull << ((sj & 7) << 3);
+        lo += sj < 8 ? one : 0ull;
+        hi += sj < 8 ? 0ull : one;
+      }
+      for (int sj = 1; sj < nsp; ++sj) {
+        const unsigned n = (unsigned)((sj < 8 ? lo : hi) >> ((sj & 7) << 3)) & 0xffu;
+        if (n) atomicAdd(&hist[(row + sj) * J.n_class + cls], n);
+      }
     }
   }
   __syncthreads();
@@ -96,13 +117,13 @@ __global__ void asro_kernel(const AsroJob* __restrict__ jp) {
 }
 
 void launch_asro(const AsroJob* d_job, const Geom& g, int n_class, cudaStream_t stream) {
-  int blocks = (g.n_sites + 255) / 256;
-  blocks = std::max(1, std::min(blocks, 152 * 4));
+  int blocks = (g.n_sites + kAsroThreads - 1) / kAsroThreads;
+  blocks = std::max(1, std::min(blocks, 152 * 8));
   const int nsp = g.ns + 1;
   const size_t smem = (size_t)(nsp * nsp * n_class + nsp) * 4;
   cudaFuncSetAttribute(asro_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   BRAWL_CARVEOUT(asro_kernel);
-  asro_kernel<<<blocks, 256, smem, stream>>>(d_job);
+  asro_kernel<<<blocks, kAsroThreads, smem, stream>>>(d_job);
 }
 
 void finish_asro(const Geom& g, int wc_range, const AsroPlan& plan,

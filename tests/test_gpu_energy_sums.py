@@ -39,3 +39,18 @@ def test_energies_at_the_edges_match_oracle(kind):
             cfg, _ = mod.initial_setup(O.OracleRng(60 + k), conc_vector(ns), c["species_numbers"])
             assert np.array_equal(b.config(k), cfg), (lattice, n, k)
             assert E[k] == mod.total_energy(cfg), (lattice, n, k)
+
+
+@pytest.mark.parametrize("lattice,n,ns,wc", [("fcc", (1, 1, 1), 2, 1), ("bcc", (2, 1, 3), 7, 4), ("fcc", (5, 4, 6), 8, 6),
+                                             ("bcc", (6, 6, 7), 15, 12), ("simple_cubic", (4, 6, 5), 9, 3)])
+def test_pair_counts_at_the_edges_match_oracle(lattice, n, ns, wc):
+    """Species counted in either word of eight, lattices that an offset spans,
+    and shells beyond the offsets' reach."""
+    V = random_V(np.random.default_rng(5), ns, 1)
+    mod = O.OracleModel(lattice, *n, V)
+    ch = B.Chain(B.Setup(lattice, *n, ns, 1), V)
+    ch.seed(77)
+    ch.initial_setup(conc_vector(ns))
+    shells = ch.lattice_shells(wc)
+    rho, _ = mod.radial_densities(ch.config(), shells)
+    assert np.array_equal(np.asarray(ch.radial_densities(shells)), rho, equal_nan=True)
