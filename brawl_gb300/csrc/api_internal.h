@@ -44,7 +44,9 @@ int api_wl_kind(brawl_wl* wl);
 // the sweep kernel's variant for the walkers: largest z, every D staged
 void api_wl_variant(brawl_wl* wl, int* max_z, bool* all_D);
 NsRun* api_ns_device_run(brawl_ns* ns, int r);
+// Shared memory of the runs' walks, and whether they go in rounds (ns_rounds.cu).
 uint32_t api_ns_smem(brawl_ns* ns);
+int api_ns_kind(brawl_ns* ns);
 void api_ns_variant(brawl_ns* ns, int* max_z, bool* all_D);
 std::string api_last_error();
 

@@ -134,7 +134,7 @@ void words_within(const Geom& g, int dmx, int dmy, int dmz, uint32_t c[3], uint3
   }
 }
 
-// Halo staging of an fcc/bcc lattice (halo_engine.cuh): halo widths from the
+// Halo staging of an fcc/bcc lattice (halo_shear.cuh): halo widths from the
 // largest compact-index step of any entry at either parity; usable when the
 // images of a site are unique (2h <= N per axis), the pair-distance test is
 // exact (offsets within n per axis) and the difference table is staged.
@@ -163,15 +163,7 @@ void make_halo(const Geom& g, HaloGeom& H, bool& ok) {
   H.hx = hx;
   H.hy = hy;
   H.hz = hz;
-  H.SY = H.NX + 2 * hx;
-  H.SZ = (H.NY + 2 * hy) * H.SY;
-  const int64_t padded = (int64_t)(H.NZ + 2 * hz) * H.SZ;
-  H.origin = hz * H.SZ + hy * H.SY + hx;
-  H.dmx = dmx;
-  H.dmy = dmy;
-  H.dmz = dmz;
-  if (padded > (int64_t)1 << 30) return;
-  H.padded = (int32_t)padded;
+  if ((int64_t)(H.NZ + 2 * hz) * (H.NY + 2 * hy) * (H.NX + 2 * hx) > (int64_t)1 << 30) return;
   // sheared layout: rows and planes start where the ones before them end
   const int PX = H.NX + 2 * hx, PY = H.NY + 2 * hy;
   H.kSY = PX;
@@ -3074,7 +3066,8 @@ void api_wl_variant(brawl_wl* wl, int* max_z, bool* all_D) {
 }
 
 NsRun* api_ns_device_run(brawl_ns* ns, int r) { return ns->d_runs + r; }
-uint32_t api_ns_smem(brawl_ns* ns) { return ns->smem; }
+uint32_t api_ns_smem(brawl_ns* ns) { return ns->rounds ? ns->rounds_smem : ns->smem; }
+int api_ns_kind(brawl_ns* ns) { return ns->rounds ? 1 : 0; }
 void api_ns_variant(brawl_ns* ns, int* max_z, bool* all_D) {
   *max_z = ns->max_z;
   *all_D = ns->all_D;

@@ -49,8 +49,9 @@ constexpr int kMTN = 624;
 // Words mirrored past the end of a ring of tempered words (halo_engine.cuh),
 // so that up to this many consecutive words can be read without wrapping.
 constexpr int kRingMirror = 96;
-// trials per speculative round of the halo Metropolis kernel (1: one trial
-// at a time); brawl_batch_set_speculation overrides it per batch
+// depth of a chain in shared memory (1: the kernel's default, 2 to 4: gathered
+// sums in rounds of that many trials); brawl_batch_set_speculation overrides it
+// per batch
 constexpr int kDefaultSpeculation = 1;
 constexpr int kMTM = 397;
 constexpr int kMaxZ = 168;           // neighbour entries of bcc with 10 shells
@@ -87,18 +88,12 @@ struct Geom {
   int32_t pad;
 };
 
-// Halo layout of an fcc/bcc lattice staged in shared memory (see
-// halo_engine.cuh).
+// Layout of an fcc/bcc lattice staged in shared memory with its periodic halo
+// (halo_shear.cuh): rows of kSY and planes of kSZ shifted so that an entry's
+// index step is the same at every site.
 struct HaloGeom {
   int32_t NX, NY, NZ;     // compact extents
   int32_t hx, hy, hz;     // halo widths
-  int32_t SY, SZ;         // padded strides (x stride 1)
-  int32_t padded;         // padded byte count
-  int32_t origin;         // hz*SZ + hy*SY + hx
-  int32_t dmx, dmy, dmz;  // largest |offset| component per axis (doubled grid)
-  // Sheared layout of the windowed kernel (halo_shear.cuh): the same cells,
-  // rows of kSY and planes of kSZ shifted so that an entry's index step is
-  // the same at every site.
   int32_t kSY, kSZ, korg, kcells;
   int32_t kx, ky, kz;     // index step of one period along each axis
   uint32_t near_c[3], near_2c[3];  // near test on the words of z, x, y (words_near)
@@ -663,23 +658,6 @@ __device__ __forceinline__ int fast_ex2_decision(float nbql2, float c0, int dE, 
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x2));
   const float thr = __fmul_rn(e, 4294967296.0f);
-  const float wf = __uint2float_rn(w);
-  if (wf < __fmul_rn(thr, 1.0f - M)) return 1;
-  if (wf > __fmul_rn(thr, 1.0f + M)) return 0;
-  return -1;
-}
-
-// The same filter in the base-2 domain: x2 = -beta*q*log2(e)*dE, 2^x2 with
-// exp2f (<= 2 ulp).  The argument's float rounding (3 roundings, relative
-// 1.8e-7 of |x2|, i.e. 1.25e-7 |x2| relative on 2^x2), the band term and the
-// libm's own error are covered by M.
-__device__ __forceinline__ int fast_exp2_decision(float beta_q_l2, float beta_band, int dE,
-                                                  uint32_t w) {
-  const float x2 = -__fmul_rn(beta_q_l2, __int2float_rn(dE));
-  const float M = fabsf(x2) * 1.5e-7f + beta_band * 1.01f + 8.0e-7f;
-  if (!(M < 0.01f)) return -1;
-  if (x2 < -57.5f) return w != 0u ? 0 : -1;
-  const float thr = __fmul_rn(exp2f(x2), 4294967296.0f);
   const float wf = __uint2float_rn(w);
   if (wf < __fmul_rn(thr, 1.0f - M)) return 1;
   if (wf > __fmul_rn(thr, 1.0f + M)) return 0;

@@ -91,33 +91,7 @@ __device__ inline void build_axis_tables(const Geom& g, int32_t* tabs, const uin
   }
 }
 
-// Shared-memory layout of a chain staged with a halo (halo_engine.cuh).
-struct HaloLayout {
-  uint32_t mt, tbuf, ptab, ctab, V, ents, sstart, I, lat, total;
-  int32_t F_off, D_off;
-};
-
 constexpr int kTbufWords = 2 * kMTN + kRingMirror;  // the ring and its mirror
-
-__host__ __device__ inline HaloLayout halo_layout(const Geom& g, const HaloGeom& H) {
-  HaloLayout L;
-  const uint32_t nsp = (uint32_t)g.ns + 1;
-  const uint32_t nF = nsp * (uint32_t)g.nsh * nsp;
-  const uint32_t nD = nsp * nsp * (uint32_t)g.nsh * nsp;
-  L.mt = 0;
-  L.tbuf = align_up(kMTN * 4, 16);
-  L.ptab = align_up(L.tbuf + kTbufWords * 4, 16);  // the site tables, one int32 per word each
-  L.ctab = L.ptab + kTbufWords * 4;
-  L.V = align_up(L.ctab + kTbufWords * 4, 16);
-  L.ents = L.V + (uint32_t)(g.ns * g.ns * g.nsh) * 8;
-  L.sstart = L.ents + (uint32_t)g.z * 4;
-  L.I = align_up(L.sstart + (uint32_t)(g.nsh + 1) * 2, 16);
-  L.F_off = 0;
-  L.D_off = (int32_t)nF;
-  L.lat = align_up(L.I + (nF + nD) * 4, 16);
-  L.total = align_up(L.lat + (uint32_t)H.padded, 16);
-  return L;
-}
 
 // Shared memory of a chain of the windowed kernel (metropolis_halo.cu): the
 // stream's rings (trial_window.cuh), the positions' records and the lattice

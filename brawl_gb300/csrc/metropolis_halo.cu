@@ -1,5 +1,5 @@
 // metropolis_halo.cu -- Metropolis-Kawasaki swap trials for fcc/bcc chains
-// staged with a periodic halo (see halo_engine.cuh): the batched path's
+// staged with a periodic halo (see halo_shear.cuh): the batched path's
 // kernel for every lattice that fits.  One warp (CTA) per chain; trials in
 // the reference's order (monte_carlo_step_lattice / _nbr,
 // src/metropolis.F90:751-891) on the chain's own mt19937ar stream.

@@ -827,13 +827,16 @@ int launch_wl(brawl_server* S, Pipe& P) {
 
 int launch_ns(brawl_server* S, Pipe& P) {
   std::stable_sort(P.jobs.begin(), P.jobs.end(),
-                   [](const JobP& a, const JobP& b) { return api_ns_smem(a->ns) > api_ns_smem(b->ns); });
+                   [](const JobP& a, const JobP& b) {
+                     const int ka = api_ns_kind(a->ns), kb = api_ns_kind(b->ns);
+                     return ka != kb ? ka > kb : api_ns_smem(a->ns) > api_ns_smem(b->ns);
+                   });
   P.launched = P.jobs;
   const int n = (int)P.launched.size();
   std::vector<NsRun*> src(n);
   std::vector<int> ints(2 * n);
   std::vector<uint32_t> r_smem(n);
-  std::vector<int> r_z(n);
+  std::vector<int> r_z(n), r_kind(n);
   std::vector<char> r_D(n);
   int total = 0;
   const double t_round = round_ns(S, P.launched);
@@ -845,6 +848,7 @@ int launch_ns(brawl_server* S, Pipe& P) {
     ints[n + k] = total;
     total += (int)j.quantum;
     r_smem[k] = api_ns_smem(j.ns);
+    r_kind[k] = api_ns_kind(j.ns);
     int jz = 0;
     bool jd = true;
     api_ns_variant(j.ns, &jz, &jd);
@@ -863,14 +867,15 @@ int launch_ns(brawl_server* S, Pipe& P) {
   BRAWL_CARVEOUT(ns_stage_kernel);
   ns_stage_kernel<<<(n + 63) / 64, 64, 0, P.s>>>(P.d_ns, P.d_ns_src, n, P.d_limits, P.d_ns_int, P.d_ns_int + n,
                                                   P.d_tns);
-  SV_TRY(launch_groups(P, smem_groups(r_smem), [&](int first, int count, cudaStream_t st) {
+  SV_TRY(launch_groups(P, smem_groups(r_smem, &r_kind), [&](int first, int count, cudaStream_t st) {
     int max_z = 0;
     bool all_D = true;
     for (int k = first; k < first + count; ++k) {
       max_z = std::max(max_z, r_z[k]);
       all_D = all_D && r_D[k];
     }
-    launch_ns_iterate(P.d_ns + first, count, r_smem[first], max_z, all_D, st);
+    if (r_kind[first]) launch_ns_rounds(P.d_ns + first, count, r_smem[first], max_z, st);
+    else launch_ns_iterate(P.d_ns + first, count, r_smem[first], max_z, all_D, st);
   }));
   BRAWL_CARVEOUT(ns_unstage_kernel);
   ns_unstage_kernel<<<(n + 63) / 64, 64, 0, P.s>>>(P.d_ns, P.d_ns_src, n);
