@@ -437,11 +437,12 @@ class Batch:
         _check(load().brawl_batch_set_beta(self._h, _ptr(b)))
 
     def set_speculation(self, trials_per_round: int) -> None:
-        """Trials per speculative round of the fcc/bcc kernel (1-4); speed only."""
+        """How fcc/bcc chains in shared memory run: 1 the library's choice per
+        chain, 2-4 gathered sums in rounds of that many trials; speed only."""
         _check(load().brawl_batch_set_speculation(self._h, int(trials_per_round)))
 
     def autotune(self, n_trials, max_depth: int = 4) -> tuple[int, np.ndarray]:
-        """Times n_trials of every chain at each trials-per-round depth
+        """Times n_trials of every chain at each depth (set_speculation)
         1..max_depth from the same state (restored after each) and keeps
         the fastest; returns (depth, milliseconds per depth)."""
         t = self._trials(n_trials)

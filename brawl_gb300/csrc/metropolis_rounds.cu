@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kRoundThreads, 1) metropolis_rounds_kernel(con
   __shared__ FieldEnd end;
   __shared__ __align__(16) RoundShare S;
   const ChainJob& J = jobs[blockIdx.x];
+  if (J.status && *J.status != 0) return;  // the chain's input was flagged: no trial runs
   const Geom g = J.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned long long t_start = global_ns();

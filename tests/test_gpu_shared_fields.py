@@ -159,3 +159,20 @@ def test_rounds_of_trials_match_oracle(case):
             assert acc[c] == a, (T, k)
             assert np.array_equal(b.config(c), cfgs[c]), (T, k)
             assert _same_stream(b.rng_state(c), rngs[c]), (T, k)
+
+
+def test_rounds_of_trials_skip_a_flagged_chain():
+    """A simple cubic chain whose grid holds a bad species runs no trial; the
+    other one does."""
+    V = random_V(np.random.default_rng(1), 3, 2)
+    b = B.Batch([dict(setup=B.Setup("simple_cubic", 3, 4, 5, 3, 2), V=V, seed=9 + k, beta=100.0,
+                      species_concentrations=conc_vector(3)) for k in range(2)])
+    grids = b.get_configs()
+    good = grids.copy()
+    assert b.metropolis_host(grids, np.array([50, 60]))[1] >= 0
+    bad = good.copy()
+    bad[np.nonzero(bad)[0][0]] = 9
+    with pytest.raises(B.BrawlError):
+        b.metropolis_host(bad, np.array([50, 60]))
+    cnt = b.counters()
+    assert cnt[0][0] == 50 and cnt[1][0] == 120
