@@ -244,8 +244,8 @@ def roofline_object(achieved_gbs, smem_peak, peaks, traffic, alg_per_step, trial
            "traffic": traffic, "algorithmic_bytes_per_step": alg_per_step,
            "hbm": {"peak": peaks["hbm_gbs"], "frac": achieved_gbs / peaks["hbm_gbs"],
                    "peak_source": peaks["source"]},
-           "note": "latency-bound sequential chains (one warp per chain, a dependent chain of "
-                   "shared loads, a warp reduction and a decision per trial); achieved = the "
+           "note": "latency-bound sequential chains (a dependent chain of shared loads, "
+                   "warp reductions and decisions per round of trials); achieved = the "
                    "canonical algorithmic bytes per trial over the kernel's event time"}
     cs = committed_smem()
     if cs:
@@ -568,7 +568,7 @@ def walker_legs(args) -> dict:
             "roofline": {"bound": "latency", "achieved": alg / dt / 1e9, "peak": peaks["hbm_gbs"],
                          "peak_kind": "HBM copy, for scale", "unit": "GB/s",
                          "frac": alg / dt / 1e9 / peaks["hbm_gbs"],
-                         "note": "algorithmic bytes over host-timed calls; each walker is one warp's "
+                         "note": "algorithmic bytes over host-timed calls; each walker is one "
                                  "dependent chain of trials (lattice and tables in shared memory), so "
                                  "neither HBM nor shared-memory bandwidth bounds it"},
             "cpu_baseline": _wl_cpu(setup, V, cfgs[0], edges, bins, period),
@@ -625,7 +625,7 @@ def walker_legs(args) -> dict:
                          "peak_kind": "HBM copy, for scale", "unit": "GB/s",
                          "frac": alg / dt / 1e9 / peaks["hbm_gbs"],
                          "note": "algorithmic bytes over host-timed calls; one sequential run of "
-                                 "dependent walk steps, its flushes' FP64 sums spread over four warps"},
+                                 "dependent walk steps, eight evaluated at once, their FP64 sums beside them"},
             "cpu_baseline": _ns_cpu(V, conc),
         }
     return out
@@ -838,7 +838,8 @@ def main() -> int:
     ap.add_argument("--ns-runs", type=int, default=152,
                     help="independent nested-sampling runs of the replica-parallel measurement")
     ap.add_argument("--speculation", type=int, default=0,
-                    help="trials per speculative round of the Metropolis kernel (0: library default)")
+                    help="depth of the shared-memory chains: 1 the default kernels, 2-4 gathered sums in rounds of "
+                         "that many trials (0: library default)")
     args = ap.parse_args()
     if args.warmup < 3:
         args.warmup = 3
@@ -890,7 +891,7 @@ def main() -> int:
             tuned = batch.autotune_classes(sites, max_depth=4)
             cta_shape = {"picked_by": "autotune per chain class (whole-batch time, median of 3)",
                          "tuning_sample": "one sweep of every chain", **tuned}
-        except Exception as exc:  # keep one warp per chain and say why
+        except Exception as exc:  # keep the default kernels and say why
             batch.set_speculation(1)
             cta_shape = {"trials_per_round": 1, "picked_by": "default", "autotune_error": str(exc)[:200]}
 

@@ -191,10 +191,11 @@ int brawl_batch_destroy(brawl_batch *batch);
 int brawl_batch_size(brawl_batch *batch, int *n_chains);
 /* New inverse temperatures, one per chain. */
 int brawl_batch_set_beta(brawl_batch *batch, const double *beta);
-/* Trials per speculative round of the fcc/bcc Metropolis kernel (1-4, 1 =
- * one trial at a time, the default).  Speed only: the trajectory is the same. */
+/* How fcc/bcc chains in shared memory run: 1 (the default) with the library's
+ * choice per chain, 2-4 with gathered sums in rounds of that many trials.
+ * Speed only: the trajectory is the same. */
 int brawl_batch_set_speculation(brawl_batch *batch, int trials_per_round);
-/* Picks the trials per round by measurement: n_trials[c] trials of every
+/* Picks that depth by measurement: n_trials[c] trials of every
  * chain are timed at each depth 1..max_depth (<= 4) from the same state,
  * which is restored after each run, so the batch's chains, streams and
  * counters are as before the call.  ms (max_depth entries, may be NULL)
@@ -204,7 +205,7 @@ int brawl_batch_autotune(brawl_batch *batch, const int64_t *n_trials, int max_de
 /* Shared-memory chains are grouped in classes (same lattice, n1, n2, n3,
  * species and shells); after this call every class runs in its own launch,
  * concurrently with the others, with its own shared memory, unrolling and
- * trials per round.  The depths are picked per class by timing the whole
+ * depth.  The depths are picked per class by timing the whole
  * batch (n_trials[c] trials of every chain, three runs per try, from the
  * same state, restored after each): the classes in order of decreasing
  * work, each class's depths 1..max_depth with the others fixed, a deeper
@@ -214,7 +215,7 @@ int brawl_batch_autotune(brawl_batch *batch, const int64_t *n_trials, int max_de
  * trajectories do not depend on the depths. */
 int brawl_batch_autotune_classes(brawl_batch *batch, const int64_t *n_trials, int max_depth,
                                  int *depths, double *ms, int *n_classes);
-/* Trials per round of every class (n_classes entries, 1-4 each), set by
+/* The depth of every class (n_classes entries, 1-4 each), set by
  * the caller; every class then runs in its own launch as above. */
 int brawl_batch_set_class_depths(brawl_batch *batch, const int *depths);
 /* The class of every chain (-1: not a shared-memory chain). */
