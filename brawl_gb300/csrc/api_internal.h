@@ -38,9 +38,9 @@ int api_batch_set_rng(brawl_batch* b, int c, const uint32_t state[625]);
 cudaStream_t api_batch_stream(brawl_batch* b);
 brawl_batch* api_wl_batch(brawl_wl* wl);
 std::vector<WlWalker>& api_wl_walkers(brawl_wl* wl);
-uint32_t api_wl_smem(brawl_wl* wl);
+uint32_t api_wl_smem(brawl_wl* wl, int n, int n_sm);
 // 0, or 8 + the field_variant of walkers that run with fields
-int api_wl_kind(brawl_wl* wl);
+int api_wl_kind(brawl_wl* wl, int n, int n_sm);
 // the sweep kernel's variant for the walkers: largest z, every D staged
 void api_wl_variant(brawl_wl* wl, int* max_z, bool* all_D);
 NsRun* api_ns_device_run(brawl_ns* ns, int r);

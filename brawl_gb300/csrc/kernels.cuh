@@ -166,6 +166,16 @@ enum shared_kernel : int {
 inline double field_load(uint32_t smem) { return 2u * (smem + 1024u) <= 228u * 1024u ? 0.5 : 1.0; }
 inline bool fields_pay(double load, int n_sm) { return load <= 2.0 * n_sm; }
 
+// Wang-Landau walkers with fields (wl_field.cu: one to an SM, its registers fill
+// one) beside wl_sweep_kernel's, of which two share an SM: all while each has an
+// SM to itself; in more waves only with 40 neighbours or more, whose gathering
+// the fields save.  3,000 trials of 304 walkers, a third to nearly all of them
+// accepted, fields and sweeps: bcc with 14 neighbours 3.8-4.2 and 3.0-3.2 ms,
+// with 26 3.8-4.0 and 3.2-3.3, with 50 1.7-2.5 and 3.1-3.4, with 64 1.9-2.7 and
+// 3.2-3.8; 608 walkers: 6.2-7.9 and 5.8-6.0, 5.7 and 5.9, 3.3-4.9 and 6.0-6.3,
+// 3.3-4.8 and 6.1-7.0.
+inline bool wl_fields_pay(int n_walkers, int min_z, int n_sm) { return n_walkers <= n_sm || min_z >= 40; }
+
 // Chains in rounds of trials (metropolis_rounds.cu) where each has an SM to itself
 // (its sixteen warps' registers fill one): 152 chains take as long as one, 0.74 ms
 // (simple cubic 6^3, 4,000 trials) and 1.0 (8^3, two species), and twice as many

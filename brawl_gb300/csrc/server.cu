@@ -744,15 +744,16 @@ int launch_wl(brawl_server* S, Pipe& P) {
   std::vector<int> w_kind;
   std::vector<char> w_D;
   int max_bins = 0;
-  std::stable_sort(P.jobs.begin(), P.jobs.end(),
-                   [](const JobP& a, const JobP& b) {
-                     const int ka = api_wl_kind(a->wl), kb = api_wl_kind(b->wl);
-                     return ka != kb ? ka > kb : api_wl_smem(a->wl) > api_wl_smem(b->wl);
-                   });
+  size_t n_all = 0;
+  for (auto& j : P.jobs) n_all += j->d.wl_walkers;
+  auto kind_of = [&](const Job& j) { return api_wl_kind(j.wl, (int)n_all, S->n_sm); };
+  auto smem_of = [&](const Job& j) { return api_wl_smem(j.wl, (int)n_all, S->n_sm); };
+  std::stable_sort(P.jobs.begin(), P.jobs.end(), [&](const JobP& a, const JobP& b) {
+    const int ka = kind_of(*a), kb = kind_of(*b);
+    return ka != kb ? ka > kb : smem_of(*a) > smem_of(*b);
+  });
   P.launched = P.jobs;
   P.call_ends.assign(P.launched.size(), 0);
-  size_t n_all = 0;
-  for (auto& j : P.launched) n_all += j->d.wl_walkers;
   SV_TRY(grow(P.d_tns, P.tns_cap, std::max<size_t>(n_all, 1), P.s));
   const double t_round = round_ns(S, P.launched);
   for (size_t q = 0; q < P.launched.size(); ++q) {
@@ -786,9 +787,9 @@ int launch_wl(brawl_server* S, Pipe& P) {
     int jz = 0;
     bool jd = true;
     api_wl_variant(j.wl, &jz, &jd);
-    w_smem.insert(w_smem.end(), w.size(), api_wl_smem(j.wl));
+    w_smem.insert(w_smem.end(), w.size(), smem_of(j));
     w_z.insert(w_z.end(), w.size(), jz);
-    w_kind.insert(w_kind.end(), w.size(), api_wl_kind(j.wl));
+    w_kind.insert(w_kind.end(), w.size(), kind_of(j));
     w_D.insert(w_D.end(), w.size(), jd ? 1 : 0);
     max_bins = std::max(max_bins, j.d.wl_bins);
   }

@@ -176,3 +176,31 @@ def test_rounds_of_trials_skip_a_flagged_chain():
         b.metropolis_host(bad, np.array([50, 60]))
     cnt = b.counters()
     assert cnt[0][0] == 50 and cnt[1][0] == 120
+
+
+@pytest.mark.parametrize("nsh", [2, 6])
+def test_many_walkers_match_oracle(nsh):
+    """More walkers than the chip has SMs, with few and with many neighbours
+    (the sweeps' kernel is chosen by both)."""
+    lattice, n, ns, bins = "bcc", (3, 4, 3), 3, 40
+    V = random_V(np.random.default_rng(8), ns, nsh)
+    mod = O.OracleModel(lattice, *n, V)
+    r = O.OracleRng(5)
+    walkers, cfgs, rngs = [], [], []
+    E = []
+    for w in range(170):
+        cfg, _ = mod.initial_setup(r, conc_vector(ns))
+        E.append(mod.total_energy(cfg))
+        cfgs.append(cfg.copy())
+        rngs.append(O.OracleRng(300 + w))
+        walkers.append(dict(setup=B.Setup(lattice, *n, ns, nsh), V=V, seed=300 + w, config=cfg.copy(), start_idx=1,
+                            end_idx=bins, window=w))
+    span = float(np.ptp(E)) + 0.1
+    edges = min(E) - span + np.arange(bins + 1) * (3 * span / bins)
+    lngs = [np.zeros(bins) for _ in walkers]
+    hists = [np.zeros(bins) for _ in walkers]
+    wl = B.WangLandauWalkers(walkers, edges)
+    assert list(wl.sweeps(250, 0.1, 5)) == _emulate([mod] * 170, cfgs, rngs, walkers, edges, lngs, hists, 250, 0.1, 5)
+    for w in range(170):
+        assert np.array_equal(wl.lng(w), lngs[w]) and np.array_equal(wl.hist(w), hists[w])
+        assert np.array_equal(wl.config(w), cfgs[w])
