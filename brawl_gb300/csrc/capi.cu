@@ -269,6 +269,7 @@ struct Model {
   std::vector<int16_t> sstart;
   int S = 0;
   int band = 0;
+  double spread = 0.0;  // of a swap's energy changes in a random configuration (rms, as V)
 };
 
 // Fixed-point image of V_ex for the fast tier.  S is the largest shift with
@@ -310,6 +311,22 @@ int make_model(const brawl_setup& s, const double* V_ex, Model& m) {
   } else {
     m.S = 0;
     m.band = 0;
+  }
+  {
+    // two sites' neighbours, each a difference of two entries of V
+    const int16_t* st = shell_starts(g.lattice);
+    double var = 0.0;
+    for (int sh = 0; sh < g.nsh; ++sh) {
+      double sq = 0.0;
+      for (int a = 0; a < g.ns; ++a)
+        for (int b = 0; b < a; ++b)
+          for (int s = 0; s < g.ns; ++s) {
+            const double dv = m.V[a + g.ns * (s + g.ns * sh)] - m.V[b + g.ns * (s + g.ns * sh)];
+            sq += dv * dv;
+          }
+      var += 2.0 * (st[sh + 1] - st[sh]) * sq / std::max(1, g.ns * g.ns * (g.ns - 1) / 2);
+    }
+    m.spread = std::sqrt(var);
   }
   // D (see fixed_delta) follows F when it is small enough to stage
   if (smem_layout(g, false).use_D) {
@@ -543,6 +560,11 @@ int chain_kernel(const brawl_batch* b, int c, int depth) {
   return depth >= 2 && b->halo[c] ? kSharedGather : b->kernel[c];
 }
 
+// The trials of a gathered round of chain c, unless the caller chose.
+int gather_depth(const brawl_batch* b, int c) {
+  return b->spec_nc == 1 ? gather_trials(b->jobs[c].beta * b->models[c].spread) : b->spec_nc;
+}
+
 // Jobs go to the device in launch order: the shared-memory chains first, group
 // after group, then the rest; each group by decreasing trial count so the
 // longest chains start first, and the group with the longest chain first.  A
@@ -568,8 +590,8 @@ int upload_jobs(brawl_batch* b) {
     for (int c = 0; c < n; ++c) {
       const int k = b->cls[c];
       if (k < 0) continue;
-      gs[k].depth = b->class_depth[k];
-      gs[k].kernel = chain_kernel(b, c, gs[k].depth);
+      gs[k].kernel = chain_kernel(b, c, b->class_depth[k]);
+      gs[k].depth = b->class_depth[k] == 1 ? kGatherDefault : b->class_depth[k];
       add(c, k);
     }
   } else {
@@ -583,7 +605,7 @@ int upload_jobs(brawl_batch* b) {
     auto variant = [&](int c) {
       const Geom& g = b->models[c].g;
       return chain_kernel(b, c, b->spec_nc) == kSharedField ? 16 * ((g.z + kFieldHalf - 1) / kFieldHalf) + field_variant(g.ns)
-                                                           : lane_entries_for(g.z);
+                                                           : 8 * lane_entries_for(g.z) + gather_depth(b, c);
     };
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
       const int kx = chain_kernel(b, x, b->spec_nc), ky = chain_kernel(b, y, b->spec_nc);
@@ -598,7 +620,7 @@ int upload_jobs(brawl_batch* b) {
       if (gs.empty() || gs.back().kernel != k || nj != z || 3ull * need(c) < 2ull * gs.back().smem) {
         gs.push_back(LaunchGroup());
         gs.back().kernel = k;
-        gs.back().depth = b->spec_nc;
+        gs.back().depth = gather_depth(b, c);
         nj = z;
       }
       add(c, (int)gs.size() - 1);

@@ -161,10 +161,13 @@ enum shared_kernel : int {
 // gathered (GB300, 900 K, four species, six shells): 116 and 572 on bcc 8^3 at
 // one chain per SM, 273 and 590 at four, 527 and 658 at eight; 153 and 396 on
 // bcc 16^3 (one per SM) at one, 308 and 402 at two, 456 and 407 at three; on fcc
-// 8^3 with two species 310 and 368 at four, 456 and 414 at six.  So: fields
-// while they take two rounds of the SMs at most.
+// 8^3 with two species 310 and 368 at four, 456 and 414 at six.  Accepted swaps
+// cost the fields most: 6,000 trials of 400 chains of bcc 14^3, five species, two
+// shells, from random configurations 2.9 ms with fields and 2.2 gathered at 1500 K,
+// 3.9 and 2.6 at 4000 K, where 300 (two on an SM) take 1.7 and 2.2.  So: fields
+// while every chain with them has its place at once.
 inline double field_load(uint32_t smem) { return 2u * (smem + 1024u) <= 228u * 1024u ? 0.5 : 1.0; }
-inline bool fields_pay(double load, int n_sm) { return load <= 2.0 * n_sm; }
+inline bool fields_pay(double load, int n_sm) { return load <= n_sm; }
 
 // Wang-Landau walkers with fields (wl_field.cu: one to an SM, its registers fill
 // one) beside wl_sweep_kernel's, of which two share an SM: all while each has an
@@ -186,17 +189,29 @@ uint32_t round_smem_bytes(const Geom& g, bool nibbles);
 void launch_metropolis_rounds(const ChainJob* d_jobs, int n_jobs, bool nibbles, uint32_t smem_bytes, int max_z,
                               cudaStream_t stream);
 
+// Trials per round of the gather kernel, by how hot the chain is: its inverse
+// temperature times the spread of its swaps' energy changes.  The hotter, the
+// fewer trials a round keeps.  Rounds of one, two and three, a first call from
+// random configurations / later ones (ms): 600 chains of bcc 10^3, two species, six
+// shells at 0.9: 2.08/2.01, 2.28/2.17 and 2.46/2.38, at 1.3: 1.98/1.92, 2.07/1.97
+// and 2.25/2.10; 563 of bcc 22^3, four shells at 0.8: 7.2/7.0, 7.4/7.2 and 7.7/7.4,
+// at 1.2: 7.0/6.7, 7.0/6.4 and 7.1/6.4, at 1.9: 6.8/6.0, 6.5/5.3 and 6.5/5.0; 400 of
+// bcc 14^3, five species, two shells at 1.0: 2.50/2.37, 2.35/2.13 and 2.50/2.21.
+// Four lose to three from random configurations (256 of bcc 24^3 at 600 K: 5.9/4.0
+// and 5.7/4.1).
+constexpr int kGatherDefault = 3;
+inline int gather_trials(double beta_spread) { return beta_spread < 0.95 ? 1 : beta_spread < 1.5 ? 2 : kGatherDefault; }
+
 // One launch of them: `count` chains from `first` in launch order, the largest
 // shared memory and neighbour count among them, and the trials per
-// round of the gather kernel (1: kGatherDefault).
+// round of the gather kernel.
 struct LaunchGroup {
-  int kernel = kSharedNone, depth = 1, first = -1, count = 0;
+  int kernel = kSharedNone, depth = kGatherDefault, first = -1, count = 0;
   uint32_t smem = 0;
   int max_z = 0;
   int ns = 0;        // species of one of them (field kernel: all are of its field_variant)
   int64_t most = 0;  // the most trials of one chain
 };
-constexpr int kGatherDefault = 4;
 void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int depth,
                             cudaStream_t stream);
 void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int ns,

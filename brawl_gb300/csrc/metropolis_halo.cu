@@ -419,9 +419,11 @@ __global__ void __launch_bounds__(32) metropolis_halo_kernel(const ChainJob* __r
       // every axis of this lane has an image there
       if (lane < 16 && ((code | code >> 1) & 0x15) == (img_axes & 0x15))
         lat[cell] = (uint8_t)(img_at == kFlagImg1 ? s2 : s1);
-      // the records of the two windows that name either site
-      const bool a0 = (ca0 == q.x) | (ca0 == q.z), b0 = (cb0 == q.x) | (cb0 == q.z);
-      const bool a1 = (ca1 == q.x) | (ca1 == q.z), b1 = (cb1 == q.x) | (cb1 == q.z);
+      // the records of the two windows, of the positions still to come, that name
+      // either site
+      const bool on0 = lane > p, on1 = kWin + lane > p;
+      const bool a0 = on0 & ((ca0 == q.x) | (ca0 == q.z)), b0 = on0 & ((cb0 == q.x) | (cb0 == q.z));
+      const bool a1 = on1 & ((ca1 == q.x) | (ca1 == q.z)), b1 = on1 & ((cb1 == q.x) | (cb1 == q.z));
       if (__any_sync(kFull, a0 | b0 | a1 | b1)) {
         auto renew = [&](int at, int ca, int cb, bool ha, bool hb) {
           const int old = flags[at];
@@ -469,8 +471,9 @@ static void launch_halo_nj(const ChainJob* d_jobs, int n_jobs, uint32_t smem_byt
 template <int NJ>
 static void launch_halo_depth(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int depth, cudaStream_t stream) {
   switch (depth) {
+    case 1: launch_halo_nj<NJ, 1>(d_jobs, n_jobs, smem_bytes, stream); break;
     case 2: launch_halo_nj<NJ, 2>(d_jobs, n_jobs, smem_bytes, stream); break;
-    case 3: launch_halo_nj<NJ, 3>(d_jobs, n_jobs, smem_bytes, stream); break;
+    case 4: launch_halo_nj<NJ, 4>(d_jobs, n_jobs, smem_bytes, stream); break;
     default: launch_halo_nj<NJ, kGatherDefault>(d_jobs, n_jobs, smem_bytes, stream); break;
   }
 }

@@ -204,3 +204,23 @@ def test_many_walkers_match_oracle(nsh):
     for w in range(170):
         assert np.array_equal(wl.lng(w), lngs[w]) and np.array_equal(wl.hist(w), hists[w])
         assert np.array_equal(wl.config(w), cfgs[w])
+
+
+@pytest.mark.parametrize("T", [300.0, 2500.0, 20000.0])
+def test_many_chains_match_oracle(T):
+    """More chains with fields than have their place at once: the gather kernel, in
+    rounds of three, two and one trials by temperature."""
+    lattice, n, ns, nsh = "bcc", (3, 3, 4), 3, 2
+    V = random_V(np.random.default_rng(2), ns, nsh)
+    mod = O.OracleModel(lattice, *n, V)
+    beta = 1.0 / (T * B.K_B_IN_RY)
+    b = B.Batch([dict(setup=B.Setup(lattice, *n, ns, nsh), V=V, seed=400 + k, beta=beta,
+                      species_concentrations=conc_vector(ns)) for k in range(330)])
+    acc = b.metropolis(700)
+    for k in range(330):
+        r = O.OracleRng(400 + k)
+        cfg, _ = mod.initial_setup(r, conc_vector(ns))
+        a, _ = mod.mc_run(cfg, r, beta, 700, False)
+        assert acc[k] == a and np.array_equal(b.config(k), cfg), k
+        if k % 40 == 0:
+            assert _same_stream(b.rng_state(k), r), k
