@@ -10,7 +10,6 @@
 #include <cstring>
 #include <ctime>
 #include <deque>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -218,46 +217,51 @@ bool make_field(const Geom& g, FieldTabs& T) {
   };
   // per displacement that is an entry's, the entries of site 1 and of site 2
   // that meet the other site, by shell
-  std::map<int, std::vector<uint8_t>> met;
+  const int row = 2 * g.nsh;
+  std::vector<uint8_t> met((size_t)cells * row, 0), hit(cells, 0);
   const int16_t* st = shell_starts(g.lattice);
   for (int sh = 0; sh < g.nsh; ++sh)
     for (int k = st[sh]; k < st[sh + 1]; ++k)
       for (int side = 0; side < 2; ++side) {
-        std::vector<uint8_t>& v = met[cell(side == 0 ? 1 : -1, offs[k])];
-        v.resize(2 * g.nsh, 0);
-        v[2 * sh + side] += 1;
+        const int at = cell(side == 0 ? 1 : -1, offs[k]);
+        met[(size_t)at * row + 2 * sh + side] += 1;
+        hit[at] = 1;
       }
   T.fg.distinct = 1;
   T.fg.symmetric = 1;
+  auto key = [](int x, int y, int z) { return (x + 64) + 128 * ((y + 64) + 128 * (z + 64)); };
+  std::vector<int> there, back;
   for (int sh = 0; sh < g.nsh; ++sh) {
     // the shell's entries and their opposites, as sets with repeats
-    std::map<int, int> count;
-    auto key = [](int x, int y, int z) { return (x + 64) + 128 * ((y + 64) + 128 * (z + 64)); };
+    there.clear();
+    back.clear();
     for (int k = st[sh]; k < st[sh + 1]; ++k) {
-      count[key(offs[k][0], offs[k][1], offs[k][2])] += 1;
-      count[key(-offs[k][0], -offs[k][1], -offs[k][2])] -= 1;
+      there.push_back(key(offs[k][0], offs[k][1], offs[k][2]));
+      back.push_back(key(-offs[k][0], -offs[k][1], -offs[k][2]));
     }
-    for (const auto& e : count)
-      if (e.second != 0) T.fg.symmetric = 0;
-  }
-  for (const auto& e : met) {
-    int once = 0;
-    for (int sh = 0; sh < g.nsh; ++sh) once += e.second[2 * sh];
-    if (once > 1) T.fg.distinct = 0;
+    std::sort(there.begin(), there.end());
+    std::sort(back.begin(), back.end());
+    if (there != back) T.fg.symmetric = 0;
   }
   T.dtab.assign(cells, 0);
-  T.sig.assign(2 * g.nsh, 0);  // class 0
-  std::map<std::vector<uint8_t>, int> ids;
-  for (const auto& e : met) {
-    auto it = ids.find(e.second);
-    if (it == ids.end()) {
-      it = ids.emplace(e.second, (int)ids.size() + 1).first;
-      T.sig.insert(T.sig.end(), e.second.begin(), e.second.end());
+  T.sig.assign(row, 0);  // class 0
+  int n_class = 1;
+  for (int at = 0; at < cells; ++at) {
+    if (!hit[at]) continue;
+    const uint8_t* m = met.data() + (size_t)at * row;
+    int once = 0;
+    for (int sh = 0; sh < g.nsh; ++sh) once += m[2 * sh];
+    if (once > 1) T.fg.distinct = 0;
+    int id = 1;
+    while (id < n_class && std::memcmp(T.sig.data() + (size_t)id * row, m, row) != 0) ++id;
+    if (id == n_class) {
+      if (n_class > 255) return false;
+      T.sig.insert(T.sig.end(), m, m + row);
+      ++n_class;
     }
-    if (it->second > 255) return false;
-    T.dtab[e.first] = (uint8_t)it->second;
+    T.dtab[at] = (uint8_t)id;
   }
-  T.fg.n_class = (int)ids.size() + 1;
+  T.fg.n_class = n_class;
   return true;
 }
 

@@ -1,5 +1,5 @@
 // ns_rounds.cu -- the walks of nested sampling (src/nested_sampling.f90:115-206)
-// in rounds of four steps, for runs whose lattice, tables and logs fit in shared
+// in rounds of eight steps, for runs whose lattice, tables and logs fit in shared
 // memory (ns_rounds_smem_bytes): what ns_iterate_kernel does, step for step, on
 // the same state.
 //
