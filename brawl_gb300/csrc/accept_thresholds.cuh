@@ -18,7 +18,8 @@ namespace brawl {
 // here (float conversion of w, lg2.approx, the subtraction: together below
 // 2e-5 on [0, 32]) with room to spare.  The float products carry a further
 // relative 1e-6 and the thresholds are rounded towards the undecided side.
-// Between the two, and for w = 0, the exact tier decides.
+// Between the two, and for w = 0, the exact tier decides.  For beta >= 0 only: with
+// any other the band holds every change (set_beta, capi.cu) and these decide none.
 struct AcceptThresholds {
   int acc_below;  // dE < acc_below: accepted
   int rej_above;  // dE > rej_above: rejected

@@ -354,8 +354,13 @@ int make_model(const brawl_setup& s, const double* V_ex, Model& m) {
   return BRAWL_OK;
 }
 
+// The kernels' uphill tests (accept_thresholds, fast_exp_decision) take beta >= 0.
+// Below zero (the sign of -0.0 included) every uphill move is accepted and with a
+// beta that is not a number none: the band then holds every change (+-2^30 at
+// most), and the exact tier decides each.
 void set_beta(ChainJob& j, const Model& m, double beta) {
   j.beta = beta;
+  j.band = beta >= 0.0 && !std::signbit(beta) ? m.band : 1 << 30;
   const double q = std::ldexp(1.0, -m.S);
   j.beta_q = (float)(beta * q);
   double bb = beta * (double)m.band * q;
@@ -990,7 +995,6 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
       if (tabs[c]) j.fg = tabs[c]->fg;
     }
     j.nbr_swap = b->nbr_swap[c];
-    j.band = m.band;
     set_beta(j, m, chains[c].beta);
     j.lat = reinterpret_cast<int8_t*>(b->arena + off_lat[c]);
     j.rng = reinterpret_cast<uint32_t*>(b->arena + off_rng[c]);
@@ -1842,7 +1846,6 @@ int brawl_set_interactions(brawl_ctx* ctx, const double* V_ex) {
   CUDA_TRY(stream_wait(b->stream));
   const double beta = j.beta;
   b->models[0] = m;
-  j.band = m.band;
   set_beta(j, m, beta);
   return BRAWL_OK;
 }
