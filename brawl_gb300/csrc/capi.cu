@@ -876,13 +876,13 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
       HaloGeom H;
       bool ok;
       make_halo(m.g, H, ok);
-      if (ok && window_layout(m.g, H).total <= (uint32_t)max_optin) {
+      if (ok && window_layout(m.g, H).total <= layout_room(max_optin, kOneWarpOwn)) {
         b->halo[c] = 1;
         b->gather_smem[c] = window_layout(m.g, H).total;
         b->kernel[c] = kSharedGather;
       }
       FieldTabs T;
-      if (make_field(m.g, T) && field_layout(m.g, T.fg).total <= (uint32_t)max_optin) {
+      if (make_field(m.g, T) && field_layout(m.g, T.fg).total <= layout_room(max_optin, kFieldOwn)) {
         field_tabs.push_back(std::move(T));
         tabs[c] = &field_tabs.back();
         b->field_smem[c] = field_layout(m.g, tabs[c]->fg).total;
@@ -916,13 +916,14 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     if (!fields_pay(load, n_sm))
       for (int c = 0; c < n_chains; ++c)
         if (b->halo[c]) b->kernel[c] = kSharedGather;
-    b->rest_nibbles = rest_bytes > (uint32_t)max_optin;
+    const uint32_t room = layout_room(max_optin, kRoundsOwn);
+    b->rest_nibbles = rest_bytes > room;
     b->rest_smem = b->rest_nibbles ? rest_nibbles : rest_bytes;
-    b->rest_rounds = n_rest > 0 && rest_fits && b->rest_smem <= (uint32_t)max_optin && rounds_pay(n_rest, n_sm);
+    b->rest_rounds = n_rest > 0 && rest_fits && b->rest_smem <= room && rounds_pay(n_rest, n_sm);
   }
-  b->smem_lat = need_smem <= (uint32_t)max_optin;
+  b->smem_lat = need_smem <= layout_room(max_optin, kOneWarpOwn);
   b->smem_bytes = b->smem_lat ? need_smem : need_gmem;
-  if (b->smem_bytes > (uint32_t)max_optin)
+  if (b->smem_bytes > layout_room(max_optin, kOneWarpOwn))
     return cleanup(fail(BRAWL_EINVAL, "interaction tables exceed shared memory"));
   // arena layout
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
@@ -2135,11 +2136,11 @@ extern "C" int brawl_ns_create(const brawl_ns_desc* descs, int n_runs, brawl_ns*
       return cleanup(fail(BRAWL_EINVAL, "run " + std::to_string(r) + ": bad n_walkers/n_steps/concentrations"));
     NsRun& R = ns->runs[r];
     std::memset(&R, 0, sizeof(R));
-    R.lazy_cap = lazy_cap_for(m.g, ns_smem_bytes(m.g, 0), (uint32_t)max_optin);
+    R.lazy_cap = lazy_cap_for(m.g, ns_smem_bytes(m.g, 0), layout_room(max_optin, kOneWarpOwn));
     if (R.lazy_cap == 0)
       return cleanup(fail(BRAWL_EINVAL, "run " + std::to_string(r) + ": lattice too large for shared memory"));
     ns->smem = std::max(ns->smem, ns_smem_bytes(m.g, R.lazy_cap));
-    if (ns_plan_rounds(m.g, R, (uint32_t)max_optin))
+    if (ns_plan_rounds(m.g, R, layout_room(max_optin, kNsRoundsOwn)))
       ns->rounds_smem = std::max(ns->rounds_smem, ns_rounds_smem_bytes(m.g, R.rounds_cap));
     else
       ns->rounds = false;
@@ -2156,7 +2157,7 @@ extern "C" int brawl_ns_create(const brawl_ns_desc* descs, int n_runs, brawl_ns*
     total_sites += (int64_t)R.K * m.g.n_sites;
     max_K = std::max(max_K, R.K);
   }
-  if (ns->smem > (uint32_t)max_optin)
+  if (ns->smem > layout_room(max_optin, kOneWarpOwn))
     return cleanup(fail(BRAWL_EINVAL, "a run's lattice and tables exceed shared memory"));
   auto nsalloc = [&](size_t bytes, void** p) -> int {
     cudaError_t e = dalloc(p, bytes, ns->stream);
@@ -2417,7 +2418,7 @@ static void wl_plan_fields(brawl_wl* wl) {
     wl->min_z = std::min(wl->min_z, (int)g.z);
     W.field_cap = 0;
     if (W.job.fg.n_class > 0 && W.job.fg.symmetric)
-      W.field_cap = lazy_cap_for(g, wl_field_smem_bytes(g, W.job.fg, nb, 0), (uint32_t)max_optin);
+      W.field_cap = lazy_cap_for(g, wl_field_smem_bytes(g, W.job.fg, nb, 0), layout_room(max_optin, kWlFieldOwn));
     if (W.field_cap < std::min(16, W.lazy_cap) || field_variant(g.ns) != wl->variant) wl->fields = false;
     if (W.field_cap > 0)
       wl->field_smem = std::max(wl->field_smem, wl_field_smem_bytes(g, W.job.fg, nb, W.field_cap));
@@ -2502,7 +2503,7 @@ extern "C" int brawl_wl_create(const brawl_wl_desc* walkers, int n, int bins,
     W.range = wl->range;
     hoff += W.end - W.start + 1;
     const uint32_t base = wl_smem_bytes(W.job.g, W.end - W.start + 1, 0);
-    W.lazy_cap = lazy_cap_for(W.job.g, base, (uint32_t)max_optin);
+    W.lazy_cap = lazy_cap_for(W.job.g, base, layout_room(max_optin, kOneWarpOwn));
     if (W.lazy_cap == 0) return cleanup(fail(BRAWL_EINVAL, "window or lattice too large for shared memory"));
     wl->smem = std::max(wl->smem, wl_smem_bytes(W.job.g, W.end - W.start + 1, W.lazy_cap));
     wl->max_z = std::max(wl->max_z, (int)W.job.g.z);
@@ -2510,7 +2511,8 @@ extern "C" int brawl_wl_create(const brawl_wl_desc* walkers, int n, int bins,
     if (c == 0 || walkers[c].window != walkers[c - 1].window) wl->groups.push_back({c, 0});
     wl->groups.back().count += 1;
   }
-  if (wl->smem > (uint32_t)max_optin) return cleanup(fail(BRAWL_EINVAL, "window or lattice too large for shared memory"));
+  if (wl->smem > layout_room(max_optin, kOneWarpOwn))
+    return cleanup(fail(BRAWL_EINVAL, "window or lattice too large for shared memory"));
   if (dalloc(&wl->d_groups, wl->groups.size() * sizeof(WlGroup), ws) != cudaSuccess)
     return cleanup(fail(BRAWL_ENOMEM, "groups"));
   wl->per_window = wl->groups[0].count;
@@ -2706,7 +2708,7 @@ extern "C" int brawl_wl_enter_windows(brawl_wl* wl, double energy_min, double en
     max_z = std::max(max_z, (int)m.g.z);
     const FieldGeom& f = E.job.fg;
     if (f.n_class > 0 && f.symmetric)
-      E.field_cap = lazy_cap_for(m.g, wl_enter_field_smem_bytes(m.g, f, 0), (uint32_t)max_optin);
+      E.field_cap = lazy_cap_for(m.g, wl_enter_field_smem_bytes(m.g, f, 0), layout_room(max_optin, kWlEnterOwn));
     if (E.field_cap < 16 || field_variant(m.g.ns) != variant) fields = false;
     else field_smem = std::max(field_smem, wl_enter_field_smem_bytes(m.g, f, E.field_cap));
   }
@@ -2750,7 +2752,7 @@ extern "C" int brawl_wl_radial_enable(brawl_wl* wl, int wc_range, const double* 
   uint32_t smem = 0;
   for (const WlWalker& W : wl->w)
     smem = std::max(smem, wl_smem_bytes(W.job.g, W.end - W.start + 1, W.lazy_cap, wl->bins, n_off, n_class));
-  if (smem > (uint32_t)max_optin) return fail(BRAWL_EINVAL, "radial-sample scratch does not fit in shared memory");
+  if (smem > layout_room(max_optin, kOneWarpOwn)) return fail(BRAWL_EINVAL, "radial-sample scratch does not fit in shared memory");
   const size_t per = (size_t)g0.ns * g0.ns * wc_range;
   cudaStream_t s = b->stream;
   std::vector<unsigned long long> masks(plan.class_mask.begin(), plan.class_mask.end());
@@ -2948,14 +2950,14 @@ extern "C" int brawl_wl_set_windows(brawl_wl* wl, const int* start_idx, const in
     for (int c = G.first; c < G.first + G.count; ++c) {
       const Geom& g = wl->w[c].job.g;
       const uint32_t base = wl_smem_bytes(g, nb, 0, rad_bins, wl->rad_n_off, wl->rad_n_class);
-      cap[c] = lazy_cap_for(g, base, (uint32_t)max_optin);
+      cap[c] = lazy_cap_for(g, base, layout_room(max_optin, kOneWarpOwn));
       if (cap[c] == 0) return fail(BRAWL_EINVAL, "window " + std::to_string(k + 1) + " too large for shared memory");
       smem = std::max(smem, wl_smem_bytes(g, nb, cap[c], rad_bins, wl->rad_n_off, wl->rad_n_class));
       all_D = all_D && walker_layout(g, nb, cap[c]).use_D;
       hist_total += (size_t)nb;
     }
   }
-  if (smem > (uint32_t)max_optin) return fail(BRAWL_EINVAL, "windows too large for shared memory");
+  if (smem > layout_room(max_optin, kOneWarpOwn)) return fail(BRAWL_EINVAL, "windows too large for shared memory");
   // mpi_arrays (src/wang-landau.F90:1351-1379): the histograms start from 0
   cudaStream_t s = b->stream;
   double* d_hist = nullptr;

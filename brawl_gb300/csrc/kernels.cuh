@@ -22,6 +22,15 @@ struct SmemLayout {
 
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
+// Shared memory that kernels hold in variables of their own, beside their layouts:
+// a layout has a block's limit less these bytes (layout_room).
+constexpr uint32_t kOneWarpOwn = 16;  // metropolis_kernel, metropolis_halo_kernel, ns_iterate_kernel, wl_sweep_kernel
+constexpr uint32_t kFieldOwn = 1584;  // metropolis_field_kernel
+constexpr uint32_t kRoundsOwn = 544;  // metropolis_rounds_kernel
+template <class... Own>
+constexpr uint32_t own_bytes() { return ((uint32_t)((sizeof(Own) + 15) / 16 * 16) + ...); }
+inline uint32_t layout_room(int limit, uint32_t own) { return (uint32_t)limit - own; }
+
 constexpr uint32_t kMaxDBytes = 12 * 1024;
 
 __host__ __device__ inline SmemLayout smem_layout(const Geom& g, bool lattice_in_smem) {

@@ -16,6 +16,7 @@ struct FieldShare {
   unsigned rej[2][2];
   int verdict;  // the exact tier's: bit 0 accepted, bit 1 uniform drawn
 };
+static_assert(own_bytes<FieldEnd, FieldShare>() == kFieldOwn, "what the layout leaves room for");
 
 // One chain per block.  All warps stage the tables and sum the fields; then four
 // make the windows' records and the team of four decides the trials.  The team

@@ -79,6 +79,7 @@ struct RoundShare {
   int stale[2][kWin];
   int verdict;
 };
+static_assert(own_bytes<FieldEnd, RoundShare>() == kRoundsOwn, "what the layout leaves room for");
 
 }  // namespace
 

@@ -64,6 +64,7 @@ void launch_ns_iterate(NsRun* d_runs, int n_runs, uint32_t smem_bytes, int max_z
 
 // The walks in rounds of steps (ns_rounds.cu), for runs of at most 65535 sites and
 // 512 cells a side whose sites are no neighbours of themselves.
+constexpr uint32_t kNsRoundsOwn = 336;  // (layout_room)
 uint32_t ns_rounds_smem_bytes(const Geom& g, int cap);
 void launch_ns_rounds(NsRun* d_runs, int n_runs, uint32_t smem_bytes, int max_z, cudaStream_t stream);
 

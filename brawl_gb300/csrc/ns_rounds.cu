@@ -95,6 +95,7 @@ struct NsShare {
   unsigned long long best[kNsTeam / 32];
   int best_at[kNsTeam / 32];
 };
+static_assert(own_bytes<FieldEnd, NsShare>() == kNsRoundsOwn, "what the layout leaves room for");
 
 // Barriers besides the makers': the team's (6), a half is handed over (7), it is
 // summed (8), the summing warps' own (9).

@@ -718,7 +718,7 @@ int launch_anneal(brawl_server* S, Pipe& P) {
     }));
   }
   if (n - nh > 0) {
-    const bool smem_lat = lat_smem <= (uint32_t)S->max_optin;
+    const bool smem_lat = lat_smem <= layout_room(S->max_optin, kOneWarpOwn);
     launch_metropolis(P.d_chain + nh, n - nh, smem_lat, use_D, smem_lat ? lat_smem : glob_smem, table_z, P.s);
   }
   SV_CUDA(cudaGetLastError());

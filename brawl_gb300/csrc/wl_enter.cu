@@ -43,6 +43,7 @@ struct EnterShare {
   double e;  // the energy after the walk, its steps, and whether it is settled
   int t, status, ok;
 };
+static_assert(own_bytes<FieldEnd, EnterShare>() == kWlEnterOwn, "what the layout leaves room for");
 
 // full_energy (src/bw_hamiltonian.f90:58-81): the site energies by all threads,
 // their sum in site order on one, and the half.

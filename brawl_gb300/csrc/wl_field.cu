@@ -56,6 +56,7 @@ struct WlShare {
   double e_sw;
   int verdict;
 };
+static_assert(own_bytes<FieldEnd, WlShare>() == kWlFieldOwn, "what the layout leaves room for");
 
 // field_walk (field_engine.cuh) for the masks of trials that draw n_base + 1
 // words and n_base words.

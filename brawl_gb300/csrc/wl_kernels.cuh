@@ -74,6 +74,7 @@ uint32_t wl_enter_smem_bytes(const Geom& g);
 void launch_wl_enter(WlEnterJob* d_jobs, int n, uint32_t smem, cudaStream_t stream);
 // The same with the sites' fields in shared memory (wl_enter.cu), for walkers with
 // a field_cap, of one field_variant.
+constexpr uint32_t kWlEnterOwn = 1600;  // (layout_room)
 uint32_t wl_enter_field_smem_bytes(const Geom& g, const FieldGeom& f, int cap);
 void launch_wl_enter_field(WlEnterJob* d_jobs, int n, uint32_t smem, int max_z, int variant, cudaStream_t stream);
 
@@ -92,6 +93,7 @@ void launch_wl_sweeps(WlWalker* d_walkers, int n, uint32_t smem, int max_z, bool
                       cudaStream_t stream);
 // The same with the sites' fields in shared memory (wl_field.cu), for walkers
 // with a field_cap, of one field_variant and without radial samples.
+constexpr uint32_t kWlFieldOwn = 2080;  // (layout_room)
 uint32_t wl_field_smem_bytes(const Geom& g, const FieldGeom& f, int nb, int cap);
 void launch_wl_field(WlWalker* d_walkers, int n, uint32_t smem, int max_z, int variant, cudaStream_t stream);
 void launch_wl_average(const WlGroup* d_groups, int n_groups, WlWalker* d_walkers, int bins,
