@@ -501,7 +501,7 @@ struct brawl_batch {
   bool per_class = false;                // class depths chosen (brawl_batch_autotune_classes)
   std::vector<unsigned long long> last_counters;
   int device = 0;
-  int max_optin = 0;
+  int n_sm = 0;
   int spec_nc = kDefaultSpeculation;     // trials per round of every chain (launch_shared_chains)
   double* d_alro = nullptr;              // ALRO counts: per chain ns x n_sites
   int64_t* d_alro_off = nullptr;
@@ -635,6 +635,9 @@ int upload_jobs(brawl_batch* b) {
       add(c, (int)gs.size() - 1);
     }
   }
+  int n_fields = 0;
+  for (const LaunchGroup& G : gs) n_fields += G.kernel == kSharedField ? G.count : 0;
+  for (LaunchGroup& G : gs) G.threads = field_threads(n_fields, b->n_sm);
   std::vector<int> rank(gs.size()), at(gs.size());
   for (size_t k = 0; k < gs.size(); ++k) at[k] = (int)k;
   std::stable_sort(at.begin(), at.end(), [&](int x, int y) { return gs[x].most > gs[y].most; });
@@ -786,8 +789,9 @@ int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accept
   if (!serial) {
     TRY(launch_sweep(b, stream));
   } else {
-    for (const LaunchGroup& G : b->groups)
+    for (LaunchGroup G : b->groups)
       for (int k = G.first; k < G.first + G.count; ++k) {
+        G.threads = field_threads(1, b->n_sm);
         launch_shared_chains(b->d_jobs + k, 1, G, stream);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(stream_wait(stream));
@@ -842,7 +846,7 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
   // (whose lattices are staged when every one of them fits).
   int max_optin = 0;
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-  b->max_optin = max_optin;
+  cudaDeviceGetAttribute(&b->n_sm, cudaDevAttrMultiProcessorCount, b->device);
   uint32_t need_smem = 0, need_gmem = 0;
   int n_rest = 0;  // chains the shared-memory kernels do not take
   bool rest_fits = true;
@@ -908,18 +912,16 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
   }
   {
     // many chains: the gather kernel keeps more of them on an SM
-    int n_sm = 0;
-    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, b->device);
     double load = 0.0;
     for (int c = 0; c < n_chains; ++c)
       if (b->kernel[c] == kSharedField) load += field_load(b->field_smem[c]);
-    if (!fields_pay(load, n_sm))
+    if (!fields_pay(load, b->n_sm))
       for (int c = 0; c < n_chains; ++c)
         if (b->halo[c]) b->kernel[c] = kSharedGather;
     const uint32_t room = layout_room(max_optin, kRoundsOwn);
     b->rest_nibbles = rest_bytes > room;
     b->rest_smem = b->rest_nibbles ? rest_nibbles : rest_bytes;
-    b->rest_rounds = n_rest > 0 && rest_fits && b->rest_smem <= room && rounds_pay(n_rest, n_sm);
+    b->rest_rounds = n_rest > 0 && rest_fits && b->rest_smem <= room && rounds_pay(n_rest, b->n_sm);
   }
   b->smem_lat = need_smem <= layout_room(max_optin, kOneWarpOwn);
   b->smem_bytes = b->smem_lat ? need_smem : need_gmem;

@@ -487,18 +487,4 @@ __device__ __forceinline__ void field_produce(const ChainJob& J, const Geom& g, 
   });
 }
 
-// Threads per chain: eight warps run the trials; the others share the staging and
-// the fields' first sums.  Chains that have an SM to themselves take 16 warps
-// (four on each scheduler).
-inline int field_threads(int n_jobs) {
-  static int n_sm = 0;
-  if (n_sm == 0) {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    n_sm = n;
-  }
-  return n_jobs <= n_sm ? 512 : 256;
-}
-
 }  // namespace brawl

@@ -178,6 +178,12 @@ enum shared_kernel : int {
 inline double field_load(uint32_t smem) { return 2u * (smem + 1024u) <= 228u * 1024u ? 0.5 : 1.0; }
 inline bool fields_pay(double load, int n_sm) { return load <= n_sm; }
 
+// Threads per chain with fields: eight warps run the trials; the others share the
+// staging and the fields' first sums.  Where the chains that run at once (of all
+// launches) have an SM each they take 16 warps, four on each scheduler; at 113
+// registers a block of 16 would leave a second chain no place on its SM.
+inline int field_threads(int n_chains, int n_sm) { return n_chains <= n_sm ? 512 : 256; }
+
 // Wang-Landau walkers with fields (wl_field.cu: one to an SM, its registers fill
 // one) beside wl_sweep_kernel's, of which two share an SM: all while each has an
 // SM to itself; in more waves only with 40 neighbours or more, whose gathering
@@ -216,6 +222,7 @@ inline int gather_trials(double beta_spread) { return beta_spread < 0.95 ? 1 : b
 // round of the gather kernel.
 struct LaunchGroup {
   int kernel = kSharedNone, depth = kGatherDefault, first = -1, count = 0;
+  int threads = 0;   // per chain with fields (field_threads)
   uint32_t smem = 0;
   int max_z = 0;
   int ns = 0;        // species of one of them (field kernel: all are of its field_variant)
@@ -223,11 +230,11 @@ struct LaunchGroup {
 };
 void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int depth,
                             cudaStream_t stream);
-void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int ns,
+void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, int threads, uint32_t smem_bytes, int max_z, int ns,
                              cudaStream_t stream);
 inline void launch_shared_chains(const ChainJob* d_jobs, int n_jobs, const LaunchGroup& G, cudaStream_t stream) {
   if (G.kernel == kSharedField)
-    launch_metropolis_field(d_jobs, n_jobs, G.smem, G.max_z, G.ns, stream);
+    launch_metropolis_field(d_jobs, n_jobs, G.threads, G.smem, G.max_z, G.ns, stream);
   else
     launch_metropolis_halo(d_jobs, n_jobs, G.smem, G.max_z, G.depth, stream);
 }

@@ -219,30 +219,30 @@ __global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob
 }
 
 template <int NJ, int R>
-static void launch_field_r(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, cudaStream_t stream) {
+static void launch_field_r(const ChainJob* d_jobs, int n_jobs, int threads, uint32_t smem_bytes, cudaStream_t stream) {
   cudaFuncSetAttribute(metropolis_field_kernel<NJ, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
   BRAWL_CARVEOUT(metropolis_field_kernel<NJ, R>);
-  metropolis_field_kernel<NJ, R><<<n_jobs, field_threads(n_jobs), smem_bytes, stream>>>(d_jobs);
+  metropolis_field_kernel<NJ, R><<<n_jobs, threads, smem_bytes, stream>>>(d_jobs);
 }
 
 template <int NJ>
-static void launch_field_nj(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int ns, cudaStream_t stream) {
+static void launch_field_nj(const ChainJob* d_jobs, int n_jobs, int threads, uint32_t smem_bytes, int ns, cudaStream_t stream) {
   switch (field_variant(ns)) {
-    case 1: launch_field_r<NJ, 1>(d_jobs, n_jobs, smem_bytes, stream); break;
-    case 2: launch_field_r<NJ, 2>(d_jobs, n_jobs, smem_bytes, stream); break;
-    case 4: launch_field_r<NJ, 4>(d_jobs, n_jobs, smem_bytes, stream); break;
-    default: launch_field_r<NJ, 0>(d_jobs, n_jobs, smem_bytes, stream); break;
+    case 1: launch_field_r<NJ, 1>(d_jobs, n_jobs, threads, smem_bytes, stream); break;
+    case 2: launch_field_r<NJ, 2>(d_jobs, n_jobs, threads, smem_bytes, stream); break;
+    case 4: launch_field_r<NJ, 4>(d_jobs, n_jobs, threads, smem_bytes, stream); break;
+    default: launch_field_r<NJ, 0>(d_jobs, n_jobs, threads, smem_bytes, stream); break;
   }
 }
 
 // The chains are of ns's variant (field_variant), their neighbour counts up to
 // max_z.
-void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, int max_z, int ns,
+void launch_metropolis_field(const ChainJob* d_jobs, int n_jobs, int threads, uint32_t smem_bytes, int max_z, int ns,
                              cudaStream_t stream) {
   if (n_jobs <= 0) return;
-  if (max_z <= kFieldHalf) launch_field_nj<1>(d_jobs, n_jobs, smem_bytes, ns, stream);
-  else if (max_z <= 2 * kFieldHalf) launch_field_nj<2>(d_jobs, n_jobs, smem_bytes, ns, stream);
-  else launch_field_nj<3>(d_jobs, n_jobs, smem_bytes, ns, stream);
+  if (max_z <= kFieldHalf) launch_field_nj<1>(d_jobs, n_jobs, threads, smem_bytes, ns, stream);
+  else if (max_z <= 2 * kFieldHalf) launch_field_nj<2>(d_jobs, n_jobs, threads, smem_bytes, ns, stream);
+  else launch_field_nj<3>(d_jobs, n_jobs, threads, smem_bytes, ns, stream);
 }
 
 template <int NJ>

@@ -667,8 +667,12 @@ int launch_anneal(brawl_server* S, Pipe& P) {
   SV_TRY(grow(P.d_tns, P.tns_cap, std::max<size_t>(P.jobs.size(), 1), P.s));
   const double t_round = round_ns(S, P.jobs);
   double load = 0.0;
-  for (const auto& j : P.jobs)
-    if (j->slot.kernel == kSharedField) load += field_load(j->slot.field_smem);
+  int n_fields = 0;
+  for (const auto& j : P.jobs) {
+    if (j->slot.kernel != kSharedField) continue;
+    load += field_load(j->slot.field_smem);
+    n_fields += 1;
+  }
   const bool fields = fields_pay(load, S->n_sm);
   std::stable_sort(P.jobs.begin(), P.jobs.end(), [fields](const JobP& a, const JobP& b) {
     const int ka = round_kind(a->slot, fields), kb = round_kind(b->slot, fields);
@@ -712,6 +716,7 @@ int launch_anneal(brawl_server* S, Pipe& P) {
       LaunchGroup G;
       G.kernel = round_kernel(P.launched[first]->slot, fields);
       G.ns = staged[first].g.ns;
+      G.threads = field_threads(n_fields, S->n_sm);
       G.smem = sm[first];
       for (int k = first; k < first + count; ++k) G.max_z = std::max(G.max_z, (int)staged[k].g.z);
       launch_shared_chains(P.d_chain + first, count, G, st);
