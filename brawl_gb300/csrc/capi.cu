@@ -2349,7 +2349,6 @@ struct brawl_wl {
   bool fields = false;
   uint32_t field_smem = 0;
   int variant = 0;
-  int min_z = 0;  // the fewest neighbours of a walker's sites
   // radial-density samples (brawl_wl_radial_enable)
   int rad_wc = 0, rad_n_off = 0, rad_n_class = 0;
   WlRadial* d_rad = nullptr;
@@ -2411,13 +2410,11 @@ static void wl_plan_fields(brawl_wl* wl) {
   int max_optin = 0;
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, wl->b->device);
   wl->fields = wl->d_rad == nullptr;
-  wl->min_z = wl->w.empty() ? 0 : (int)wl->w[0].job.g.z;
   wl->field_smem = 0;
   wl->variant = field_variant(wl->w[0].job.g.ns);
   for (WlWalker& W : wl->w) {
     const Geom& g = W.job.g;
     const int nb = W.end - W.start + 1;
-    wl->min_z = std::min(wl->min_z, (int)g.z);
     W.field_cap = 0;
     if (W.job.fg.n_class > 0 && W.job.fg.symmetric)
       W.field_cap = lazy_cap_for(g, wl_field_smem_bytes(g, W.job.fg, nb, 0), layout_room(max_optin, kWlFieldOwn));
@@ -2551,7 +2548,7 @@ extern "C" int brawl_wl_sweeps(brawl_wl* wl, int64_t n_trials, double wl_f, int 
   CUDA_TRY(cudaMemcpyAsync(wl->d_w, wl->w.data(), n * sizeof(WlWalker), cudaMemcpyHostToDevice, b->stream));
   int n_sm = 0;
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, wl->b->device);
-  if (wl->fields && wl_fields_pay((int)wl->w.size(), wl->min_z, n_sm))
+  if (wl->fields && wl_fields_pay((int)wl->w.size(), n_sm))
     launch_wl_field(wl->d_w, n, wl->field_smem, wl->max_z, wl->variant, b->stream);
   else
     launch_wl_sweeps(wl->d_w, n, wl->smem, wl->max_z, wl->all_D, b->stream);
@@ -3096,7 +3093,7 @@ int api_batch_set_rng(brawl_batch* b, int c, const uint32_t state[625]) {
 cudaStream_t api_batch_stream(brawl_batch* b) { return b->stream; }
 brawl_batch* api_wl_batch(brawl_wl* wl) { return wl->b; }
 std::vector<WlWalker>& api_wl_walkers(brawl_wl* wl) { return wl->w; }
-bool wl_fields(const brawl_wl* wl, int n, int n_sm) { return wl->fields && wl_fields_pay(n, wl->min_z, n_sm); }
+bool wl_fields(const brawl_wl* wl, int n, int n_sm) { return wl->fields && wl_fields_pay(n, n_sm); }
 uint32_t api_wl_smem(brawl_wl* wl, int n, int n_sm) { return wl_fields(wl, n, n_sm) ? wl->field_smem : wl->smem; }
 int api_wl_kind(brawl_wl* wl, int n, int n_sm) { return wl_fields(wl, n, n_sm) ? 8 + wl->variant : 0; }
 void api_wl_variant(brawl_wl* wl, int* max_z, bool* all_D) {

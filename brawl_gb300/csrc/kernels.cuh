@@ -185,14 +185,13 @@ inline bool fields_pay(double load, int n_sm) { return load <= n_sm; }
 inline int field_threads(int n_chains, int n_sm) { return n_chains <= n_sm ? 512 : 256; }
 
 // Wang-Landau walkers with fields (wl_field.cu: one to an SM, its registers fill
-// one) beside wl_sweep_kernel's, of which two share an SM: all while each has an
-// SM to itself; in more waves only with 40 neighbours or more, whose gathering
-// the fields save.  3,000 trials of 304 walkers, a third to nearly all of them
-// accepted, fields and sweeps: bcc with 14 neighbours 3.8-4.2 and 3.0-3.2 ms,
-// with 26 3.8-4.0 and 3.2-3.3, with 50 1.7-2.5 and 3.1-3.4, with 64 1.9-2.7 and
-// 3.2-3.8; 608 walkers: 6.2-7.9 and 5.8-6.0, 5.7 and 5.9, 3.3-4.9 and 6.0-6.3,
-// 3.3-4.8 and 6.1-7.0.
-inline bool wl_fields_pay(int n_walkers, int min_z, int n_sm) { return n_walkers <= n_sm || min_z >= 40; }
+// one) beside wl_sweep_kernel's, of which two share an SM: while each has an SM to
+// itself.  3,000 trials of 152 walkers, fields and sweeps: bcc 6^3 with 8
+// neighbours 2.1-2.4 and 2.6-2.9 ms, 8^3 with 50 (nearly all accepted) 3.2-3.5 and
+// 3.6, 12^3 with 64 2.7-3.5 and 3.5-3.9, fcc 9^3 with 78 1.4-3.3 and 3.3-4.2.  In a
+// second wave it would depend on the acceptance, which is not known beforehand: 304
+// walkers 6.3-6.8 and 3.7, 5.1-6.8 and 3.6-4.0, 2.5-6.4 and 3.4-4.3.
+inline bool wl_fields_pay(int n_walkers, int n_sm) { return n_walkers <= n_sm; }
 
 // Chains in rounds of trials (metropolis_rounds.cu) where each has an SM to itself
 // (its sixteen warps' registers fill one): 152 chains take as long as one, 0.74 ms
