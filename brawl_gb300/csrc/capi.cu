@@ -486,6 +486,7 @@ struct brawl_batch {
   // Chains run in shared memory: per chain the kernel it takes by default
   // (shared_kernel), whether the gather kernel can take it, and what each needs.
   std::vector<int> kernel, halo;
+  bool crowded = false;                  // more chains could run with fields than there are SMs
   std::vector<uint32_t> gather_smem, field_smem;
   std::vector<ChainJob> staged;          // jobs in launch order
   int n_shared = 0;                      // of them in shared memory (first)
@@ -564,14 +565,22 @@ int ensure_grid(brawl_batch* b, size_t bytes) {
   return BRAWL_OK;
 }
 
-// The kernel that chain c takes at `depth` trials per round.
-int chain_kernel(const brawl_batch* b, int c, int depth) {
+// The kernel that the chains of c's class take at `depth` trials per round.
+int class_kernel(const brawl_batch* b, int c, int depth) {
   return depth >= 2 && b->halo[c] ? kSharedGather : b->kernel[c];
+}
+
+// The kernel that chain c takes in a batch whose classes have no depths of their own.
+int chain_kernel(const brawl_batch* b, int c) {
+  const int k = class_kernel(b, c, b->spec_nc);
+  if (k != kSharedField || !b->halo[c] || !b->crowded) return k;
+  const Model& m = b->models[c];
+  return too_hot_for_fields(b->jobs[c].beta * m.spread, m.g.z, m.g.n_sites) ? (int)kSharedGather : k;
 }
 
 // The trials of a gathered round of chain c, unless the caller chose.
 int gather_depth(const brawl_batch* b, int c) {
-  return b->spec_nc == 1 ? gather_trials(b->jobs[c].beta * b->models[c].spread) : b->spec_nc;
+  return b->spec_nc == 1 ? gather_trials(b->jobs[c].beta * b->models[c].spread, b->models[c].g.ns) : b->spec_nc;
 }
 
 // Jobs go to the device in launch order: the shared-memory chains first, group
@@ -599,33 +608,33 @@ int upload_jobs(brawl_batch* b) {
     for (int c = 0; c < n; ++c) {
       const int k = b->cls[c];
       if (k < 0) continue;
-      gs[k].kernel = chain_kernel(b, c, b->class_depth[k]);
+      gs[k].kernel = class_kernel(b, c, b->class_depth[k]);
       gs[k].depth = b->class_depth[k] == 1 ? kGatherDefault : b->class_depth[k];
       add(c, k);
     }
   } else {
-    std::vector<int> by;
-    for (int c = 0; c < n; ++c)
-      if (b->kernel[c] != kSharedNone) by.push_back(c);
-    auto need = [&](int c) {
-      return chain_kernel(b, c, b->spec_nc) == kSharedField ? b->field_smem[c] : b->gather_smem[c];
-    };
+    std::vector<int> by, kernel(n, kSharedNone);
+    for (int c = 0; c < n; ++c) {
+      if (b->kernel[c] == kSharedNone) continue;
+      by.push_back(c);
+      kernel[c] = chain_kernel(b, c);
+    }
+    auto need = [&](int c) { return kernel[c] == kSharedField ? b->field_smem[c] : b->gather_smem[c]; };
     // the unrolling, and with fields their number per site
     auto variant = [&](int c) {
       const Geom& g = b->models[c].g;
-      return chain_kernel(b, c, b->spec_nc) == kSharedField ? 16 * ((g.z + kFieldHalf - 1) / kFieldHalf) + field_variant(g.ns)
-                                                           : 8 * lane_entries_for(g.z) + gather_depth(b, c);
+      return kernel[c] == kSharedField ? 16 * ((g.z + kFieldHalf - 1) / kFieldHalf) + field_variant(g.ns)
+                                       : 8 * lane_entries_for(g.z) + gather_depth(b, c);
     };
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
-      const int kx = chain_kernel(b, x, b->spec_nc), ky = chain_kernel(b, y, b->spec_nc);
-      if (kx != ky) return kx > ky;
+      if (kernel[x] != kernel[y]) return kernel[x] > kernel[y];
       const int vx = variant(x), vy = variant(y);
       if (vx != vy) return vx > vy;
       return need(x) > need(y);
     });
     int nj = 0;
     for (int c : by) {
-      const int k = chain_kernel(b, c, b->spec_nc), z = variant(c);
+      const int k = kernel[c], z = variant(c);
       if (gs.empty() || gs.back().kernel != k || nj != z || 3ull * need(c) < 2ull * gs.back().smem) {
         gs.push_back(LaunchGroup());
         gs.back().kernel = k;
@@ -913,8 +922,13 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
   {
     // many chains: the gather kernel keeps more of them on an SM
     double load = 0.0;
-    for (int c = 0; c < n_chains; ++c)
-      if (b->kernel[c] == kSharedField) load += field_load(b->field_smem[c]);
+    int n_fields = 0;
+    for (int c = 0; c < n_chains; ++c) {
+      if (b->kernel[c] != kSharedField) continue;
+      load += field_load(b->field_smem[c]);
+      n_fields += 1;
+    }
+    b->crowded = n_fields > b->n_sm;
     if (!fields_pay(load, b->n_sm))
       for (int c = 0; c < n_chains; ++c)
         if (b->halo[c]) b->kernel[c] = kSharedGather;

@@ -178,6 +178,18 @@ enum shared_kernel : int {
 inline double field_load(uint32_t smem) { return 2u * (smem + 1024u) <= 228u * 1024u ? 0.5 : 1.0; }
 inline bool fields_pay(double load, int n_sm) { return load <= n_sm; }
 
+// Of two chains on an SM a very hot one (beta_spread as for gather_trials) gathers,
+// as it accepts most swaps, unless the sites around a swapped one are so much of its
+// lattice that the gather kernel's next trials mostly wait for it.  5,000 trials of
+// 300 chains at 0.1, with fields and gathered (ms): bcc 14^3, five species, two shells
+// 3.10 and 2.69, bcc 16^3, three and three 2.77 and 2.49, fcc 10^3, four and six 3.40
+// and 3.01; at 0.45 2.80 and 2.64, 2.58 and 2.49, 3.11 and 2.92; at 0.8 2.51 and 2.57,
+// 2.40 and 2.42, 2.75 and 2.84.  bcc 6^3 with 64 neighbours of 432 sites at 0.1: 2.31
+// and 2.83.  One chain on an SM: within 5% of each other at 0.1.
+inline bool too_hot_for_fields(double beta_spread, int z, int n_sites) {
+  return beta_spread < 0.4 && 16 * z <= n_sites;
+}
+
 // Threads per chain with fields: eight warps run the trials; the others share the
 // staging and the fields' first sums.  Where the chains that run at once (of all
 // launches) have an SM each they take 16 warps, four on each scheduler; at 113
@@ -205,16 +217,20 @@ void launch_metropolis_rounds(const ChainJob* d_jobs, int n_jobs, bool nibbles, 
 
 // Trials per round of the gather kernel, by how hot the chain is: its inverse
 // temperature times the spread of its swaps' energy changes.  The hotter, the
-// fewer trials a round keeps.  Rounds of one, two and three, a first call from
-// random configurations / later ones (ms): 600 chains of bcc 10^3, two species, six
-// shells at 0.9: 2.08/2.01, 2.28/2.17 and 2.46/2.38, at 1.3: 1.98/1.92, 2.07/1.97
-// and 2.25/2.10; 563 of bcc 22^3, four shells at 0.8: 7.2/7.0, 7.4/7.2 and 7.7/7.4,
-// at 1.2: 7.0/6.7, 7.0/6.4 and 7.1/6.4, at 1.9: 6.8/6.0, 6.5/5.3 and 6.5/5.0; 400 of
-// bcc 14^3, five species, two shells at 1.0: 2.50/2.37, 2.35/2.13 and 2.50/2.21.
-// Four lose to three from random configurations (256 of bcc 24^3 at 600 K: 5.9/4.0
-// and 5.7/4.1).
+// fewer trials a round keeps.  5,000 trials in rounds of one, two and three, a first
+// call from random configurations / later ones (ms): 400 chains of bcc 14^3, five
+// species, two shells at 0.95: 1.95/1.90, 2.17/2.02 and 2.32/2.15, at 1.3: 1.94/1.84,
+// 2.07/1.83 and 2.21/1.86, at 1.5: 1.91/1.80, 2.03/1.74 and 2.13/1.75, at 2:
+// 1.90/1.76, 1.96/1.63 and 2.07/1.55; of bcc 24^3, four species, six shells at 1.3:
+// 2.31/2.15, 2.56/2.24 and 2.59/2.25, at 2: 2.28/2.09, 2.46/2.06 and 2.47/2.01; of
+// fcc 10^3 alike at 1.3: 2.21/2.05, 2.54/2.03 and 2.76/2.09.  Two species order
+// earlier: 600 chains of bcc 10^3, six shells at 0.7: 1.78/1.68, 2.07/1.68 and
+// 2.27/1.75, at 0.95: 1.74/1.57, 1.93/1.46 and 2.07/1.43.  Four lose to three from
+// random configurations (256 of bcc 24^3 at 600 K: 5.9/4.0 and 5.7/4.1).
 constexpr int kGatherDefault = 3;
-inline int gather_trials(double beta_spread) { return beta_spread < 0.95 ? 1 : beta_spread < 1.5 ? 2 : kGatherDefault; }
+inline int gather_trials(double beta_spread, int ns) {
+  return beta_spread < (ns == 2 ? 0.95 : 1.4) ? 1 : beta_spread < 1.5 ? 2 : kGatherDefault;
+}
 
 // One launch of them: `count` chains from `first` in launch order, the largest
 // shared memory and neighbour count among them, and the trials per

@@ -31,6 +31,29 @@ def test_mixed_sizes_match_oracle():
         assert acc[k] == a and np.array_equal(b.config(k), cfg), k
 
 
+@pytest.mark.parametrize("chains", [150, 200])
+def test_very_hot_chains_beside_cool_ones_match_oracle(chains):
+    """One and two chains to an SM, every second one at an infinite temperature
+    (which gather their sums where two share an SM), in calls at two temperatures
+    and with classes of their own."""
+    V = random_V(np.random.default_rng(4), 3, 2)
+    T = np.where(np.arange(chains) % 2, 400.0, 1.0e7)
+    mod = O.OracleModel("bcc", 5, 5, 5, V)
+    b = B.Batch([dict(setup=B.Setup("bcc", 5, 5, 5, 3, 2), V=V, seed=90 + k, beta=1.0 / (T[k] * B.K_B_IN_RY),
+                      nbr_swap=k % 3 == 0, species_concentrations=conc_vector(3)) for k in range(chains)])
+    acc = b.metropolis(400)
+    b.set_beta(1.0 / (T[::-1] * B.K_B_IN_RY))
+    acc = acc + b.metropolis(401)
+    b.set_class_depths([1])
+    acc = acc + b.metropolis(402)
+    for k in (0, 1, 2, 3, chains - 2, chains - 1):
+        r = O.OracleRng(90 + k)
+        cfg, _ = mod.initial_setup(r, conc_vector(3))
+        a = sum(mod.mc_run(cfg, r, 1.0 / (t * B.K_B_IN_RY), n, k % 3 == 0)[0]
+                for t, n in ((T[k], 400), (T[::-1][k], 401), (T[::-1][k], 402)))
+        assert acc[k] == a and np.array_equal(b.config(k), cfg), k
+
+
 def test_two_chains_to_an_sm_run_at_once():
     """300 chains take little longer than 150 (1.2 times, measured); in two waves
     they took 1.8 times as long."""
