@@ -480,6 +480,7 @@ struct brawl_batch {
   // (metropolis_rounds.cu), their lattices as half bytes, its shared memory
   bool rest_rounds = false, rest_nibbles = false;
   uint32_t rest_smem = 0;
+  int rest_sites = 0;  // of the largest
   bool smem_lat = true;
   bool use_D = true;
   int max_z = 0;
@@ -573,14 +574,21 @@ int class_kernel(const brawl_batch* b, int c, int depth) {
 // The kernel that chain c takes in a batch whose classes have no depths of their own.
 int chain_kernel(const brawl_batch* b, int c) {
   const int k = class_kernel(b, c, b->spec_nc);
-  if (k != kSharedField || !b->halo[c] || !b->crowded) return k;
+  if (k != kSharedField || !b->halo[c]) return k;
   const Model& m = b->models[c];
-  return too_hot_for_fields(b->jobs[c].beta * m.spread, m.g.z, m.g.n_sites) ? (int)kSharedGather : k;
+  if (b->crowded && too_hot_for_fields(b->jobs[c].beta * m.spread, m.g.z, m.g.n_sites)) return kSharedGather;
+  return k;
 }
 
 // The trials of a gathered round of chain c, unless the caller chose.
 int gather_depth(const brawl_batch* b, int c) {
   return b->spec_nc == 1 ? gather_trials(b->jobs[c].beta * b->models[c].spread, b->models[c].g.ns) : b->spec_nc;
+}
+
+// (a batch of one kind is in order: one pass instead of n log n on every call)
+template <class Less>
+void sort_unless_sorted(std::vector<int>& v, Less less) {
+  if (!std::is_sorted(v.begin(), v.end(), less)) std::stable_sort(v.begin(), v.end(), less);
 }
 
 // Jobs go to the device in launch order: the shared-memory chains first, group
@@ -619,23 +627,24 @@ int upload_jobs(brawl_batch* b) {
       by.push_back(c);
       kernel[c] = chain_kernel(b, c);
     }
-    auto need = [&](int c) { return kernel[c] == kSharedField ? b->field_smem[c] : b->gather_smem[c]; };
-    // the unrolling, and with fields their number per site
-    auto variant = [&](int c) {
+    // kernel; the unrolling, and with fields their number per site, gathered the
+    // depth; shared memory
+    std::vector<int> variant(n, 0);
+    std::vector<uint32_t> need(n, 0);
+    std::vector<uint64_t> key(n, 0);
+    for (int c : by) {
       const Geom& g = b->models[c].g;
-      return kernel[c] == kSharedField ? 16 * ((g.z + kFieldHalf - 1) / kFieldHalf) + field_variant(g.ns)
-                                       : 8 * lane_entries_for(g.z) + gather_depth(b, c);
-    };
-    std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
-      if (kernel[x] != kernel[y]) return kernel[x] > kernel[y];
-      const int vx = variant(x), vy = variant(y);
-      if (vx != vy) return vx > vy;
-      return need(x) > need(y);
-    });
+      const bool field = kernel[c] == kSharedField;
+      variant[c] = field ? 16 * ((g.z + kFieldHalf - 1) / kFieldHalf) + field_variant(g.ns)
+                         : 8 * lane_entries_for(g.z) + gather_depth(b, c);
+      need[c] = field ? b->field_smem[c] : b->gather_smem[c];
+      key[c] = (uint64_t)kernel[c] << 56 | (uint64_t)variant[c] << 32 | need[c];
+    }
+    sort_unless_sorted(by, [&](int x, int y) { return key[x] > key[y]; });
     int nj = 0;
     for (int c : by) {
-      const int k = kernel[c], z = variant(c);
-      if (gs.empty() || gs.back().kernel != k || nj != z || 3ull * need(c) < 2ull * gs.back().smem) {
+      const int k = kernel[c], z = variant[c];
+      if (gs.empty() || gs.back().kernel != k || nj != z || 3ull * need[c] < 2ull * gs.back().smem) {
         gs.push_back(LaunchGroup());
         gs.back().kernel = k;
         gs.back().depth = gather_depth(b, c);
@@ -653,7 +662,7 @@ int upload_jobs(brawl_batch* b) {
   for (size_t r = 0; r < at.size(); ++r) rank[at[r]] = (int)r;
   std::vector<int> order(n);
   for (int c = 0; c < n; ++c) order[c] = c;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+  sort_unless_sorted(order, [&](int x, int y) {
     if ((gid[x] < 0) != (gid[y] < 0)) return gid[x] >= 0;
     if (gid[x] >= 0 && gid[x] != gid[y]) return rank[gid[x]] < rank[gid[y]];
     return b->jobs[x].n_trials > b->jobs[y].n_trials;
@@ -761,17 +770,17 @@ int run_metropolis(brawl_batch* b, const int64_t* n_trials, int64_t* accepted, b
   return BRAWL_OK;
 }
 
-// Every chain's uploaded job (b->d_jobs) once on `stream`: the shared-memory
-// chains' launches, the others in one launch of the plain kernel.
 // Chains first .. first + n - 1 of the launch order, which no shared-memory group
-// takes.
+// takes, the longest first.
 void launch_rest(brawl_batch* b, int first, int n, cudaStream_t stream) {
-  if (b->rest_rounds)
+  if (b->rest_rounds && (b->smem_lat || nibbles_paid(b->staged[first].n_trials, b->rest_sites)))
     launch_metropolis_rounds(b->d_jobs + first, n, b->rest_nibbles, b->rest_smem, b->max_z, stream);
   else
     launch_metropolis(b->d_jobs + first, n, b->smem_lat, b->use_D, b->smem_bytes, b->max_z, stream);
 }
 
+// Every chain's uploaded job (b->d_jobs) once on `stream`: the shared-memory chains'
+// launches, and one of the others.
 int launch_sweep(brawl_batch* b, cudaStream_t stream) {
   const int n = (int)b->jobs.size();
   if (n > b->n_shared) launch_rest(b, b->n_shared, n - b->n_shared, stream);
@@ -911,6 +920,7 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     b->cls[c] = kind_class[k];
     if (b->kernel[c] != kSharedNone) continue;
     n_rest += 1;
+    b->rest_sites = std::max(b->rest_sites, m.g.n_sites);
     rest_fits = rest_fits && m.g.n1 <= 512 && m.g.n2 <= 512 && m.g.n3 <= 512 && !meets_itself(m.g);
     rest_bytes = std::max(rest_bytes, round_smem_bytes(m.g, false));
     rest_nibbles = std::max(rest_nibbles, round_smem_bytes(m.g, true));

@@ -211,6 +211,10 @@ inline bool wl_fields_pay(int n_walkers, int n_sm) { return n_walkers <= n_sm; }
 // twice that, where metropolis_kernel, a warp a chain, takes 2.7 and 1.75 for
 // either.
 inline bool rounds_pay(int n_chains, int n_sm) { return n_chains <= n_sm; }
+// And whether the longest of them pays for half bytes in shared memory, where
+// metropolis_kernel leaves the lattice in global memory: 1, 10 and 100 trials of eight
+// chains of fcc 40^3 take 74, 76 and 98 us so, and 52, 59 and 123 there.
+inline bool nibbles_paid(int64_t n_trials, int n_sites) { return n_trials >= 8 + n_sites / 4096; }
 uint32_t round_smem_bytes(const Geom& g, bool nibbles);
 void launch_metropolis_rounds(const ChainJob* d_jobs, int n_jobs, bool nibbles, uint32_t smem_bytes, int max_z,
                               cudaStream_t stream);

@@ -177,8 +177,11 @@ __global__ void __launch_bounds__(32, kSpec == 1 || NJ == 2 ? 16 : 0) metropolis
     // the lane entries past z)
     int32_t* D = reinterpret_cast<int32_t*>(smem + L.D);
     const int per = g.nsh * nsp, all = L.Dk / 4;
-    for (int p = 0; p < nsp * nsp; ++p)
-      for (int i = lane; i < all; i += 32) D[p * all + i] = i < per ? Jg->F[nF + p * per + i] : 0;
+#pragma unroll 4
+    for (int i = lane; i < nsp * nsp * all; i += 32) {
+      const int p = i / all, r = i - p * all;
+      D[i] = r < per ? Jg->F[nF + p * per + r] : 0;
+    }
   }
   for (int i = lane; i < nV; i += 32) V[i] = Jg->V[i];
   for (int i = lane; i <= g.nsh; i += 32) sstart[i] = Jg->shell_start[i];

@@ -224,3 +224,23 @@ def test_many_chains_match_oracle(T):
         assert acc[k] == a and np.array_equal(b.config(k), cfg), k
         if k % 40 == 0:
             assert _same_stream(b.rng_state(k), r), k
+
+
+@pytest.mark.parametrize("case", [
+    ("fcc", (40, 40, 40), 4, 4, False, 70),   # rounds of trials from 70 trials on
+    ("bcc", (47, 47, 51), 3, 2, True, 63),    # from 63
+], ids=lambda c: f"{c[0]}-{c[1]}-s{c[2]}-sh{c[3]}")
+def test_calls_of_few_and_many_trials_match_oracle(case):
+    """Calls on both sides of the line up to which a lattice of half bytes does not
+    pay, in turn on the same chain."""
+    lattice, n, ns, nsh, nbr, line = case
+    V, mod, r, cfg = _chain(case[:5], ns)
+    beta = 1.0 / (1200.0 * B.K_B_IN_RY)
+    b = B.Batch([dict(setup=B.Setup(lattice, *n, ns, nsh), V=V, seed=7000 + ns, beta=beta, nbr_swap=nbr,
+                      species_concentrations=conc_vector(ns))])
+    for trials in (1, line - 1, 200, line, line + 1, 0, 2, 300):
+        acc = b.metropolis(trials)
+        a, _ = mod.mc_run(cfg, r, beta, trials, nbr)
+        assert acc[0] == a, trials
+        assert np.array_equal(b.config(0), cfg), trials
+        assert _same_stream(b.rng_state(0), r), trials
