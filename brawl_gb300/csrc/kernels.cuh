@@ -327,11 +327,15 @@ __host__ __device__ __forceinline__ bool inside_binade(long long b, long long e)
 // the first that leaves it (or lies halfway between two ulps) are done, and that
 // one is added by itself.  A sum that keeps leaving its binade (one that stays
 // near zero) is added up one by one for a while, longer each time.  256 chains
-// of up to 27,648 sites: 1.12 ms one by one, 0.19 ms so.
-__device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int n, int lane) {
+// of up to 27,648 sites: 1.12 ms one by one, 0.19 ms so.  Up to `few` terms are
+// added up one by one: a sum of one chain gains from 128 on, the longest of many
+// chains' from 512 (64 chains of 250 and of 432 sites, the whole call, 49 and 60 us
+// one by one and 57 and 69 so; of 864 82 and 70 to 83).
+constexpr int kFewTerms = 128, kFewTermsOfMany = 512;
+__device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int n, int lane, int few = kFewTerms) {
   constexpr int kTerms = 8;
   double energy = 0.0;
-  int base = 0, slow = n < 128 ? n : 32, run = 32;  // terms to add one by one; then how many
+  int base = 0, slow = n < few ? n : 32, run = 32;  // terms to add one by one; then how many
   while (base < n) {
     if (slow > 0) {
       // 32 at a time, the next 32 already in flight

@@ -68,7 +68,8 @@ __global__ void __launch_bounds__(32 * kSumWarps) sum_sites_kernel(const EnergyJ
   const int c = blockIdx.x * kSumWarps + (threadIdx.x >> 5);
   if (c >= n_jobs) return;  // the whole warp
   const EnergyJob& J = jobs[c];
-  const double energy = ordered_half_sum_warp(J.site_energy, J.g.n_sites, lane);
+  const int few = n_jobs < 8 ? kFewTerms : kFewTermsOfMany;
+  const double energy = ordered_half_sum_warp(J.site_energy, J.g.n_sites, lane, few);
   if (lane == 0) *J.out = energy;
 }
 

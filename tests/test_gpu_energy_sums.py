@@ -54,3 +54,19 @@ def test_pair_counts_at_the_edges_match_oracle(lattice, n, ns, wc):
     shells = ch.lattice_shells(wc)
     rho, _ = mod.radial_densities(ch.config(), shells)
     assert np.array_equal(np.asarray(ch.radial_densities(shells)), rho, equal_nan=True)
+
+
+@pytest.mark.parametrize("chains", [7, 8])
+def test_energies_of_few_and_many_chains_match_oracle(chains):
+    """Sums of 128 to 512 terms, which few chains take 256 at a time and many one
+    by one, and one term more."""
+    rng = np.random.default_rng(6)
+    for lattice, n, ns, nsh in [("bcc", (4, 4, 4), 3, 2), ("bcc", (5, 5, 5), 3, 4), ("fcc", (8, 4, 4), 4, 3),
+                                ("bcc", (19, 3, 9), 2, 2)]:
+        V = random_V(rng, ns, nsh)
+        mod = O.OracleModel(lattice, *n, V)
+        b = B.Batch([dict(setup=B.Setup(lattice, *n, ns, nsh), V=V, seed=60 + k, beta=1.0,
+                          species_concentrations=conc_vector(ns)) for k in range(chains)])
+        E = b.total_energy()
+        for k in range(chains):
+            assert E[k] == mod.total_energy(b.config(k)), (lattice, n, k)
