@@ -294,21 +294,21 @@ __device__ inline double site_energy_ref(const Geom& g, const int8_t* lat, const
 // the binade rounds its term to a whole number of the binade's ulps, the same
 // whatever the sum, unless the term lies halfway between two.  That number for
 // term t (bits) and the binade of e (bits; a normal number), in the direction in
-// which e's bits grow; ok: not halfway, and not past what 63 bits hold.
-__host__ __device__ __forceinline__ long long ulps_of(long long t, long long e, bool& ok) {
+// which e's bits grow, modulo 2^64; ok: not halfway, and not past what 63 bits hold.
+__host__ __device__ __forceinline__ unsigned long long ulps_of(long long t, long long e, bool& ok) {
   const int et = (int)(t >> 52) & 0x7ff, s = ((int)(e >> 52) & 0x7ff) - (et > 0 ? et : 1);
-  const long long m = (t & 0xfffffffffffffll) | (et > 0 ? 1ll << 52 : 0ll);
-  long long k;
+  const unsigned long long m = (t & 0xfffffffffffffull) | (et > 0 ? 1ull << 52 : 0ull);
+  unsigned long long k;
   if (s <= 0) {
     ok = ok && s >= -8;
     k = m << (-s & 15);
   } else {
     const int r = s < 55 ? s : 55;  // (from 55 on it is under half an ulp)
-    const long long half = 1ll << (r - 1);
+    const unsigned long long half = 1ull << (r - 1);
     ok = ok && (m & (2 * half - 1)) != half;
     k = (m + half) >> r;
   }
-  return (t ^ e) < 0 ? -k : k;
+  return (t ^ e) < 0 ? 0ull - k : k;
 }
 
 // A value passed through: inside the binade of e, and not its first value (a sum
@@ -355,7 +355,7 @@ __device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int
     for (int j = 0; j < kTerms; ++j) v[j] = first + j < n ? e[first + j] : 0.0;
     const long long eb = __double_as_longlong(energy);
     const int ex = (int)(eb >> 52) & 0x7ff;
-    long long k[kTerms], sum = 0;
+    unsigned long long k[kTerms], sum = 0;  // (modulo 2^64: past a term that is not settled they may be anything)
     unsigned bad = ex > 60 && ex < 0x7ff ? 0u : 1u;  // bit j: term j is not settled
 #pragma unroll
     for (int j = 0; j < kTerms; ++j) {
@@ -364,18 +364,18 @@ __device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int
       sum += k[j];
       bad |= ok ? 0u : 1u << j;
     }
-    long long upto = sum;  // with the lanes before
+    unsigned long long upto = sum;  // with the lanes before
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long u = __shfl_up_sync(kFull, upto, o);
-      upto += lane >= o ? u : 0ll;
+      const unsigned long long u = __shfl_up_sync(kFull, upto, o);
+      upto += lane >= o ? u : 0ull;
     }
-    long long x = eb + upto - sum;
-    const long long x0 = x;
+    unsigned long long x = (unsigned long long)eb + upto - sum;
+    const unsigned long long x0 = x;
 #pragma unroll
     for (int j = 0; j < kTerms; ++j) {
       x += k[j];
-      bad |= inside_binade(x, eb) ? 0u : 1u << j;
+      bad |= inside_binade((long long)x, eb) ? 0u : 1u << j;
     }
     // the first term that is not settled
     const unsigned lanes = __ballot_sync(kFull, bad != 0);
@@ -386,10 +386,10 @@ __device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int
       const int j = __ffs(__shfl_sync(kFull, bad, l)) - 1;
       at = min(m, kTerms * l + j);
       // the sum before it, and it
-      long long before = x0;
+      unsigned long long before = x0;
 #pragma unroll
-      for (int i = 0; i < kTerms; ++i) before += i < j ? k[i] : 0ll;
-      energy = __longlong_as_double(__shfl_sync(kFull, before, l));
+      for (int i = 0; i < kTerms; ++i) before += i < j ? k[i] : 0ull;
+      energy = __longlong_as_double((long long)__shfl_sync(kFull, before, l));
       if (at < m) {
         energy = __dadd_rn(energy, e[base + at]);
         base += at + 1;
@@ -398,7 +398,7 @@ __device__ inline double ordered_half_sum_warp(const double* __restrict__ e, int
         continue;
       }
     } else {
-      energy = __longlong_as_double(__shfl_sync(kFull, x, 31));
+      energy = __longlong_as_double((long long)__shfl_sync(kFull, x, 31));
     }
     base += m;
     run = 32;

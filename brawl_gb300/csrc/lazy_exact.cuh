@@ -389,9 +389,10 @@ static __device__ __noinline__ double lazy_fold(LazyLog L, int n, double e, int 
       const long long b = __double_as_longlong(x);
       inside(b);
       ok = ok && (__double_as_longlong(off) & 0x7fffffffffffffffll) < half;
-      return b - eb;
+      return (unsigned long long)b - (unsigned long long)eb;
     };
-    long long r[2][2] = {{0, 0}, {0, 0}};
+    // (modulo 2^64: where one leaves the binade the sums may be anything)
+    unsigned long long r[2][2] = {{0, 0}, {0, 0}};
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int m = 2 * lane + k;
@@ -404,20 +405,21 @@ static __device__ __noinline__ double lazy_fold(LazyLog L, int n, double e, int 
         }
       }
     }
-    const long long first = r[0][0] + r[0][1], both = first + r[1][0] + r[1][1];
-    long long sum = both;  // with the lanes before
+    const unsigned long long first = r[0][0] + r[0][1], both = first + r[1][0] + r[1][1];
+    unsigned long long sum = both;  // with the lanes before
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long v = __shfl_up_sync(kFull, sum, o);
-      sum += lane >= o ? v : 0ll;
+      const unsigned long long v = __shfl_up_sync(kFull, sum, o);
+      sum += lane >= o ? v : 0ull;
     }
-    const long long x0 = eb + sum - both;
-    if (lane > 0) inside(x0);
-    inside(x0 + r[0][0]);
-    inside(x0 + first);
-    inside(x0 + first + r[1][0]);
-    inside(x0 + both);
-    if (__all_sync(kFull, ok)) return __longlong_as_double(eb + __shfl_sync(kFull, sum, 31));
+    const unsigned long long x0 = (unsigned long long)eb + sum - both;
+    if (lane > 0) inside((long long)x0);
+    inside((long long)(x0 + r[0][0]));
+    inside((long long)(x0 + first));
+    inside((long long)(x0 + first + r[1][0]));
+    inside((long long)(x0 + both));
+    if (__all_sync(kFull, ok))
+      return __longlong_as_double((long long)((unsigned long long)eb + __shfl_sync(kFull, sum, 31)));
   }
   if (fold == kFoldWangLandau) {
     // e = (e - pair_before) + pair_after, two dependent adds per move

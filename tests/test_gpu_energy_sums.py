@@ -70,3 +70,18 @@ def test_energies_of_few_and_many_chains_match_oracle(chains):
         E = b.total_energy()
         for k in range(chains):
             assert E[k] == mod.total_energy(b.config(k)), (lattice, n, k)
+
+
+@pytest.mark.parametrize("ratio", [2.0 ** 7, 2.0 ** 10, 2.0 ** 40, 1.0e200])
+def test_energies_of_terms_of_two_sizes_match_oracle(ratio):
+    """Some sites' energies so much larger than the others' that a sum of whole
+    ulps passes 2^63 behind the first of them."""
+    V = random_V(np.random.default_rng(8), 3, 2)
+    V[2, 2, :] *= ratio
+    mod = O.OracleModel("bcc", 8, 8, 8, V)
+    few = np.array([500, 520, 4], dtype=np.int64)
+    b = B.Batch([dict(setup=B.Setup("bcc", 8, 8, 8, 3, 2), V=V, seed=70 + k, beta=1.0,
+                      species_concentrations=conc_vector(3), species_numbers=few if k % 2 else None) for k in range(4)])
+    E = b.total_energy()
+    for k in range(4):
+        assert E[k] == mod.total_energy(b.config(k)), k
