@@ -391,13 +391,19 @@ __global__ void __launch_bounds__(kRoundThreads, 1) metropolis_rounds_kernel(con
   if (tid == 0 && J.t_ns) *J.t_ns = global_ns() - t_start;
 }
 
+template <int NJ, bool kNibbles>
+static void launch_rounds_lat(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, cudaStream_t stream) {
+  cudaFuncSetAttribute(metropolis_rounds_kernel<NJ, kNibbles>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem_bytes);
+  BRAWL_CARVEOUT((metropolis_rounds_kernel<NJ, kNibbles>));
+  metropolis_rounds_kernel<NJ, kNibbles><<<n_jobs, kRoundThreads, smem_bytes, stream>>>(d_jobs);
+}
+
 template <int NJ>
 static void launch_rounds_nj(const ChainJob* d_jobs, int n_jobs, bool nibbles, uint32_t smem_bytes,
                              cudaStream_t stream) {
-  auto* kernel = nibbles ? metropolis_rounds_kernel<NJ, true> : metropolis_rounds_kernel<NJ, false>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  BRAWL_CARVEOUT(kernel);
-  kernel<<<n_jobs, kRoundThreads, smem_bytes, stream>>>(d_jobs);
+  if (nibbles) launch_rounds_lat<NJ, true>(d_jobs, n_jobs, smem_bytes, stream);
+  else launch_rounds_lat<NJ, false>(d_jobs, n_jobs, smem_bytes, stream);
 }
 
 void launch_metropolis_rounds(const ChainJob* d_jobs, int n_jobs, bool nibbles, uint32_t smem_bytes, int max_z,
