@@ -1018,7 +1018,6 @@ int brawl_batch_create(const brawl_chain_desc* chains, int n_chains, brawl_batch
     {
       bool ok;
       make_halo(m.g, j.hg, ok);
-      j.halo = b->halo[c];
       if (tabs[c]) j.fg = tabs[c]->fg;
     }
     j.nbr_swap = b->nbr_swap[c];

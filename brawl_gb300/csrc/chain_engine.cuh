@@ -55,7 +55,6 @@ constexpr int kRingMirror = 96;
 constexpr int kDefaultSpeculation = 1;
 constexpr int kMTM = 397;
 constexpr int kMaxZ = 168;           // neighbour entries of bcc with 10 shells
-constexpr int kMaxLaneEntries = 11;  // ceil(2 * kMaxZ / 32)
 constexpr int kMaxSpecies = 15;      // species codes 1..15 (int8 storage)
 
 enum Counter : int {
@@ -124,7 +123,6 @@ struct ChainJob {
   float beta_q;               // beta * 2^-S (float)
   float beta_band;            // beta * band * 2^-S, rounded up (float)
   float beta_q_l2;            // beta * 2^-S * log2(e) (float)
-  int32_t halo;               // 1: staged with a halo (halo kernel)
   int64_t n_trials;
   int8_t* lat;                // compact species array, n_sites bytes
   uint32_t* rng;              // mt[624], then the stream position
@@ -604,28 +602,6 @@ __device__ inline void exact_pair_energies_staged(const Geom& g, const Lat& lat,
   __syncwarp();  // vbuf is reused by the next call
 }
 
-// Fixed-point swap delta for any pair, from canonical neighbour indices
-// (lanes 0-15 site 1, 16-31 site 2).
-__device__ __forceinline__ int compact_fixed_delta(const Geom& g, const int8_t* lat, const int32_t* F,
-                                              const uint32_t* ents, const SitePair& p, int lane) {
-  const bool h = lane >= 16;
-  const int cx = h ? p.bx : p.ax, cy = h ? p.by : p.ay, cz = h ? p.bz : p.az;
-  const int own = h ? p.bi : p.ai, other = h ? p.ai : p.bi;
-  const int so = h ? p.sb : p.sa, sn = h ? p.sa : p.sb;
-  const int nsp = g.ns + 1;
-  const int rowN = sn * g.nsh * nsp, rowO = so * g.nsh * nsp;
-  int acc = 0;
-  for (int k = lane & 15; k < g.z; k += 16) {
-    int dx, dy, dz, sh;
-    unpack_entry(ents[k], dx, dy, dz, sh);
-    const int ni = neighbour_index(g, cx, cy, cz, dx, dy, dz);
-    const int sb = lat[ni];
-    const int sa = ni == other ? so : (ni == own ? sn : sb);
-    acc += F[rowN + sh * nsp + sa] - F[rowO + sh * nsp + sb];
-  }
-  return __reduce_add_sync(kFull, acc);
-}
-
 // FP32 filter of u < exp(-beta*dE) for a fixed-point dE > band.
 // Returns 1 accept, 0 reject, -1 undecided.
 __device__ __forceinline__ int fast_exp_decision(const ChainJob& J, int dE, uint32_t w) {
@@ -636,29 +612,6 @@ __device__ __forceinline__ int fast_exp_decision(const ChainJob& J, int dE, uint
   if (xf < -40.0f) return w != 0u ? 0 : -1;
   float thr = __fmul_rn(expf(xf), 4294967296.0f);
   float wf = __uint2float_rn(w);
-  if (wf < __fmul_rn(thr, 1.0f - M)) return 1;
-  if (wf > __fmul_rn(thr, 1.0f + M)) return 0;
-  return -1;
-}
-
-// The base-2 filter below with the hardware 2^x (ex2.approx, whose error is
-// far inside the 4e-6 relative allowed for it here) and the per-chain part of
-// the margin taken once: c0 = 1.01 beta_band + 4.5e-6 when that is under
-// 0.0099, else +inf (every test undecided).  Only x2 in [-57.5, 0] is
-// decided with 2^x2; below, u = w 2^-32 >= 2^-32 is above 2^x2 for w > 0.
-__device__ __forceinline__ float exp2_filter_c0(float beta_band) {
-  const float c0 = beta_band * 1.01f + 4.5e-6f;
-  return c0 < 0.0099f ? c0 : INFINITY;
-}
-
-__device__ __forceinline__ int fast_ex2_decision(float nbql2, float c0, int dE, uint32_t w) {
-  const float x2 = __fmul_rn(nbql2, __int2float_rn(dE));
-  if (!(x2 >= -57.5f && x2 <= 0.0f)) return (x2 < -57.5f && w != 0u && c0 < 1.0f) ? 0 : -1;
-  const float M = __fmaf_rn(-x2, 1.5e-7f, c0);
-  float e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x2));
-  const float thr = __fmul_rn(e, 4294967296.0f);
-  const float wf = __uint2float_rn(w);
   if (wf < __fmul_rn(thr, 1.0f - M)) return 1;
   if (wf > __fmul_rn(thr, 1.0f + M)) return 0;
   return -1;

@@ -162,7 +162,8 @@ __device__ __forceinline__ int fixed_delta_rec(const Geom& g, int lat_off, int I
   return __reduce_add_sync(kFull, acc);
 }
 
-// compact_fixed_delta, also writing the neighbour codes of both sites to
+// Fixed-point swap delta for any pair, from canonical neighbour indices (lanes
+// 0-15 site 1, 16-31 site 2), also writing the neighbour codes of both sites to
 // rec[0, 2z) (site 1's entries first).
 __device__ __forceinline__ int compact_fixed_delta_rec(const Geom& g, const int8_t* lat,
                                                        const int32_t* F, const uint32_t* ents,
