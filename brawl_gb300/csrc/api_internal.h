@@ -27,6 +27,7 @@ struct ChainSlot {
   ChainJob job;
   int kernel;              // shared_kernel: with fields where it can
   uint32_t gather_smem, field_smem;  // shared memory of the two (0: it cannot)
+  double spread;           // of a swap's energy changes (gather_trials)
   uint32_t smem_lat_bytes, smem_glob_bytes;
   bool use_D;
   EnergyJob energy;

@@ -3090,6 +3090,7 @@ int api_batch_chain(brawl_batch* b, int c, ChainSlot& out) {
   out.kernel = b->field_smem[c] > 0 ? kSharedField : b->kernel[c];
   out.gather_smem = b->gather_smem[c];
   out.field_smem = b->field_smem[c];
+  out.spread = m.spread;
   out.smem_lat_bytes = smem_layout(m.g, true).total;
   out.smem_glob_bytes = smem_layout(m.g, false).total;
   out.use_D = smem_layout(m.g, false).use_D;

@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(32, kSpec == 1 || NJ == 2 ? 16 : 0) metropolis
     // this lane's word of the batch: trial (lane & 3)'s
     const int pl = (int)((pos >> (8 * min(lane & 3, kSpec - 1))) & 0xff);
     int2 v[kSpec];
-    int4 q;  // the record of the trial that ends the batch: with one, its own
+    int4 q{};  // the record of the trial that ends the batch: with one, its own
     if constexpr (kSpec == 1) {
       q = rec[(half + pl) & (kRecRing - 1)];
       v[0] = on_b ? make_int2(q.z, q.w) : make_int2(q.x, q.y);
@@ -537,14 +537,20 @@ void launch_metropolis_halo(const ChainJob* d_jobs, int n_jobs, uint32_t smem_by
   }
 }
 
-// The default's code (a server runs every chain at it).
-void preload_halo_kernels() {
+template <int K>
+static void preload_halo_depth() {
   cudaFuncAttributes a;
-  cudaFuncGetAttributes(&a, metropolis_halo_kernel<2, kGatherDefault>);
-  cudaFuncGetAttributes(&a, metropolis_halo_kernel<4, kGatherDefault>);
-  cudaFuncGetAttributes(&a, metropolis_halo_kernel<6, kGatherDefault>);
-  cudaFuncGetAttributes(&a, metropolis_halo_kernel<8, kGatherDefault>);
-  cudaFuncGetAttributes(&a, metropolis_halo_kernel<11, kGatherDefault>);
+  cudaFuncGetAttributes(&a, metropolis_halo_kernel<2, K>);
+  cudaFuncGetAttributes(&a, metropolis_halo_kernel<4, K>);
+  cudaFuncGetAttributes(&a, metropolis_halo_kernel<6, K>);
+  cudaFuncGetAttributes(&a, metropolis_halo_kernel<8, K>);
+  cudaFuncGetAttributes(&a, metropolis_halo_kernel<11, K>);
+}
+
+// The depths that a server runs chains at.
+void preload_halo_kernels() {
+  preload_halo_depth<1>();
+  preload_halo_depth<kGatherDefault>();
 }
 
 }  // namespace brawl

@@ -177,7 +177,7 @@ __global__ void ns_unstage_kernel(const NsRun* __restrict__ from, NsRun* const* 
 // others on side streams forked from it and joined back: one launch sized
 // for the largest lattice would give every small one the same shared
 // memory and leave most of each SM's slots empty.
-constexpr int kSide = 7;
+constexpr int kSide = 8;
 
 struct Pipe {
   cudaStream_t s = nullptr;
@@ -301,21 +301,24 @@ struct Group {
 
 // The kernel a chain takes in a round where fields pay (or do not), its shared
 // memory, and what the chains of one launch have alike: the kernel, with fields
-// their number per site.
+// their number per site, gathered one trial a round (very hot chains) or the default.
 int round_kernel(const ChainSlot& s, bool fields) {
   return s.kernel == kSharedField && !fields && s.gather_smem > 0 ? (int)kSharedGather : s.kernel;
 }
 uint32_t round_smem(const ChainSlot& s, bool fields) {
   return round_kernel(s, fields) == kSharedField ? s.field_smem : s.gather_smem;
 }
+int round_depth(const ChainSlot& s) {
+  return gather_trials(s.job.beta * s.spread, s.job.g.ns) == 1 ? 1 : kGatherDefault;
+}
 int round_kind(const ChainSlot& s, bool fields) {
   const int k = round_kernel(s, fields);
-  return k == kSharedField ? 8 + field_variant(s.job.g.ns) : k;
+  return k == kSharedField ? 8 + field_variant(s.job.g.ns) : k == kSharedGather ? round_depth(s) : k;
 }
 
 std::vector<Group> smem_groups(const std::vector<uint32_t>& smem, const std::vector<int>* kind = nullptr) {
   std::vector<Group> gs;
-  const int most = kind ? 3 : kSide;  // room for the changes of kind (at most four)
+  const int most = kind ? 3 : kSide;  // room for the changes of kind (at most five)
   for (int i = 0; i < (int)smem.size(); ++i) {
     const bool other = kind && i > 0 && (*kind)[i] != (*kind)[i - 1];
     if (gs.empty() || other ||
@@ -716,6 +719,7 @@ int launch_anneal(brawl_server* S, Pipe& P) {
       LaunchGroup G;
       G.kernel = round_kernel(P.launched[first]->slot, fields);
       G.ns = staged[first].g.ns;
+      G.depth = round_depth(P.launched[first]->slot);
       G.threads = field_threads(n_fields, S->n_sm);
       G.smem = sm[first];
       for (int k = first; k < first + count; ++k) G.max_z = std::max(G.max_z, (int)staged[k].g.z);
