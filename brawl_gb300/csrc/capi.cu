@@ -653,9 +653,11 @@ int upload_jobs(brawl_batch* b) {
       add(c, (int)gs.size() - 1);
     }
   }
-  int n_fields = 0;
-  for (const LaunchGroup& G : gs) n_fields += G.kernel == kSharedField ? G.count : 0;
-  for (LaunchGroup& G : gs) G.threads = field_threads(n_fields, b->n_sm);
+  std::vector<int64_t> with_fields;
+  for (int c = 0; c < n; ++c)
+    if (gid[c] >= 0 && gs[gid[c]].kernel == kSharedField) with_fields.push_back(b->jobs[c].n_trials);
+  const int threads = field_threads(with_fields, b->n_sm);
+  for (LaunchGroup& G : gs) G.threads = threads;
   std::vector<int> rank(gs.size()), at(gs.size());
   for (size_t k = 0; k < gs.size(); ++k) at[k] = (int)k;
   std::stable_sort(at.begin(), at.end(), [&](int x, int y) { return gs[x].most > gs[y].most; });
@@ -809,7 +811,7 @@ int run_metropolis_once(brawl_batch* b, const int64_t* n_trials, int64_t* accept
   } else {
     for (LaunchGroup G : b->groups)
       for (int k = G.first; k < G.first + G.count; ++k) {
-        G.threads = field_threads(1, b->n_sm);
+        G.threads = 512;  // each chain by itself
         launch_shared_chains(b->d_jobs + k, 1, G, stream);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(stream_wait(stream));

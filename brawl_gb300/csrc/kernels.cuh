@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "chain_engine.cuh"
@@ -191,10 +192,15 @@ inline bool too_hot_for_fields(double beta_spread, int z, int n_sites) {
 }
 
 // Threads per chain with fields: eight warps run the trials; the others share the
-// staging and the fields' first sums.  Where the chains that run at once (of all
-// launches) have an SM each they take 16 warps, four on each scheduler; at 113
-// registers a block of 16 would leave a second chain no place on its SM.
-inline int field_threads(int n_chains, int n_sm) { return n_chains <= n_sm ? 512 : 256; }
+// staging and the fields' first sums.  With an SM to itself a chain takes 16 warps,
+// four on each scheduler; at 113 registers a block of 16 leaves a second chain no
+// place on its SM, and with eight warps two that share one take some 1.2 times as
+// long each.  So 16 warps while the chains of all launches, the longest first and one to
+// an SM, the next where one has ended, end hardly later than the longest (trials:
+// theirs, in any order).  6,000 trials of 100 chains each of
+// bcc 6^3, 9^3 and 14^3 at 4000 K: 2.21 ms with 16 warps, 1.48 with eight; two sweeps of
+// each (864 to 10,976 trials) 1.88 and 1.96.
+int field_threads(std::vector<int64_t>& trials, int n_sm);
 
 // Wang-Landau walkers with fields (wl_field.cu: one to an SM, its registers fill
 // one) beside wl_sweep_kernel's, of which two share an SM: while each has an SM to

@@ -2,6 +2,9 @@
 // whose sites' fields fit in shared memory (field_engine.cuh); trials in the
 // reference's order (monte_carlo_step_lattice / _nbr,
 // src/metropolis.F90:751-891) on the chain's own mt19937ar stream.
+#include <algorithm>
+#include <functional>
+
 #include "accept_thresholds.cuh"
 #include "field_engine.cuh"
 
@@ -216,6 +219,23 @@ __global__ void __launch_bounds__(512, 1) metropolis_field_kernel(const ChainJob
   for (int i = tid; i < n4; i += blockDim.x) dst[i] = ((src[i] >> 2) & 0x3f3f3f3fu) + 0x01010101u;
   for (int i = (n4 << 2) + tid; i < g.n_sites; i += blockDim.x) J.lat[i] = (int8_t)((smem[L.lat + i] >> 2) + 1);
   if (tid == 0 && J.t_ns) *J.t_ns = global_ns() - t_start;
+}
+
+int field_threads(std::vector<int64_t>& trials, int n_sm) {
+  const int n = (int)trials.size();
+  if (n <= n_sm) return 512;
+  std::sort(trials.begin(), trials.end(), std::greater<int64_t>());
+  // when each SM is free, the earliest first; the next chain takes that one
+  const auto later = std::greater<int64_t>();
+  std::vector<int64_t> free_at(trials.begin(), trials.begin() + n_sm);
+  std::make_heap(free_at.begin(), free_at.end(), later);
+  for (int k = n_sm; k < n; ++k) {
+    std::pop_heap(free_at.begin(), free_at.end(), later);
+    free_at.back() += trials[k];
+    if (8 * free_at.back() > 9 * trials[0]) return 256;
+    std::push_heap(free_at.begin(), free_at.end(), later);
+  }
+  return 512;
 }
 
 template <int NJ, int R>

@@ -670,12 +670,8 @@ int launch_anneal(brawl_server* S, Pipe& P) {
   SV_TRY(grow(P.d_tns, P.tns_cap, std::max<size_t>(P.jobs.size(), 1), P.s));
   const double t_round = round_ns(S, P.jobs);
   double load = 0.0;
-  int n_fields = 0;
-  for (const auto& j : P.jobs) {
-    if (j->slot.kernel != kSharedField) continue;
-    load += field_load(j->slot.field_smem);
-    n_fields += 1;
-  }
+  for (const auto& j : P.jobs)
+    if (j->slot.kernel == kSharedField) load += field_load(j->slot.field_smem);
   const bool fields = fields_pay(load, S->n_sm);
   std::stable_sort(P.jobs.begin(), P.jobs.end(), [fields](const JobP& a, const JobP& b) {
     const int ka = round_kind(a->slot, fields), kb = round_kind(b->slot, fields);
@@ -711,16 +707,19 @@ int launch_anneal(brawl_server* S, Pipe& P) {
   if (nh > 0) {
     std::vector<uint32_t> sm(nh);
     std::vector<int> kind(nh);
+    std::vector<int64_t> with_fields;
     for (int k = 0; k < nh; ++k) {
       sm[k] = round_smem(P.launched[k]->slot, fields);
       kind[k] = round_kind(P.launched[k]->slot, fields);
+      if (kind[k] >= 8) with_fields.push_back(staged[k].n_trials);
     }
+    const int threads = field_threads(with_fields, S->n_sm);
     SV_TRY(launch_groups(P, smem_groups(sm, &kind), [&](int first, int count, cudaStream_t st) {
       LaunchGroup G;
       G.kernel = round_kernel(P.launched[first]->slot, fields);
       G.ns = staged[first].g.ns;
       G.depth = round_depth(P.launched[first]->slot);
-      G.threads = field_threads(n_fields, S->n_sm);
+      G.threads = threads;
       G.smem = sm[first];
       for (int k = first; k < first + count; ++k) G.max_z = std::max(G.max_z, (int)staged[k].g.z);
       launch_shared_chains(P.d_chain + first, count, G, st);

@@ -70,3 +70,17 @@ def test_two_chains_to_an_sm_run_at_once():
         return min(t[2:])
 
     assert fastest(300) < 1.5 * fastest(150)
+
+
+def test_a_few_long_chains_among_many_short_ones_match_oracle():
+    """Trials in proportion to the sites: the short chains wait for a place."""
+    V = random_V(np.random.default_rng(5), 4, 6)
+    b = _batch(240, V, 1500.0)
+    trials = np.array([s.n_atoms // 4 for s in b.setups])
+    acc = b.metropolis(trials)
+    for k in range(0, 240, 23):
+        mod = O.OracleModel("bcc", *[SIZES[k % 3]] * 3, V)
+        r = O.OracleRng(500 + k)
+        cfg, _ = mod.initial_setup(r, conc_vector(4))
+        a, _ = mod.mc_run(cfg, r, 1.0 / (1500.0 * B.K_B_IN_RY), int(trials[k]), False)
+        assert acc[k] == a and np.array_equal(b.config(k), cfg), k
