@@ -5,6 +5,7 @@
 #include <set>
 
 #include "asro.cuh"
+#include "kernels.cuh"
 
 namespace brawl {
 
@@ -121,8 +122,7 @@ void launch_asro(const AsroJob* d_job, const Geom& g, int n_class, cudaStream_t 
   blocks = std::max(1, std::min(blocks, 152 * 8));
   const int nsp = g.ns + 1;
   const size_t smem = (size_t)(nsp * nsp * n_class + nsp) * 4;
-  cudaFuncSetAttribute(asro_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  BRAWL_CARVEOUT(asro_kernel);
+  BRAWL_SHARED(0, asro_kernel);
   asro_kernel<<<blocks, kAsroThreads, smem, stream>>>(d_job);
 }
 

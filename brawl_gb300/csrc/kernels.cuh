@@ -32,6 +32,21 @@ template <class... Own>
 constexpr uint32_t own_bytes() { return ((uint32_t)((sizeof(Own) + 15) / 16 * 16) + ...); }
 inline uint32_t layout_room(int limit, uint32_t own) { return (uint32_t)limit - own; }
 
+// Before a launch: the kernel may take all the dynamic shared memory that its own
+// variables leave (the same value at every launch, so that a launch from another
+// thread never finds less than it needs), at the largest carveout.
+inline int dynamic_most(uint32_t own) {
+  int dev = 0, most = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return (int)layout_room(most, own);
+}
+#define BRAWL_SHARED(own, ...)                                                                        \
+  do {                                                                                                \
+    cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic_most(own)); \
+    BRAWL_CARVEOUT(__VA_ARGS__);                                                                      \
+  } while (0)
+
 constexpr uint32_t kMaxDBytes = 12 * 1024;
 
 __host__ __device__ inline SmemLayout smem_layout(const Geom& g, bool lattice_in_smem) {

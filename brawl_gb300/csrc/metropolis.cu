@@ -179,9 +179,7 @@ __global__ void __launch_bounds__(32) metropolis_kernel(const ChainJob* __restri
 template <int NJ, bool kSmemLat, bool kUseD>
 static void launch_one(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes,
                        cudaStream_t stream) {
-  cudaFuncSetAttribute(metropolis_kernel<NJ, kSmemLat, kUseD>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  BRAWL_CARVEOUT(metropolis_kernel<NJ, kSmemLat, kUseD>);
+  BRAWL_SHARED(kOneWarpOwn, metropolis_kernel<NJ, kSmemLat, kUseD>);
   metropolis_kernel<NJ, kSmemLat, kUseD><<<n_jobs, 32, smem_bytes, stream>>>(d_jobs);
 }
 

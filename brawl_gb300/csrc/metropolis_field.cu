@@ -240,8 +240,7 @@ int field_threads(std::vector<int64_t>& trials, int n_sm) {
 
 template <int NJ, int R>
 static void launch_field_r(const ChainJob* d_jobs, int n_jobs, int threads, uint32_t smem_bytes, cudaStream_t stream) {
-  cudaFuncSetAttribute(metropolis_field_kernel<NJ, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  BRAWL_CARVEOUT(metropolis_field_kernel<NJ, R>);
+  BRAWL_SHARED(kFieldOwn, metropolis_field_kernel<NJ, R>);
   metropolis_field_kernel<NJ, R><<<n_jobs, threads, smem_bytes, stream>>>(d_jobs);
 }
 

@@ -510,8 +510,7 @@ __global__ void __launch_bounds__(32, kSpec == 1 || NJ == 2 ? 16 : 0) metropolis
 
 template <int NJ, int K>
 static void launch_halo_nj(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, cudaStream_t stream) {
-  cudaFuncSetAttribute(metropolis_halo_kernel<NJ, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  BRAWL_CARVEOUT(metropolis_halo_kernel<NJ, K>);
+  BRAWL_SHARED(kOneWarpOwn, metropolis_halo_kernel<NJ, K>);
   metropolis_halo_kernel<NJ, K><<<n_jobs, 32, smem_bytes, stream>>>(d_jobs);
 }
 

@@ -393,9 +393,7 @@ __global__ void __launch_bounds__(kRoundThreads, 1) metropolis_rounds_kernel(con
 
 template <int NJ, bool kNibbles>
 static void launch_rounds_lat(const ChainJob* d_jobs, int n_jobs, uint32_t smem_bytes, cudaStream_t stream) {
-  cudaFuncSetAttribute(metropolis_rounds_kernel<NJ, kNibbles>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem_bytes);
-  BRAWL_CARVEOUT((metropolis_rounds_kernel<NJ, kNibbles>));
+  BRAWL_SHARED(kRoundsOwn, (metropolis_rounds_kernel<NJ, kNibbles>));
   metropolis_rounds_kernel<NJ, kNibbles><<<n_jobs, kRoundThreads, smem_bytes, stream>>>(d_jobs);
 }
 

@@ -330,9 +330,7 @@ void launch_ns_jitter(NsRun* d_runs, int n_runs, int max_K, cudaStream_t stream)
 
 template <int NJ, bool kUseD>
 static void launch_ns_nj(NsRun* d_runs, int n_runs, uint32_t smem_bytes, cudaStream_t stream) {
-  cudaFuncSetAttribute(ns_iterate_kernel<NJ, kUseD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem_bytes);
-  BRAWL_CARVEOUT(ns_iterate_kernel<NJ, kUseD>);
+  BRAWL_SHARED(kOneWarpOwn, ns_iterate_kernel<NJ, kUseD>);
   ns_iterate_kernel<NJ, kUseD><<<n_runs, 32 * kNsWarps, smem_bytes, stream>>>(d_runs);
 }
 

@@ -652,8 +652,7 @@ __global__ void __launch_bounds__(kNsThreads, 1) ns_rounds_kernel(NsRun* __restr
 
 template <int NJ>
 static void launch_rounds_nj(NsRun* d_runs, int n_runs, uint32_t smem_bytes, cudaStream_t stream) {
-  cudaFuncSetAttribute(ns_rounds_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  BRAWL_CARVEOUT(ns_rounds_kernel<NJ>);
+  BRAWL_SHARED(kNsRoundsOwn, ns_rounds_kernel<NJ>);
   ns_rounds_kernel<NJ><<<n_runs, kNsThreads, smem_bytes, stream>>>(d_runs);
 }
 

@@ -531,8 +531,7 @@ uint32_t wl_enter_smem_bytes(const Geom& g) {
 }
 
 void launch_wl_enter(WlEnterJob* d_jobs, int n, uint32_t smem, cudaStream_t stream) {
-  cudaFuncSetAttribute(wl_enter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  BRAWL_CARVEOUT(wl_enter_kernel);
+  BRAWL_SHARED(0, wl_enter_kernel);
   if (n > 0) wl_enter_kernel<<<n, 32, smem, stream>>>(d_jobs);
 }
 
@@ -570,8 +569,7 @@ uint32_t wl_smem_bytes(const Geom& g, int nb, int lazy_cap, int rad_bins, int ra
 
 template <int NJ, bool kUseD>
 static void launch_wl_nj(WlWalker* d_walkers, int n, uint32_t smem, cudaStream_t stream) {
-  cudaFuncSetAttribute(wl_sweep_kernel<NJ, kUseD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  BRAWL_CARVEOUT(wl_sweep_kernel<NJ, kUseD>);
+  BRAWL_SHARED(kOneWarpOwn, wl_sweep_kernel<NJ, kUseD>);
   wl_sweep_kernel<NJ, kUseD><<<n, 32 * kWlWarps, smem, stream>>>(d_walkers);
 }
 
@@ -766,8 +764,7 @@ void launch_wl_exchange(WlWalker* d_walkers, const double* d_energy, const WlGro
                         int n_windows, int per_window, int* d_ibin, int2* d_ov, int* d_partner,
                         int* d_exchanged, int* d_n_accepted, cudaStream_t stream) {
   const uint32_t smem = wl_exchange_smem_bytes(per_window);
-  cudaFuncSetAttribute(wl_exchange_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  BRAWL_CARVEOUT(wl_exchange_kernel);
+  BRAWL_SHARED(0, wl_exchange_kernel);
   wl_exchange_kernel<<<1, 32, smem, stream>>>(d_walkers, d_energy, d_groups, n_windows, per_window,
                                               d_ibin, d_ov, d_partner, d_exchanged, d_n_accepted);
 }

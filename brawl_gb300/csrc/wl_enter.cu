@@ -407,8 +407,7 @@ __global__ void __launch_bounds__(256, 1) wl_enter_field_kernel(WlEnterJob* __re
 
 template <int NJ, int R>
 static void launch_enter_r(WlEnterJob* d_jobs, int n, uint32_t smem, cudaStream_t stream) {
-  cudaFuncSetAttribute(wl_enter_field_kernel<NJ, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  BRAWL_CARVEOUT(wl_enter_field_kernel<NJ, R>);
+  BRAWL_SHARED(kWlEnterOwn, wl_enter_field_kernel<NJ, R>);
   wl_enter_field_kernel<NJ, R><<<n, 256, smem, stream>>>(d_jobs);
 }
 

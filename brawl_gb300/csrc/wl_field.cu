@@ -547,8 +547,7 @@ __global__ void __launch_bounds__(256, 1) wl_field_kernel(WlWalker* __restrict__
 
 template <int NJ, int R>
 static void launch_wl_field_r(WlWalker* d_walkers, int n, uint32_t smem, int threads, cudaStream_t stream) {
-  cudaFuncSetAttribute(wl_field_kernel<NJ, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  BRAWL_CARVEOUT(wl_field_kernel<NJ, R>);
+  BRAWL_SHARED(kWlFieldOwn, wl_field_kernel<NJ, R>);
   wl_field_kernel<NJ, R><<<n, threads, smem, stream>>>(d_walkers);
 }
 
