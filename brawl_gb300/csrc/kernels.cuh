@@ -36,9 +36,12 @@ inline uint32_t layout_room(int limit, uint32_t own) { return (uint32_t)limit - 
 // variables leave (the same value at every launch, so that a launch from another
 // thread never finds less than it needs), at the largest carveout.
 inline int dynamic_most(uint32_t own) {
-  int dev = 0, most = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  static const int most = [] {  // (the same on every device that runs this code)
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    return v;
+  }();
   return (int)layout_room(most, own);
 }
 #define BRAWL_SHARED(own, ...)                                                                        \
