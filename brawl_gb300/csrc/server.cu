@@ -1039,11 +1039,14 @@ void fail_pipe(brawl_server* S, Pipe& P, int rc) {
 // job larger than the budget is admitted alone) and build their device
 // objects on the objects' own streams, so the pipelines keep running.
 // Wang-Landau and nested-sampling jobs have their own resident caps: a
-// walker or run on a large lattice holds a whole SM (its shared memory) for
-// a long round, and past a few dozen of them the anneal chains lose more
-// SMs than the walks add work (on a mixed stream at 250 jobs/s, 45 s:
-// 7.3e8 trials/s with 32 of each kind resident, 6.8e8 with 64, 2.5e8 with
-// 128), while anneal chains keep gaining up to thousands.  A queued job of
+// run in rounds holds a whole SM (its registers), a walker on a large lattice
+// too (its shared memory), for a long round, and past a few dozen of them the
+// anneal chains lose more SMs than the walks add work, while anneal chains keep
+// gaining up to thousands.  A mixed stream at 250 jobs/s for 45 s with 64
+// Wang-Landau jobs and 32, 40, 48 and 64 runs: 12.1, 11.2, 10.5-11.9 and 6.0-6.4e8 trials/s,
+// 2.9, 3.6, 4.0-4.2 and 4.3e7 of them the runs' (6.8e8 and 3.6e7 with 64 where a run took
+// half an SM, ns_iterate_kernel); the slowest hundredth of 300 jobs at 80 a
+// second waits 2.8, 1.2, 0.33 and 0.11 s (1.5 then).  A queued job of
 // a kind at its cap waits; the first later job of another kind is admitted
 // instead.
 int kind_cap(const brawl_server* S, int kind) {
@@ -1237,7 +1240,7 @@ int brawl_serve_create(const brawl_server_opts* opts, brawl_server** out) {
   }
   if (S->o.max_active <= 0) S->o.max_active = 4096;
   if (S->o.max_active_wl <= 0) S->o.max_active_wl = 64;
-  if (S->o.max_active_ns <= 0) S->o.max_active_ns = 64;
+  if (S->o.max_active_ns <= 0) S->o.max_active_ns = 48;
   if (!(S->o.round_ms > 0.0)) S->o.round_ms = 20.0;
   if (S->o.max_trials < 0) S->o.max_trials = 0;
   if (S->o.max_iterations < 0) S->o.max_iterations = 0;
