@@ -235,7 +235,7 @@ def committed_smem() -> dict | None:
 
 def roofline_object(achieved_gbs, smem_peak, peaks, traffic, alg_per_step, trials_per_s) -> dict:
     """The Metropolis kernel against the ceiling that bounds it: its bytes
-    are served from shared memory (DRAM traffic per launch is the lattices'
+    are served from shared memory (DRAM traffic per step is the lattices'
     staging only), so the peak is the measured shared-memory bandwidth; the
     HBM copy rate is given beside it."""
     out = {"bound": "smem", "achieved": achieved_gbs, "unit": "GB/s",
@@ -260,9 +260,9 @@ def roofline_object(achieved_gbs, smem_peak, peaks, traffic, alg_per_step, trial
 
 
 def committed_traffic() -> dict | None:
-    """DRAM traffic per launch of the Metropolis kernel on the 1024-replica
-    workload, from the committed ncu summary
-    (profiles/metropolis_batched_traffic.json), if present."""
+    """DRAM traffic of one step's launches on the 1024-replica workload,
+    from the committed ncu summary (profiles/metropolis_batched_traffic.json),
+    if present."""
     p = os.path.join(ROOT, "profiles", "metropolis_batched_traffic.json")
     if os.path.exists(p):
         with open(p) as f:
@@ -943,8 +943,8 @@ def main() -> int:
     smem_peak = smem_bandwidth_gbs()
     traffic = None
     tr = committed_traffic()
-    if tr and tr.get("dram_bytes_per_launch") and args.replicas == 1024:
-        traffic = float(tr["dram_bytes_per_launch"])     # one launch per step
+    if tr and tr.get("dram_bytes_per_step") and args.replicas == 1024:
+        traffic = float(tr["dram_bytes_per_step"])       # of all its launches
 
     # ---- end to end through the C ABI with host buffers -------------------
     grid_bytes = batch.grid_bytes

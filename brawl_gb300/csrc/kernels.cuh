@@ -233,7 +233,9 @@ inline bool wl_fields_pay(int n_walkers, int n_sm) { return n_walkers <= n_sm; }
 // (its sixteen warps' registers fill one): 152 chains take as long as one, 0.74 ms
 // (simple cubic 6^3, 4,000 trials) and 1.0 (8^3, two species), and twice as many
 // twice that, where metropolis_kernel, a warp a chain, takes 2.7 and 1.75 for
-// either.
+// either.  So a second wave would still gain where changes of exactly zero are few
+// (1.48 against 2.7) and lose where two species make them common (2.0 against 1.75):
+// which it is shows only as the chains run, so the line is where no chain waits.
 inline bool rounds_pay(int n_chains, int n_sm) { return n_chains <= n_sm; }
 // And whether the longest of them pays for half bytes in shared memory, where
 // metropolis_kernel leaves the lattice in global memory: 1, 10 and 100 trials of eight
